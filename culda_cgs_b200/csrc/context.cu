@@ -844,6 +844,7 @@ extern "C" int culda_create(const culda_corpus *c, const culda_params *p, culda_
         ctx->num_items = (int32_t)items.size();
         ctx->num_hot = nhot;
         ctx->num_hot_items = (int32_t)hot.size();
+        ctx->num_long_items = (int32_t)long_items(items.data(), (int64_t)items.size());
     }
     ctx->sample_grid = std::max(1, std::min(ctx->num_items, sms * sbps));
 
@@ -901,6 +902,7 @@ extern "C" int culda_create(const culda_corpus *c, const culda_params *p, culda_
         const size_t o_iter = add(sizeof(uint32_t));
         const size_t o_stats = add(sizeof(DevStats));
         const size_t o_nk = add(sizeof(int32_t) * (size_t)K);
+        const size_t o_partials = add(sizeof(double) * kMaxPartials);
         // the region set-up borrows, in the order it gives the buffers back
         const size_t o_doc_tok = add(sizeof(int32_t) * (size_t)N);
         const size_t o_seg_start = add(sizeof(int32_t) * (size_t)N);  // at most one segment per token
@@ -937,6 +939,7 @@ extern "C" int culda_create(const culda_corpus *c, const culda_params *p, culda_
         ctx->d_iter = reinterpret_cast<uint32_t *>(b + o_iter);
         ctx->d_stats = reinterpret_cast<DevStats *>(b + o_stats);
         ctx->d_nk = reinterpret_cast<int32_t *>(b + o_nk);
+        ctx->d_partials = reinterpret_cast<double *>(b + o_partials);
         ctx->d_z[0] = reinterpret_cast<uint16_t *>(b + o_z0);
         ctx->d_z[1] = reinterpret_cast<uint16_t *>(b + o_z1);
         ctx->d_zx = reinterpret_cast<uint16_t *>(b + o_zx);
@@ -1295,33 +1298,35 @@ extern "C" int culda_loglik_joint(culda_ctx *ctx, double *ll) {
     if (!ctx || !ll) return fail(ctx, CULDA_ERR_INVALID_ARG, "culda_loglik_joint: null argument");
     CK(cudaSetDevice(ctx->device));
     cudaStream_t s = ctx->stream;
-    const int P = num_sms(ctx->device) * 4;
-    double *d_part = nullptr;
-    CK(dalloc(&d_part, (size_t)P));
-    CK(launch_loglik_joint(ctx->K, ctx->V, ctx->D, ctx->params.alpha, ctx->params.beta, ctx->d_word_ptr,
-                           ctx->d_z[ctx->cur], ctx->d_rows, ctx->d_theta, ctx->d_doc_ptr, d_part, P, ctx->d_error,
-                           s));
-    std::vector<double> part((size_t)P);
-    std::vector<int32_t> nk((size_t)ctx->K);
-    CK(cudaMemcpyAsync(part.data(), d_part, sizeof(double) * (size_t)P, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(nk.data(), ctx->d_nk, sizeof(int32_t) * (size_t)ctx->K, cudaMemcpyDeviceToHost, s));
+    if (ctx->num_hot > 0) {
+        CK(cudaMemsetAsync(ctx->d_hot_phi, 0, sizeof(int32_t) * (size_t)ctx->num_hot * ctx->K, s));
+        CK(launch_hot_rows(ctx->K, ctx->d_hot_items, ctx->num_hot_items, ctx->d_z[ctx->cur], ctx->d_hot_phi,
+                           ctx->d_error, s));
+    }
+    JointParams p{};
+    p.k = ctx->K;
+    p.num_words = ctx->V;
+    p.num_docs = ctx->D;
+    p.num_items = ctx->num_items;
+    p.num_long = ctx->num_long_items;
+    p.alpha = ctx->params.alpha;
+    p.beta = ctx->params.beta;
+    p.items = ctx->d_items;
+    p.hot_phi = ctx->d_hot_phi;
+    p.topics = ctx->d_z[ctx->cur];
+    p.rows = ctx->d_rows;
+    p.theta = ctx->d_theta;
+    p.doc_ptr = ctx->d_doc_ptr;
+    p.nk = ctx->d_nk;
+    p.partials = ctx->d_partials;
+    p.done = ctx->d_counter + 32;
+    p.result = &ctx->h_stats->joint;  // pinned, mapped
+    p.error = ctx->d_error;
+    CK(launch_loglik_joint(p, kMaxPartials, s));
     CK(cudaStreamSynchronize(s));
-    cudaFree(d_part);
-    const double a = ctx->params.alpha, b = ctx->params.beta, vb = (double)ctx->V * b, ka = (double)ctx->K * a;
-    double sum = 0, comp = 0;
-    auto add = [&](double x) {
-        const double t = sum + x;
-        if (std::fabs(sum) >= std::fabs(x))
-            comp += (sum - t) + x;
-        else
-            comp += (x - t) + sum;
-        sum = t;
-    };
-    for (double x : part) add(x);
-    add((double)ctx->K * std::lgamma(vb));
-    for (int32_t k : nk) add(-std::lgamma((double)k + vb));
-    add((double)ctx->D * std::lgamma(ka));
-    *ll = sum + comp;
+    const double a = ctx->params.alpha, b = ctx->params.beta;
+    *ll = ctx->h_stats->joint + (double)ctx->K * std::lgamma((double)ctx->V * b) +
+          (double)ctx->D * std::lgamma((double)ctx->K * a);
     return CULDA_OK;
 }
 

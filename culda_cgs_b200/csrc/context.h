@@ -11,6 +11,9 @@
 
 #include "kernels.cuh"
 
+// Per-CTA partial sums a reduction may leave in culda_ctx::d_partials.
+constexpr int kMaxPartials = 4096;
+
 struct culda_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -39,6 +42,8 @@ struct culda_ctx {
     int32_t *d_nk = nullptr;
     culda_item *d_items = nullptr, *d_hot_items = nullptr;
     int32_t num_items = 0, num_hot_items = 0, num_hot = 0;
+    int32_t num_long_items = 0;          // items counted by a whole CTA (long_items)
+    double *d_partials = nullptr;        // [kMaxPartials] per-CTA sums of the reductions
     int32_t *d_seg_start = nullptr;  // first stored token of every segment
     int32_t num_segs = 0;
     int32_t *d_hot_phi = nullptr;

@@ -57,6 +57,7 @@ struct DevStats {
     int64_t token_nnz;    // sum_d L_d * nnz_d after the rebuild            (stats slot 2)
     int32_t error;
     uint32_t iteration;   // Philox iteration the sampler used
+    double joint;         // joint log-likelihood sum (written to the host copy only)
 };
 
 inline int pow2_ceil(int k) {
@@ -116,10 +117,27 @@ cudaError_t launch_phi_head(int k, float beta, int num_words, const int32_t *phi
 cudaError_t launch_doc_check(int64_t n, int num_docs, const int32_t *doc_ids, int32_t *doc_count, int32_t *error,
                              cudaStream_t s);
 
-cudaError_t launch_loglik_joint(int k, int num_words, int num_docs, float alpha, float beta, const int64_t *word_ptr,
-                                const uint16_t *topics, const int2 *rows, const ThetaEntry *theta,
-                                const int64_t *doc_ptr, double *partials, int num_partials, int32_t *error,
-                                cudaStream_t s);
+// Joint log-likelihood (see kernels.cu): items are the sampler's work list,
+// largest first, with the hot rows of the current topics.
+struct JointParams {
+    int32_t k, num_words, num_docs;
+    int32_t num_items, num_long;  // num_long: long_items() of the list
+    double alpha, beta;
+    const culda_item *items;
+    const int32_t *hot_phi;
+    const uint16_t *topics;
+    const int2 *rows;
+    const ThetaEntry *theta;
+    const int64_t *doc_ptr;
+    const int32_t *nk;
+    double *partials;  // one per CTA
+    int32_t *done;     // CTAs finished (cleared by the launch)
+    double *result;    // receives the sum; may be mapped host memory
+    int32_t *error;
+};
+cudaError_t launch_loglik_joint(const JointParams &p, int max_partials, cudaStream_t s);
+// The items of a work list (largest first) that a whole CTA counts.
+int64_t long_items(const culda_item *items, int64_t n);
 
 // Internal token order: within each word, tokens sorted by their doc's length
 // (longest first, doc id breaking ties).  keys[t] = (word << 16) | (65535 - L).
