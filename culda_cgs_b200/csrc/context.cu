@@ -5,9 +5,11 @@
 // Replaces SingleChunkSingleGPU (src_culda/train/SingleChunkSingleGPU.h:5-157)
 // and the device-owning parts of DocChunk, ModelPhi/ModelPhiGPU and
 // ModelTheta/ModelThetaChunk.  One iteration is one graph launch:
-//   memset(work counter, hot rows) -> hot_rows -> sample(z[c] -> z[1-c])
-//   -> finalize_ll -> memset(n_k, stats) -> theta_rebuild(z[1-c])
-//   -> stats D2H (pinned)
+//   prologue (counters, totals and hot rows cleared, uniforms) -> hot_rows
+//   -> sample(z[c] -> z[1-c]) -> theta_rebuild(z[1-c]), whose last CTA writes
+//   the iteration's statistics to pinned memory
+// (with memset, event and copy nodes between the kernels an iteration of 1M
+// tokens idled for 75 of 300 us).
 // Two graphs alternate the topic buffers (z is double-buffered so hot words
 // split over several CTAs read a stable snapshot while others write).
 #include <cuda_runtime.h>
@@ -116,6 +118,8 @@ int fail(culda_ctx *c, int code, const char *fmt, ...) {
 // Queue counter of the theta rebuild's block bin: its own 64-byte line of the
 // counter array (slot 0 is the sampler's work queue).
 static int32_t *theta_queue(culda_ctx *ctx) { return ctx->d_counter + 16; }
+// CTAs finished, for kernels whose last CTA has more to do.
+static int32_t *done_counter(culda_ctx *ctx) { return ctx->d_counter + 32; }
 
 // Docs of at least min_len tokens (a prefix of the longest-first doc order).
 static int count_long_docs(const culda_ctx *ctx, int min_len) {
@@ -159,7 +163,7 @@ SampleParams sample_params(const culda_ctx *ctx, int cur, uint32_t iteration, co
     p.topics_out = ctx->d_z[1 - cur];
     p.theta = ctx->d_theta;
     p.rows = ctx->d_rows;
-    p.nk = ctx->d_nk;
+    p.nk = ctx->d_nk[cur];
     p.items = ctx->d_items;
     p.seg_start = ctx->d_seg_start;
     p.num_segs = ctx->num_segs;
@@ -172,52 +176,55 @@ SampleParams sample_params(const culda_ctx *ctx, int cur, uint32_t iteration, co
     p.iteration = iteration;
     p.iteration_ptr = iteration_ptr;
     p.error = ctx->d_error;
+    p.clock = &ctx->d_stats->sample_t0;
     return p;
 }
 
-namespace {
+cudaError_t iteration_prologue(culda_ctx *ctx, int cur, bool uniforms, uint32_t iteration,
+                               const uint32_t *iteration_ptr) {
+    PrologueParams p{};
+    p.n = uniforms ? ctx->N : 0;
+    p.seed = ctx->params.seed;
+    p.iteration_dev = iteration_ptr;
+    p.iteration = iteration;
+    p.tok_index = ctx->d_tok_index;
+    p.u = ctx->d_u;
+    p.counter = ctx->d_counter;
+    p.theta_queue = theta_queue(ctx);
+    p.done = done_counter(ctx);
+    p.hot_phi = ctx->d_hot_phi;
+    p.hot_n = ctx->d_frozen_phi ? 0 : (int64_t)ctx->num_hot * ctx->K;
+    p.nk_next = ctx->d_nk[1 - cur];
+    p.k = ctx->K;
+    p.stats = ctx->d_stats;
+    cudaError_t e = launch_prologue(p, ctx->stream);
+    if (e == cudaSuccess && p.hot_n > 0)
+        e = launch_hot_rows(ctx->K, ctx->d_hot_items, ctx->num_hot_items, ctx->d_z[cur], ctx->d_hot_phi, ctx->d_error,
+                            ctx->stream);
+    return e;
+}
 
-__global__ void copy_error_kernel(const int32_t *err, DevStats *st) { st->error = *err; }
-
-}  // namespace
-
-// Inside a stream capture a plain event record only orders the capture; the
-// external flag turns it into an event-record node of the graph so the event
-// can be timed after each launch.
-cudaError_t record_event(cudaEvent_t ev, cudaStream_t s) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    cudaError_t e = cudaStreamIsCapturing(s, &cs);
-    if (e != cudaSuccess) return e;
-    return cs == cudaStreamCaptureStatusActive ? cudaEventRecordWithFlags(ev, s, cudaEventRecordExternal)
-                                               : cudaEventRecord(ev, s);
+cudaError_t iteration_rebuild(culda_ctx *ctx, int cur, int num_items) {
+    IterationEnd end;
+    end.stats = ctx->d_stats;
+    end.item_ll = ctx->d_item_ll;
+    end.num_items = num_items;
+    end.partials = ctx->d_partials;
+    end.done = done_counter(ctx);
+    end.iteration_dev = ctx->d_iter;
+    end.ring = ctx->h_stats;
+    return launch_theta_rebuild(ctx->K, ctx->D, ctx->d_doc_ptr, ctx->d_doc_tok, ctx->d_z[1 - cur], ctx->d_doc_order,
+                                ctx->d_rows, ctx->d_theta, ctx->d_nk[1 - cur], &ctx->d_stats->row_entries,
+                                ctx->d_error, ctx->theta_grid, ctx->stream, ctx->theta_long, theta_queue(ctx), end);
 }
 
 namespace {
 
 int record_iteration(culda_ctx *ctx, cudaStream_t s, int cur) {
-    const int nxt = 1 - cur;
-    CK(cudaMemsetAsync(ctx->d_counter, 0, sizeof(int32_t), s));
-    if (ctx->num_hot > 0 && !ctx->d_frozen_phi) {
-        CK(cudaMemsetAsync(ctx->d_hot_phi, 0, sizeof(int32_t) * (size_t)ctx->num_hot * ctx->K, s));
-        CK(launch_hot_rows(ctx->K, ctx->d_hot_items, ctx->num_hot_items, ctx->d_z[cur], ctx->d_hot_phi, ctx->d_error,
-                           s));
-    }
-    CK(launch_uniforms(ctx->N, ctx->params.seed, ctx->d_iter, 0u, ctx->d_tok_index, ctx->d_u, s));
-    CK(record_event(ctx->ev_s0, s));
+    CK(iteration_prologue(ctx, cur, true, 0u, ctx->d_iter));
     CK(launch_sample(sample_params(ctx, cur, 0u, ctx->d_iter), ctx->group_lanes, ctx->sample_blocks,
                      ctx->sample_grid, s));
-    CK(record_event(ctx->ev_s1, s));
-    CK(launch_finalize_ll(ctx->d_item_ll, ctx->num_items, ctx->d_stats, ctx->d_iter, s));
-    CK(cudaMemsetAsync(ctx->d_nk, 0, sizeof(int32_t) * (size_t)ctx->K, s));
-    CK(cudaMemsetAsync(&ctx->d_stats->row_entries, 0, 3 * sizeof(int64_t), s));
-    CK(record_event(ctx->ev_t0, s));
-    CK(launch_theta_rebuild(ctx->K, ctx->D, ctx->d_doc_ptr, ctx->d_doc_tok, ctx->d_z[nxt], ctx->d_doc_order,
-                            ctx->d_rows, ctx->d_theta, ctx->d_nk, &ctx->d_stats->row_entries, ctx->d_error,
-                            ctx->theta_grid, s, ctx->theta_long, theta_queue(ctx)));
-    CK(record_event(ctx->ev_t1, s));
-    copy_error_kernel<<<1, 1, 0, s>>>(ctx->d_error, ctx->d_stats);
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(ctx->h_stats, ctx->d_stats, sizeof(DevStats), cudaMemcpyDeviceToHost, s));
+    CK(iteration_rebuild(ctx, cur, ctx->num_items));
     return CULDA_OK;
 }
 
@@ -226,10 +233,10 @@ int record_iteration(culda_ctx *ctx, cudaStream_t s, int cur) {
 // Rebuild theta rows and n_k from the current topics (set-up and set_topics).
 int rebuild_counts(culda_ctx *ctx) {
     cudaStream_t s = ctx->stream;
-    CK(cudaMemsetAsync(ctx->d_nk, 0, sizeof(int32_t) * (size_t)ctx->K, s));
+    CK(cudaMemsetAsync(ctx->d_nk[ctx->cur], 0, sizeof(int32_t) * (size_t)ctx->K, s));
     CK(cudaMemsetAsync(&ctx->d_stats->row_entries, 0, 3 * sizeof(int64_t), s));
     CK(launch_theta_rebuild(ctx->K, ctx->D, ctx->d_doc_ptr, ctx->d_doc_tok, ctx->d_z[ctx->cur], ctx->d_doc_order,
-                            ctx->d_rows, ctx->d_theta, ctx->d_nk, &ctx->d_stats->row_entries, ctx->d_error,
+                            ctx->d_rows, ctx->d_theta, ctx->d_nk[ctx->cur], &ctx->d_stats->row_entries, ctx->d_error,
                             ctx->theta_grid, s, ctx->theta_long, theta_queue(ctx)));
     CK(cudaStreamSynchronize(s));
     int32_t e = 0;
@@ -260,11 +267,11 @@ int autotune_rebuild(culda_ctx *ctx, TuneResult &best) {
         seen_long.push_back(nl);
         float t = 0.f;
         for (int rep = 0; rep < 3; ++rep) {
-            CK(cudaMemsetAsync(ctx->d_nk, 0, sizeof(int32_t) * (size_t)ctx->K, s));
+            CK(cudaMemsetAsync(ctx->d_nk[ctx->cur], 0, sizeof(int32_t) * (size_t)ctx->K, s));
             CK(cudaMemsetAsync(&ctx->d_stats->row_entries, 0, 3 * sizeof(int64_t), s));
             CK(cudaEventRecord(ctx->ev0, s));
             CK(launch_theta_rebuild(ctx->K, ctx->D, ctx->d_doc_ptr, ctx->d_doc_tok, ctx->d_z[ctx->cur],
-                                    ctx->d_doc_order, ctx->d_rows, ctx->d_theta, ctx->d_nk,
+                                    ctx->d_doc_order, ctx->d_rows, ctx->d_theta, ctx->d_nk[ctx->cur],
                                     &ctx->d_stats->row_entries, ctx->d_error, ctx->theta_grid, s, nl,
                                     theta_queue(ctx)));
             CK(cudaEventRecord(ctx->ev1, s));
@@ -311,12 +318,7 @@ int autotune_sampler(culda_ctx *ctx) {
     }
     cudaStream_t s = ctx->stream;
     const int cur = ctx->cur;
-    if (ctx->num_hot > 0 && !ctx->d_frozen_phi) {
-        CK(cudaMemsetAsync(ctx->d_hot_phi, 0, sizeof(int32_t) * (size_t)ctx->num_hot * ctx->K, s));
-        CK(launch_hot_rows(ctx->K, ctx->d_hot_items, ctx->num_hot_items, ctx->d_z[cur], ctx->d_hot_phi, ctx->d_error,
-                           s));
-    }
-    CK(launch_uniforms(ctx->N, ctx->params.seed, nullptr, 1u, ctx->d_tok_index, ctx->d_u, s));
+    CK(iteration_prologue(ctx, cur, true, 1u, nullptr));
     const SampleParams sp = sample_params(ctx, cur, 1u, nullptr);
     best.ms = 0.f;
     for (const auto &c : kCands) {
@@ -556,9 +558,9 @@ __global__ void item_segments_kernel(culda_item *items, int num_items, const int
     }
 }
 
-// A process-wide pool of pinned DevStats slots: a cudaMallocHost costs
-// milliseconds, so contexts take slots from shared pinned pages and give them
-// back on destroy (the pages live as long as the process).
+// A process-wide pool of pinned slots of kStatsRing DevStats: a cudaMallocHost
+// costs milliseconds, so contexts take slots from shared pinned pages and give
+// them back on destroy (the pages live as long as the process).
 std::mutex g_pinned_mu;
 std::vector<DevStats *> g_pinned_free;
 
@@ -567,8 +569,8 @@ DevStats *pinned_stats_get() {
     if (g_pinned_free.empty()) {
         constexpr int kSlots = 64;
         DevStats *page = nullptr;
-        if (cudaMallocHost((void **)&page, sizeof(DevStats) * kSlots) != cudaSuccess) return nullptr;
-        for (int i = kSlots - 1; i >= 0; --i) g_pinned_free.push_back(page + i);
+        if (cudaMallocHost((void **)&page, sizeof(DevStats) * kStatsRing * kSlots) != cudaSuccess) return nullptr;
+        for (int i = kSlots - 1; i >= 0; --i) g_pinned_free.push_back(page + i * kStatsRing);
     }
     DevStats *p = g_pinned_free.back();
     g_pinned_free.pop_back();
@@ -760,10 +762,7 @@ extern "C" int culda_create(const culda_corpus *c, const culda_params *p, culda_
     CKB(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     CKB(cudaEventCreate(&ctx->ev0));
     CKB(cudaEventCreate(&ctx->ev1));
-    CKB(cudaEventCreate(&ctx->ev_s0));
-    CKB(cudaEventCreate(&ctx->ev_s1));
-    CKB(cudaEventCreate(&ctx->ev_t0));
-    CKB(cudaEventCreate(&ctx->ev_t1));
+    for (cudaEvent_t &ev : ctx->ev_iter) CKB(cudaEventCreate(&ev));
     cudaStream_t s = ctx->stream;
     const int64_t N = ctx->N;
     const int32_t D = ctx->D, V = ctx->V, K = ctx->K;
@@ -901,7 +900,8 @@ extern "C" int culda_create(const culda_corpus *c, const culda_params *p, culda_
         const size_t o_counter = add(64 * sizeof(int32_t));
         const size_t o_iter = add(sizeof(uint32_t));
         const size_t o_stats = add(sizeof(DevStats));
-        const size_t o_nk = add(sizeof(int32_t) * (size_t)K);
+        const size_t o_nk0 = add(sizeof(int32_t) * (size_t)K);
+        const size_t o_nk1 = add(sizeof(int32_t) * (size_t)K);
         const size_t o_partials = add(sizeof(double) * kMaxPartials);
         // the region set-up borrows, in the order it gives the buffers back
         const size_t o_doc_tok = add(sizeof(int32_t) * (size_t)N);
@@ -938,7 +938,8 @@ extern "C" int culda_create(const culda_corpus *c, const culda_params *p, culda_
         ctx->d_counter = reinterpret_cast<int32_t *>(b + o_counter);
         ctx->d_iter = reinterpret_cast<uint32_t *>(b + o_iter);
         ctx->d_stats = reinterpret_cast<DevStats *>(b + o_stats);
-        ctx->d_nk = reinterpret_cast<int32_t *>(b + o_nk);
+        ctx->d_nk[0] = reinterpret_cast<int32_t *>(b + o_nk0);
+        ctx->d_nk[1] = reinterpret_cast<int32_t *>(b + o_nk1);
         ctx->d_partials = reinterpret_cast<double *>(b + o_partials);
         ctx->d_z[0] = reinterpret_cast<uint16_t *>(b + o_z0);
         ctx->d_z[1] = reinterpret_cast<uint16_t *>(b + o_z1);
@@ -1097,7 +1098,7 @@ extern "C" int culda_create(const culda_corpus *c, const culda_params *p, culda_
         fail(ctx, CULDA_ERR_OOM, "culda_create: pinned host memory for the iteration statistics");
         return bail(CULDA_ERR_OOM);
     }
-    memset(ctx->h_stats, 0, sizeof(DevStats));
+    memset(ctx->h_stats, 0, sizeof(DevStats) * kStatsRing);
     CKB(cudaMemsetAsync(ctx->d_stats, 0, sizeof(DevStats), s));
     const uint32_t one = 1;
     CKB(cudaMemcpyAsync(ctx->d_iter, &one, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
@@ -1136,49 +1137,84 @@ extern "C" int culda_create(const culda_corpus *c, const culda_params *p, culda_
 }
 
 // -------------------------------------------------------------- iterate
-extern "C" int culda_iterate(culda_ctx *ctx, int n, culda_iter_stats *stats) {
-    if (!ctx || n < 0) return fail(ctx, CULDA_ERR_INVALID_ARG, "culda_iterate: invalid argument");
-    CK(cudaSetDevice(ctx->device));
-    for (int i = 0; i < n; ++i) {
-        if (ctx->tune_pending && ctx->next_iteration >= kTuneIteration) {
+// Iterations are queued up to kQueueDepth ahead of the host, so the GPU does
+// not wait for the host to read one iteration's statistics before it starts
+// the next (30 us of a 300 us iteration at 1M tokens).  Slot i of the event
+// ring lies between iterations i-1 and i of the call.
+int run_iterations(culda_ctx *ctx, int n, culda_iter_stats *stats, bool mh, const std::function<int()> &launch) {
+    constexpr int kQueueDepth = kStatsRing / 2;
+    cudaStream_t s = ctx->stream;
+    const uint32_t first = ctx->next_iteration;
+    int launched = 0, done = 0;
+    bool fresh = true;  // nothing is queued: the next iteration's start needs an event of its own
+    auto collect = [&]() -> int {
+        CK(cudaEventSynchronize(ctx->ev_iter[(done + 1) % kStatsRing]));
+        float ms = 0.f;
+        CK(cudaEventElapsedTime(&ms, ctx->ev_iter[done % kStatsRing], ctx->ev_iter[(done + 1) % kStatsRing]));
+        const DevStats h = ctx->h_stats[(first + (uint32_t)done) % kStatsRing];
+        ctx->next_iteration = h.iteration + 1;
+        if (stats) {
+            culda_iter_stats &o = stats[done];
+            o = culda_iter_stats{};
+            o.iteration = (int32_t)h.iteration;
+            o.status = h.error;
+            o.seconds = ms * 1e-3;
+            o.loglik = mh ? NAN : (h.ll_sum - ctx->doc_term) / (double)ctx->N;
+            o.tokens_per_sec = ms > 0 ? (double)ctx->N / (ms * 1e-3) : 0.0;
+            o.row_entries = h.row_entries;
+            o.theta_nnz = h.nnz;
+            o.token_nnz = h.token_nnz;
+            o.sample_seconds = h.sample_t1 > h.sample_t0 ? (double)(h.sample_t1 - h.sample_t0) * 1e-9 : 0.0;
+            o.rebuild_seconds = h.rebuild_t1 > h.rebuild_t0 ? (double)(h.rebuild_t1 - h.rebuild_t0) * 1e-9 : 0.0;
+            o.accept_rate = h.mh_proposed ? (double)h.mh_accepted / (double)h.mh_proposed : 0.0;
+        }
+        ++done;
+        if (h.error)
+            return fail(ctx, CULDA_ERR_DEVICE_STATE, "iteration %u: device error word 0x%x", h.iteration, h.error);
+        return CULDA_OK;
+    };
+    // after a failure: whatever is queued has run, and the next iteration follows it
+    auto give_up = [&](int rc) {
+        cudaStreamSynchronize(s);
+        ctx->next_iteration = first + (uint32_t)launched;
+        return rc;
+    };
+    for (; launched < n; ++launched) {
+        if (launched - done == kQueueDepth)
+            if (const int rc = collect()) return give_up(rc);
+        if (!mh && ctx->tune_pending && first + (uint32_t)launched >= kTuneIteration) {
+            while (done < launched)
+                if (const int rc = collect()) return give_up(rc);
             ctx->tune_pending = false;
             int rc = autotune_sampler(ctx);
             if (rc) return rc;
             rc = build_graphs(ctx);
             if (rc) return rc;
+            fresh = true;
         }
-        CK(cudaEventRecord(ctx->ev0, ctx->stream));
-        if (ctx->graph[ctx->cur]) {
-            CK(cudaGraphLaunch(ctx->graph[ctx->cur], ctx->stream));
-        } else {
-            int rc = record_iteration(ctx, ctx->stream, ctx->cur);
-            if (rc) return rc;
-        }
-        CK(cudaEventRecord(ctx->ev1, ctx->stream));
-        CK(cudaEventSynchronize(ctx->ev1));
-        float ms = 0.f, ms_s = 0.f, ms_t = 0.f;
-        CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
-        CK(cudaEventElapsedTime(&ms_s, ctx->ev_s0, ctx->ev_s1));
-        CK(cudaEventElapsedTime(&ms_t, ctx->ev_t0, ctx->ev_t1));
+        if (fresh) CK(cudaEventRecord(ctx->ev_iter[launched % kStatsRing], s));
+        fresh = false;
+        if (const int rc = launch()) return give_up(rc);
         ctx->cur = 1 - ctx->cur;
-        const DevStats h = *ctx->h_stats;
-        ctx->next_iteration = h.iteration + 1;
-        if (stats) {
-            culda_iter_stats &o = stats[i];
-            o.iteration = (int32_t)h.iteration;
-            o.status = h.error;
-            o.seconds = ms * 1e-3;
-            o.loglik = (h.ll_sum - ctx->doc_term) / (double)ctx->N;
-            o.tokens_per_sec = ms > 0 ? (double)ctx->N / (ms * 1e-3) : 0.0;
-            o.row_entries = h.row_entries;
-            o.theta_nnz = h.nnz;
-            o.token_nnz = h.token_nnz;
-            o.sample_seconds = ms_s * 1e-3;
-            o.rebuild_seconds = ms_t * 1e-3;
+        const cudaError_t e = cudaEventRecord(ctx->ev_iter[(launched + 1) % kStatsRing], s);
+        if (e != cudaSuccess) {
+            ++launched;
+            return give_up(fail(ctx, CULDA_ERR_CUDA, "iteration: %s", cudaGetErrorString(e)));
         }
-        if (h.error) return fail(ctx, CULDA_ERR_DEVICE_STATE, "iteration %u: device error word 0x%x", h.iteration, h.error);
     }
+    while (done < launched)
+        if (const int rc = collect()) return give_up(rc);
     return CULDA_OK;
+}
+
+extern "C" int culda_iterate(culda_ctx *ctx, int n, culda_iter_stats *stats) {
+    if (!ctx || n < 0) return fail(ctx, CULDA_ERR_INVALID_ARG, "culda_iterate: invalid argument");
+    CK(cudaSetDevice(ctx->device));
+    return run_iterations(ctx, n, stats, false, [ctx]() -> int {
+        if (!ctx->graph[ctx->cur]) return record_iteration(ctx, ctx->stream, ctx->cur);
+        CK(cudaGraphLaunch(ctx->graph[ctx->cur], ctx->stream));
+        return CULDA_OK;
+    });
 }
 
 // Device topics in stored order -> host array in input (word-major) order.
@@ -1235,7 +1271,7 @@ extern "C" int culda_get_phi(culda_ctx *ctx, int32_t *phi, int32_t *nk) {
         cudaFree(d_nk2);
     }
     if (nk) {
-        CK(cudaMemcpyAsync(nk, ctx->d_nk, sizeof(int32_t) * (size_t)ctx->K, cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(nk, ctx->d_nk[ctx->cur], sizeof(int32_t) * (size_t)ctx->K, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
     }
     return CULDA_OK;
@@ -1274,16 +1310,10 @@ extern "C" int culda_sample_snapshot(culda_ctx *ctx, uint32_t iteration, uint16_
     CK(cudaSetDevice(ctx->device));
     cudaStream_t s = ctx->stream;
     const int cur = ctx->cur, nxt = 1 - cur;
-    CK(cudaMemsetAsync(ctx->d_counter, 0, sizeof(int32_t), s));
-    if (ctx->num_hot > 0 && !ctx->d_frozen_phi) {
-        CK(cudaMemsetAsync(ctx->d_hot_phi, 0, sizeof(int32_t) * (size_t)ctx->num_hot * ctx->K, s));
-        CK(launch_hot_rows(ctx->K, ctx->d_hot_items, ctx->num_hot_items, ctx->d_z[cur], ctx->d_hot_phi, ctx->d_error,
-                           s));
-    }
-    CK(launch_uniforms(ctx->N, ctx->params.seed, nullptr, iteration, ctx->d_tok_index, ctx->d_u, s));
+    CK(iteration_prologue(ctx, cur, true, iteration, nullptr));
     CK(launch_sample(sample_params(ctx, cur, iteration, nullptr), ctx->group_lanes, ctx->sample_blocks,
                      ctx->sample_grid, s));
-    CK(launch_finalize_ll(ctx->d_item_ll, ctx->num_items, ctx->d_stats, nullptr, s));
+    CK(launch_finalize_ll(ctx->d_item_ll, ctx->num_items, ctx->d_stats, done_counter(ctx), s));
     DevStats h{};
     int32_t e = 0;
     CK(cudaMemcpyAsync(&h, ctx->d_stats, sizeof(DevStats), cudaMemcpyDeviceToHost, s));
@@ -1317,9 +1347,9 @@ extern "C" int culda_loglik_joint(culda_ctx *ctx, double *ll) {
     p.rows = ctx->d_rows;
     p.theta = ctx->d_theta;
     p.doc_ptr = ctx->d_doc_ptr;
-    p.nk = ctx->d_nk;
+    p.nk = ctx->d_nk[ctx->cur];
     p.partials = ctx->d_partials;
-    p.done = ctx->d_counter + 32;
+    p.done = done_counter(ctx);
     p.result = &ctx->h_stats->joint;  // pinned, mapped
     p.error = ctx->d_error;
     CK(launch_loglik_joint(p, kMaxPartials, s));
@@ -1345,8 +1375,8 @@ extern "C" int culda_get_info(const culda_ctx *ctx, culda_info *info) {
     info->theta_long_docs = ctx->theta_long;
     info->theta_tune_ms = ctx->theta_tune_ms;
     info->theta_grid = ctx->theta_grid;
-    // hot_rows (when words are split), uniforms, sample, finalize_ll, theta_rebuild, copy_error
-    info->kernels_per_iteration = (ctx->num_hot > 0 ? 1 : 0) + 5;
+    // hot_rows (when words are split), prologue, sample, theta_rebuild
+    info->kernels_per_iteration = (ctx->num_hot > 0 ? 1 : 0) + 3;
     info->theta_capacity = ctx->theta_cap;
     const int64_t N = ctx->N, D = ctx->D, V = ctx->V, K = ctx->K;
     (void)N;
@@ -1387,7 +1417,9 @@ extern "C" void culda_destroy(culda_ctx *ctx) {
         }
     }
     if (ctx->h_stats) pinned_stats_put(ctx->h_stats);
-    for (cudaEvent_t ev : {ctx->ev0, ctx->ev1, ctx->ev_s0, ctx->ev_s1, ctx->ev_t0, ctx->ev_t1})
+    for (cudaEvent_t ev : {ctx->ev0, ctx->ev1})
+        if (ev) cudaEventDestroy(ev);
+    for (cudaEvent_t ev : ctx->ev_iter)
         if (ev) cudaEventDestroy(ev);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;

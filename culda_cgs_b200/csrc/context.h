@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -39,7 +40,7 @@ struct culda_ctx {
     culda::ThetaEntry *d_theta = nullptr;
     int64_t theta_cap = 0;
     int2 *d_rows = nullptr;
-    int32_t *d_nk = nullptr;
+    int32_t *d_nk[2] = {nullptr, nullptr};  // topic totals of d_z[cur] in d_nk[cur]; the rebuild fills the other
     culda_item *d_items = nullptr, *d_hot_items = nullptr;
     int32_t num_items = 0, num_hot_items = 0, num_hot = 0;
     int32_t num_long_items = 0;          // items counted by a whole CTA (long_items)
@@ -52,7 +53,7 @@ struct culda_ctx {
     uint32_t *d_iter = nullptr;
     culda::DevStats *d_stats = nullptr;
     int32_t *d_error = nullptr;
-    culda::DevStats *h_stats = nullptr;  // pinned (a slot of the process-wide pool)
+    culda::DevStats *h_stats = nullptr;  // pinned ring of kStatsRing (a slot of the process-wide pool)
     char *d_block = nullptr;             // every buffer above that culda_create allocates, in one allocation
     size_t block_bytes = 0;
     bool block_pooled = false;           // d_block came from the device's block pool (freed back to it)
@@ -67,8 +68,7 @@ struct culda_ctx {
     std::vector<int32_t> h_max_ia;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    // recorded inside the iteration graph around the sampling and rebuild kernels
-    cudaEvent_t ev_s0 = nullptr, ev_s1 = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
+    cudaEvent_t ev_iter[culda::kStatsRing] = {};  // between queued iterations
     uint32_t next_iteration = 1;
     std::string err;
 
@@ -80,7 +80,6 @@ struct culda_ctx {
     float *d_cdf = nullptr;          // [D x K] inclusive prefix sums of each doc's encoder proposal
     float *d_cdf_blk = nullptr;      // [D x K/32] the prefix at the end of every 32 topics
     float *d_probs = nullptr;        // [batch x K] encoder output scratch
-    unsigned long long *d_mh_stats = nullptr;  // accepted moves, proposals of the last MH iteration
     bool has_proposal = false;
 
     // Fold-in: word-topic counts and topic totals held fixed (from a trained
@@ -113,8 +112,18 @@ cudaError_t dalloc(T **p, size_t n) {
 // comes from the device counter when iteration_ptr is set (graph launches).
 culda::SampleParams sample_params(const culda_ctx *ctx, int cur, uint32_t iteration, const uint32_t *iteration_ptr);
 
-// Event record that becomes an event node when the stream is being captured.
-cudaError_t record_event(cudaEvent_t ev, cudaStream_t s);
+// The iteration's prologue kernel for topics d_z[cur]: counters, statistics
+// and d_nk[1-cur] cleared, hot rows cleared when they will be counted, and the
+// uniforms of `iteration` (or *iteration_ptr) formed when `uniforms` is set.
+cudaError_t iteration_prologue(culda_ctx *ctx, int cur, bool uniforms, uint32_t iteration,
+                               const uint32_t *iteration_ptr);
+// Theta and d_nk[1-cur] from the sampled topics d_z[1-cur], and the
+// iteration's statistics into the pinned ring.
+cudaError_t iteration_rebuild(culda_ctx *ctx, int cur, int num_items);
+// Runs n iterations that `launch` queues on the context's stream (each from
+// d_z[cur] to d_z[1-cur], with the two calls above), a few of them ahead of
+// the host, and fills stats.
+int run_iterations(culda_ctx *ctx, int n, culda_iter_stats *stats, bool mh, const std::function<int()> &launch);
 
 // Theta rows and n_k from the current topics d_z[cur].
 int rebuild_counts(culda_ctx *ctx);

@@ -5,11 +5,11 @@
 // Iteration data flow (all resident in HBM; tokens stored word by word, and
 // inside a word ordered by their doc's length so neighbouring tokens walk
 // theta rows of similar length):
-//   uniforms_kernel      one Philox4x32-10 uniform per token
+//   prologue_kernel      one Philox4x32-10 uniform per token, and everything the
+//                        iteration starts from zero
 //   hot_rows_kernel      full phi rows of words split over several work items
 //   sample_kernel<G>     the draw (sampler.cu)
-//   finalize_ll_kernel   fixed-order sum of the per-item log terms
-//   theta_rebuild_kernel block per long doc, warp per other doc (longest
+//   theta_rebuild_kernel fixed-order sum of the per-item log terms; block per long doc, warp per other doc (longest
 //                        first): 16-bit shared-memory histogram of the doc's
 //                        new topics (docs of at most 32 tokens: match groups
 //                        in registers), CSR compaction in ascending topic,
@@ -18,6 +18,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <numeric>
 
@@ -168,12 +169,25 @@ __device__ __forceinline__ void theta_short(int K, int d, int64_t b, int len, in
     }
 }
 
+// Sum over the CTA's threads, in a fixed order; thread 0 gets it.
+__device__ __forceinline__ double theta_block_sum(double x) {
+    __shared__ double red[kThetaWarps];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    __syncthreads();  // an earlier sum has been read
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = x;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int w = 1; w < kThetaWarps; ++w) x += red[w];
+    return x;
+}
+
 }  // namespace
 
 __global__ void __launch_bounds__(kThetaWarps * 32) theta_rebuild_kernel(
     int K, int num_docs, const int64_t *__restrict__ doc_ptr, const int32_t *__restrict__ doc_tok,
     const uint16_t *__restrict__ topics, const int32_t *__restrict__ doc_order, int num_long, int32_t *long_queue,
-    int2 *rows, ThetaEntry *theta, int32_t *nk, int64_t *stats, int32_t *error) {
+    int2 *rows, ThetaEntry *theta, int32_t *nk, int64_t *stats, int32_t *error, const IterationEnd end) {
     extern __shared__ uint32_t sm_u32[];
     __shared__ int s_next;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -183,6 +197,13 @@ __global__ void __launch_bounds__(kThetaWarps * 32) theta_rebuild_kernel(
     uint32_t *mask = cnt + cwords;
     for (int i = threadIdx.x; i < K; i += blockDim.x) nk_acc[i] = 0u;
     for (int i = lane; i < cwords + mwords; i += 32) cnt[i] = 0u;
+    double ll = 0.0;  // this CTA's share of the sampler's per-item terms, added up at the end
+    if (end.stats) {
+        if (threadIdx.x == 0) clock_start(&end.stats->rebuild_t0);
+        const int share = (end.num_items + gridDim.x - 1) / gridDim.x;
+        const int i1 = min((int)(blockIdx.x + 1) * share, end.num_items);
+        for (int i = blockIdx.x * share + threadIdx.x; i < i1; i += blockDim.x) ll += end.item_ll[i];
+    }
     __syncthreads();
 
     int64_t my_rows = 0, my_nnz = 0, my_tok_nnz = 0;
@@ -236,7 +257,42 @@ __global__ void __launch_bounds__(kThetaWarps * 32) theta_rebuild_kernel(
         atomicAdd(reinterpret_cast<unsigned long long *>(&stats[1]), (unsigned long long)my_nnz);
         atomicAdd(reinterpret_cast<unsigned long long *>(&stats[2]), (unsigned long long)my_tok_nnz);
     }
+    if (!end.stats) return;
+    ll = theta_block_sum(ll);  // barriers inside: the CTA's atomics above are issued
+    if (threadIdx.x == 0) {
+        end.partials[blockIdx.x] = ll;
+        clock_end(&end.stats->rebuild_t0);
+        __threadfence();
+        s_next = atomicAdd(end.done, 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_next) return;
+    // the last CTA: every other CTA's atomics and partials are visible
+    __threadfence();
+    ll = 0.0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) ll += __ldcg(end.partials + i);
+    // the statistics word by word, one load per thread; thread 0's fields are the sums below
+    constexpr int kWords = (int)(sizeof(DevStats) / sizeof(unsigned long long));
+    const uint32_t iter = *end.iteration_dev;
+    DevStats *out = end.ring + iter % kStatsRing;
+    unsigned long long word = 0ull;
+    if (threadIdx.x < kWords) word = __ldcg(reinterpret_cast<const unsigned long long *>(end.stats) + threadIdx.x);
+    const int32_t err = threadIdx.x == 0 ? __ldcg(error) : 0;
+    ll = theta_block_sum(ll);
+    if (threadIdx.x == 0) {
+        end.stats->ll_sum = ll;
+        out->ll_sum = ll;
+        out->error = err;
+        out->iteration = iter;
+        *end.iteration_dev = iter + 1u;
+    } else if (threadIdx.x < kWords && threadIdx.x != offsetof(DevStats, error) / sizeof(unsigned long long)) {
+        reinterpret_cast<unsigned long long *>(out)[threadIdx.x] = word;
+    }
 }
+static_assert(sizeof(DevStats) % sizeof(unsigned long long) == 0 && offsetof(DevStats, ll_sum) == 0 &&
+                  offsetof(DevStats, error) % sizeof(unsigned long long) == 0 &&
+                  offsetof(DevStats, iteration) == offsetof(DevStats, error) + sizeof(int32_t),
+              "the rebuild's last CTA copies the statistics as 64-bit words");
 
 size_t theta_smem_bytes(int k) {
     return ((size_t)k + (size_t)kThetaWarps * (size_t)((k >> 1) + (k >> 5))) * sizeof(uint32_t);
@@ -255,18 +311,18 @@ int theta_blocks_per_sm(int k) {
 cudaError_t launch_theta_rebuild(int k, int num_docs, const int64_t *doc_ptr, const int32_t *doc_tok,
                                  const uint16_t *topics, const int32_t *doc_order, int2 *rows, ThetaEntry *theta,
                                  int32_t *nk, int64_t *stats, int32_t *error, int grid, cudaStream_t s,
-                                 int num_long, int32_t *long_queue) {
+                                 int num_long, int32_t *long_queue, const IterationEnd &end) {
     if (num_long > 0 && (!doc_order || !long_queue || num_long > num_docs)) return cudaErrorInvalidValue;
     const size_t smem = theta_smem_bytes(k);
     cudaError_t e = allow_smem(reinterpret_cast<const void *>(&theta_rebuild_kernel), smem, s);
     if (e != cudaSuccess) return e;
-    if (num_long > 0) {
+    if (num_long > 0 && !end.stats) {
         e = cudaMemsetAsync(long_queue, 0, sizeof(int32_t), s);
         if (e != cudaSuccess) return e;
     }
     theta_rebuild_kernel<<<grid, kThetaWarps * 32, smem, s>>>(k, num_docs, doc_ptr, doc_tok, topics, doc_order,
                                                               num_long > 0 ? num_long : 0, long_queue, rows, theta,
-                                                              nk, stats, error);
+                                                              nk, stats, error, end);
     return cudaGetLastError();
 }
 
@@ -290,19 +346,32 @@ cudaError_t launch_init_topics(int64_t n, int k, uint64_t seed, const int32_t *t
 
 // One Philox4x32-10 block per token, computed by all threads in parallel
 // (the sampler's groups would otherwise leave most lanes idle while a
-// segment's one or two tokens draw theirs).
-__global__ void uniforms_kernel(int64_t n, uint64_t seed, const uint32_t *__restrict__ iteration_dev,
-                                uint32_t iteration, const int32_t *__restrict__ tok_index, float *u) {
-    const uint32_t iter = iteration_dev ? *iteration_dev : iteration;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint64_t t = tok_index ? (uint64_t)tok_index[i] : (uint64_t)i;
-        u[i] = uniform_from_bits(philox_token(seed, t, iter, kPurposeSample));
+// segment's one or two tokens draw theirs), after the iteration's counters,
+// totals and hot rows are cleared: one launch instead of five graph nodes.
+__global__ void __launch_bounds__(256) prologue_kernel(const PrologueParams p) {
+    const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+    if (t0 == 0) {
+        *p.counter = 0;
+        *p.theta_queue = 0;
+        *p.done = 0;
+        DevStats *st = p.stats;
+        st->row_entries = st->nnz = st->token_nnz = 0;
+        st->mh_accepted = st->mh_proposed = 0ull;
+        st->sample_t0 = st->rebuild_t0 = ~0ull;
+        st->sample_t1 = st->rebuild_t1 = 0ull;
+    }
+    if (p.nk_next)
+        for (int64_t i = t0; i < p.k; i += nt) p.nk_next[i] = 0;
+    for (int64_t i = t0; i < p.hot_n; i += nt) p.hot_phi[i] = 0;
+    const uint32_t iter = p.iteration_dev ? *p.iteration_dev : p.iteration;
+    for (int64_t i = t0; i < p.n; i += nt) {
+        const uint64_t t = p.tok_index ? (uint64_t)p.tok_index[i] : (uint64_t)i;
+        p.u[i] = uniform_from_bits(philox_token(p.seed, t, iter, kPurposeSample));
     }
 }
 
-cudaError_t launch_uniforms(int64_t n, uint64_t seed, const uint32_t *iteration_dev, uint32_t iteration,
-                            const int32_t *tok_index, float *u, cudaStream_t s) {
-    uniforms_kernel<<<grid_for(n), 256, 0, s>>>(n, seed, iteration_dev, iteration, tok_index, u);
+cudaError_t launch_prologue(const PrologueParams &p, cudaStream_t s) {
+    prologue_kernel<<<grid_for(std::max<int64_t>(std::max<int64_t>(p.n, p.hot_n), p.k)), 256, 0, s>>>(p);
     return cudaGetLastError();
 }
 
@@ -1028,7 +1097,7 @@ extern "C" int culda_sample(const culda_sample_args *a, void *d_workspace, size_
     rc = cuda_status(launch_sample(p, a->group_lanes, blocks, grid, s));
     if (rc) return rc;
     DevStats *st = (DevStats *)(counter + 8);
-    rc = cuda_status(launch_finalize_ll(item_ll, a->num_items, st, nullptr, s));
+    rc = cuda_status(launch_finalize_ll(item_ll, a->num_items, st, counter + 3, s));
     if (rc) return rc;
     return cuda_status(cudaMemcpyAsync(a->loglik_sum, &st->ll_sum, sizeof(double), cudaMemcpyDeviceToDevice, s));
 }

@@ -48,6 +48,7 @@ struct SampleParams {
     uint32_t iteration;          // used when iteration_ptr is null
     const uint32_t *iteration_ptr;
     int32_t *error;
+    unsigned long long *clock;   // {first start, last end} of the launch's CTAs (global timer), or null
 };
 
 struct DevStats {
@@ -57,7 +58,45 @@ struct DevStats {
     int64_t token_nnz;    // sum_d L_d * nnz_d after the rebuild            (stats slot 2)
     int32_t error;
     uint32_t iteration;   // Philox iteration the sampler used
+    unsigned long long mh_accepted, mh_proposed;  // Metropolis-Hastings iterations
+    // global timer (ns) at the first start and the last end of a CTA of the
+    // sampling kernel and of the rebuild
+    unsigned long long sample_t0, sample_t1, rebuild_t0, rebuild_t1;
     double joint;         // joint log-likelihood sum (written to the host copy only)
+};
+
+// What an iteration clears and forms before it samples, in one kernel.
+struct PrologueParams {
+    int64_t n;                       // tokens whose uniforms are formed (0: none)
+    uint64_t seed;
+    const uint32_t *iteration_dev;   // Philox iteration: *iteration_dev, or `iteration` when null
+    uint32_t iteration;
+    const int32_t *tok_index;
+    float *u;
+    int32_t *counter;                // the sampler's queue head, cleared
+    int32_t *theta_queue;            // the rebuild's queue head, cleared
+    int32_t *done;                   // CTAs of the rebuild finished, cleared
+    int32_t *hot_phi;                // cleared
+    int64_t hot_n;
+    int32_t *nk_next;                // topic totals the rebuild adds into, cleared (or null)
+    int32_t k;
+    DevStats *stats;                 // counts cleared, clocks set to their neutral values
+};
+cudaError_t launch_prologue(const PrologueParams &p, cudaStream_t s);
+
+// What the rebuild's last CTA does at the end of an iteration: adds up the
+// per-item log terms (each CTA has summed its share into partials) and
+// writes the iteration's statistics to slot *iteration_dev % kStatsRing of
+// the pinned ring.  stats null: nothing.
+constexpr int kStatsRing = 8;
+struct IterationEnd {
+    DevStats *stats = nullptr;
+    const double *item_ll = nullptr;
+    int32_t num_items = 0;
+    double *partials = nullptr;  // one per CTA
+    int32_t *done = nullptr;
+    uint32_t *iteration_dev = nullptr;
+    DevStats *ring = nullptr;
 };
 
 inline int pow2_ceil(int k) {
@@ -83,18 +122,19 @@ cudaError_t launch_sample(const SampleParams &p, int group_lanes, int blocks_per
 size_t theta_smem_bytes(int k);
 int theta_blocks_per_sm(int k);
 // The first num_long docs of doc_order (which must then be given) are taken
-// a whole CTA each from the queue counter long_queue (cleared by the launch);
-// the rest one warp each.
+// a whole CTA each from the queue counter long_queue (cleared by the launch,
+// or by the prologue when `end` is given); the rest one warp each.
 cudaError_t launch_theta_rebuild(int k, int num_docs, const int64_t *doc_ptr, const int32_t *doc_tok,
                                  const uint16_t *topics, const int32_t *doc_order, int2 *rows, ThetaEntry *theta,
                                  int32_t *nk, int64_t *stats, int32_t *error, int grid, cudaStream_t s,
-                                 int num_long = 0, int32_t *long_queue = nullptr);
+                                 int num_long = 0, int32_t *long_queue = nullptr,
+                                 const IterationEnd &end = IterationEnd{});
 
 cudaError_t launch_hot_rows(int k, const culda_item *hot_items, int num_hot_items, const uint16_t *topics,
                             int32_t *hot_phi, int32_t *error, cudaStream_t s);
 
-cudaError_t launch_finalize_ll(const double *item_ll, int num_items, DevStats *st, uint32_t *iteration_dev,
-                               cudaStream_t s);
+// Sum of item_ll (overwritten) into st->ll_sum; `done` must be zero.
+cudaError_t launch_finalize_ll(double *item_ll, int num_items, DevStats *st, int32_t *done, cudaStream_t s);
 
 // Flags theta rows outside the array or misaligned, and entries whose topic
 // is not below K (the kernel-level sampler checks a caller's theta with it).
@@ -103,10 +143,6 @@ cudaError_t launch_check_theta(int num_docs, int k, const int2 *rows, const Thet
 
 cudaError_t launch_init_topics(int64_t n, int k, uint64_t seed, const int32_t *tok_index, uint16_t *z,
                                cudaStream_t s);
-
-// u[i] = uniform of Philox(seed, {t_i, iteration, 0}), t_i = tok_index[i] (or i)
-cudaError_t launch_uniforms(int64_t n, uint64_t seed, const uint32_t *iteration_dev, uint32_t iteration,
-                            const int32_t *tok_index, float *u, cudaStream_t s);
 
 cudaError_t launch_update_phi(int k, int num_words, const int64_t *word_ptr, const uint16_t *topics, int32_t *phi,
                               int32_t *nk, int32_t *error, cudaStream_t s);

@@ -128,6 +128,7 @@ struct MHParams {
     int steps;
     int32_t *error;
     unsigned long long *stats;  // {accepted, proposed}
+    unsigned long long *clock;  // {first start, last end} of the launch's CTAs
 };
 
 constexpr int kMHThreads = 256;
@@ -189,6 +190,7 @@ __global__ void __launch_bounds__(kMHThreads) mh_kernel(const MHParams p) {
     const float ka = (float)K * p.alpha;
     const int nb = K >> 5;
     unsigned long long acc_n = 0, prop_n = 0;
+    if (tid == 0) clock_start(p.clock);
 
     for (int j = tid; j < K; j += blockDim.x) inv[j] = 1.0f / ((float)p.nk[j] + p.vbeta);
     for (;;) {
@@ -262,6 +264,7 @@ __global__ void __launch_bounds__(kMHThreads) mh_kernel(const MHParams p) {
             atomicAdd(&p.stats[1], prop_n);
         }
     }
+    if (tid == 0) clock_end(p.clock);
 }
 
 // Warm start: warp per token; the token's topic is drawn from
@@ -337,8 +340,6 @@ __global__ void __launch_bounds__(kMHThreads) warm_start_kernel(const MHParams p
         __syncthreads();
     }
 }
-
-__global__ void bump_iteration_kernel(uint32_t *iteration) { *iteration += 1u; }
 
 // Block per word (rows past V are zero): the word's topic profile
 // (n_wk + beta) / (n_w + K beta) in BF16, from a histogram of its tokens.
@@ -420,7 +421,7 @@ MHParams mh_params(culda_ctx *ctx, int cur, uint32_t iteration, int steps) {
     p.topics_out = ctx->d_z[1 - cur];
     p.doc_ptr = ctx->d_doc_ptr;
     p.doc_tok = ctx->d_doc_tok;
-    p.nk = ctx->d_frozen_phi ? ctx->d_frozen_nk : ctx->d_nk;
+    p.nk = ctx->d_frozen_phi ? ctx->d_frozen_nk : ctx->d_nk[cur];
     p.items = ctx->d_items;
     p.hot_phi = ctx->d_hot_phi;
     p.frozen_phi = ctx->d_frozen_phi;
@@ -432,7 +433,8 @@ MHParams mh_params(culda_ctx *ctx, int cur, uint32_t iteration, int steps) {
     p.iteration = iteration;
     p.steps = steps;
     p.error = ctx->d_error;
-    p.stats = ctx->d_mh_stats;
+    p.stats = &ctx->d_stats->mh_accepted;
+    p.clock = &ctx->d_stats->sample_t0;
     return p;
 }
 
@@ -458,21 +460,15 @@ int persistent_grid(culda_ctx *ctx, Kernel kernel, size_t smem, int *grid) {
 // Hot rows, the dense n_dk table and the MH kernel: topics d_z[cur] -> d_z[1-cur].
 int launch_mh_pass(culda_ctx *ctx, int cur, uint32_t iteration, int steps) {
     cudaStream_t s = ctx->stream;
-    if (!ctx->d_mh_stats) CK(dalloc(&ctx->d_mh_stats, 2));
-    CK(cudaMemsetAsync(ctx->d_mh_stats, 0, 2 * sizeof(unsigned long long), s));
-    CK(cudaMemsetAsync(ctx->d_counter, 0, sizeof(int32_t), s));
-    int rc = hot_rows_if_needed(ctx, cur);
-    if (rc) return rc;
-    rc = build_dense_theta(ctx);
+    CK(iteration_prologue(ctx, cur, false, iteration, nullptr));
+    int rc = build_dense_theta(ctx);
     if (rc) return rc;
     const size_t smem = 3 * (size_t)ctx->K * sizeof(float);
     int grid = 1;
     rc = persistent_grid(ctx, mh_kernel, smem, &grid);
     if (rc) return rc;
-    CK(record_event(ctx->ev_s0, s));
     mh_kernel<<<grid, kMHThreads, smem, s>>>(mh_params(ctx, cur, iteration, steps));
     CK(cudaGetLastError());
-    CK(record_event(ctx->ev_s1, s));
     return CULDA_OK;
 }
 
@@ -488,7 +484,7 @@ int check_device_error(culda_ctx *ctx, const char *what) {
 
 void free_learned_state(culda_ctx *ctx) {
     void *bufs[] = {ctx->d_doc_words, ctx->d_acc,    ctx->d_ndk,        ctx->d_cdf,        ctx->d_cdf_blk,
-                    ctx->d_probs,     ctx->d_mh_stats, ctx->frozen_borrowed ? nullptr : ctx->d_frozen_phi,
+                    ctx->d_probs,     ctx->frozen_borrowed ? nullptr : ctx->d_frozen_phi,
                     ctx->frozen_borrowed ? nullptr : ctx->d_frozen_nk};
     for (void *b : bufs)
         if (b) cudaFree(b);
@@ -499,7 +495,6 @@ void free_learned_state(culda_ctx *ctx) {
     ctx->d_cdf = nullptr;
     ctx->d_cdf_blk = nullptr;
     ctx->d_probs = nullptr;
-    ctx->d_mh_stats = nullptr;
     ctx->d_frozen_phi = nullptr;
     ctx->d_frozen_nk = nullptr;
     ctx->has_proposal = false;
@@ -683,54 +678,13 @@ extern "C" int culda_iterate_mh(culda_ctx *ctx, int32_t n, int32_t steps, culda_
     if (!ctx || n < 0 || steps < 1 || steps > 64)
         return fail(ctx, CULDA_ERR_INVALID_ARG, "culda_iterate_mh: invalid argument");
     CK(cudaSetDevice(ctx->device));
-    cudaStream_t s = ctx->stream;
-    for (int i = 0; i < n; ++i) {
-        const int cur = ctx->cur, nxt = 1 - cur;
-        const uint32_t iteration = ctx->next_iteration;
-        CK(cudaEventRecord(ctx->ev0, s));
-        int rc = launch_mh_pass(ctx, cur, iteration, steps);
+    uint32_t iteration = ctx->next_iteration;
+    return run_iterations(ctx, n, stats, true, [&]() -> int {
+        const int rc = launch_mh_pass(ctx, ctx->cur, iteration++, steps);
         if (rc) return rc;
-        CK(cudaMemsetAsync(ctx->d_nk, 0, sizeof(int32_t) * (size_t)ctx->K, s));
-        CK(cudaMemsetAsync(&ctx->d_stats->row_entries, 0, 3 * sizeof(int64_t), s));
-        CK(record_event(ctx->ev_t0, s));
-        CK(launch_theta_rebuild(ctx->K, ctx->D, ctx->d_doc_ptr, ctx->d_doc_tok, ctx->d_z[nxt], ctx->d_doc_order,
-                                ctx->d_rows, ctx->d_theta, ctx->d_nk, &ctx->d_stats->row_entries, ctx->d_error,
-                                ctx->theta_grid, s));
-        CK(record_event(ctx->ev_t1, s));
-        bump_iteration_kernel<<<1, 1, 0, s>>>(ctx->d_iter);
-        CK(cudaGetLastError());
-        CK(cudaEventRecord(ctx->ev1, s));
-        DevStats h{};
-        unsigned long long mh[2] = {0, 0};
-        int32_t err = 0;
-        CK(cudaMemcpyAsync(&h, ctx->d_stats, sizeof(DevStats), cudaMemcpyDeviceToHost, s));
-        CK(cudaMemcpyAsync(mh, ctx->d_mh_stats, sizeof(mh), cudaMemcpyDeviceToHost, s));
-        CK(cudaMemcpyAsync(&err, ctx->d_error, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        float ms = 0.f, ms_s = 0.f, ms_t = 0.f;
-        CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
-        CK(cudaEventElapsedTime(&ms_s, ctx->ev_s0, ctx->ev_s1));
-        CK(cudaEventElapsedTime(&ms_t, ctx->ev_t0, ctx->ev_t1));
-        ctx->cur = nxt;
-        ctx->next_iteration = iteration + 1;
-        if (stats) {
-            culda_iter_stats &o = stats[i];
-            o = culda_iter_stats{};
-            o.iteration = (int32_t)iteration;
-            o.status = err;
-            o.seconds = ms * 1e-3;
-            o.loglik = NAN;
-            o.tokens_per_sec = ms > 0 ? (double)ctx->N / (ms * 1e-3) : 0.0;
-            o.row_entries = h.row_entries;
-            o.theta_nnz = h.nnz;
-            o.token_nnz = h.token_nnz;
-            o.sample_seconds = ms_s * 1e-3;
-            o.rebuild_seconds = ms_t * 1e-3;
-            o.accept_rate = mh[1] ? (double)mh[0] / (double)mh[1] : 0.0;
-        }
-        if (err) return fail(ctx, CULDA_ERR_DEVICE_STATE, "culda_iterate_mh: device error 0x%x", err);
-    }
-    return CULDA_OK;
+        CK(iteration_rebuild(ctx, ctx->cur, 0));
+        return CULDA_OK;
+    });
 }
 
 extern "C" int culda_mh_snapshot(culda_ctx *ctx, uint32_t iteration, int32_t steps, uint16_t *topics_out) {

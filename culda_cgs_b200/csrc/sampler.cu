@@ -312,6 +312,7 @@ __global__ void __launch_bounds__(kSampleThreads, MINB) sample_kernel(const Samp
     float *pref = pref_all + group * Shape::kMaxSteps;
     const unsigned m = group_mask<G>(lane);
     const uint32_t iter = p.iteration_ptr ? *p.iteration_ptr : p.iteration;
+    if (tid == 0) clock_start(p.clock);
 
     for (int j = tid; j < K; j += blockDim.x) inv[j] = 1.0f / ((float)p.nk[j] + p.vbeta);
     for (int j = K + tid; j < KP; j += blockDim.x) ph[j] = 0.f;
@@ -439,6 +440,7 @@ __global__ void __launch_bounds__(kSampleThreads, MINB) sample_kernel(const Samp
             p.item_ll[it] = s;
         }
     }
+    if (tid == 0) clock_end(p.clock);
 }
 
 // ------------------------------------------------------ the flat walk
@@ -715,7 +717,10 @@ __global__ void __launch_bounds__(kSampleThreads, MINB) sample_flat_kernel(const
     const uint32_t iter = p.iteration_ptr ? *p.iteration_ptr : p.iteration;
 
     for (int j = K + tid; j < KP; j += blockDim.x) ph[j] = 0.f;
-    if (tid == 0) s_tiny = 0;
+    if (tid == 0) {
+        s_tiny = 0;
+        clock_start(p.clock);
+    }
 
     for (;;) {
         if (tid == 0) {
@@ -995,6 +1000,7 @@ __global__ void __launch_bounds__(kSampleThreads, MINB) sample_flat_kernel(const
         if (tiny && tid < s_tm)
             ph[s_tk[tid]] = (0.f + p.beta) * (1.0f / ((float)__ldg(p.nk + s_tk[tid]) + p.vbeta));
     }
+    if (tid == 0) clock_end(p.clock);
 }
 
 size_t sample_smem_bytes(int k, int group_lanes) {
@@ -1093,29 +1099,43 @@ cudaError_t launch_hot_rows(int k, const culda_item *hot_items, int num_hot_item
 }
 
 // ------------------------------------------------------------- LL finalize
-__global__ void __launch_bounds__(256) finalize_ll_kernel(const double *__restrict__ item_ll, int num_items,
-                                                          DevStats *st, uint32_t *iteration_dev) {
+// Each CTA sums a fixed share of the per-item terms into the share's first
+// element; the last CTA adds those in order.  (One CTA over all items took
+// 31 us at 100k items and 276 us at 1M.)
+constexpr int kFinalizeShare = 4096;  // items per CTA
+
+__global__ void __launch_bounds__(256) finalize_ll_kernel(double *item_ll, int num_items, DevStats *st,
+                                                          int32_t *done) {
     __shared__ double red[256];
-    double s = 0.0;
-    for (int i = threadIdx.x; i < num_items; i += 256) s += item_ll[i];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+    __shared__ bool s_last;
+    auto block_sum = [&](double x) {
+        red[threadIdx.x] = x;
         __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        st->ll_sum = red[0];
-        if (iteration_dev) {
-            st->iteration = *iteration_dev;
-            *iteration_dev += 1u;
+        for (int w = 128; w > 0; w >>= 1) {
+            if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+            __syncthreads();
         }
+    };
+    const int b = blockIdx.x * kFinalizeShare, e = min(b + kFinalizeShare, num_items);
+    double s = 0.0;
+    for (int i = b + threadIdx.x; i < e; i += 256) s += item_ll[i];
+    block_sum(s);
+    if (threadIdx.x == 0) {
+        item_ll[b] = red[0];
+        __threadfence();
+        s_last = atomicAdd(done, 1) == (int)gridDim.x - 1;
     }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    s = 0.0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += 256) s += __ldcg(item_ll + (size_t)i * kFinalizeShare);
+    block_sum(s);
+    if (threadIdx.x == 0) st->ll_sum = red[0];
 }
 
-cudaError_t launch_finalize_ll(const double *item_ll, int num_items, DevStats *st, uint32_t *iteration_dev,
-                               cudaStream_t s) {
-    finalize_ll_kernel<<<1, 256, 0, s>>>(item_ll, num_items, st, iteration_dev);
+cudaError_t launch_finalize_ll(double *item_ll, int num_items, DevStats *st, int32_t *done, cudaStream_t s) {
+    finalize_ll_kernel<<<(num_items + kFinalizeShare - 1) / kFinalizeShare, 256, 0, s>>>(item_ll, num_items, st, done);
     return cudaGetLastError();
 }
 
