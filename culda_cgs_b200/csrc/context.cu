@@ -118,6 +118,8 @@ int fail(culda_ctx *c, int code, const char *fmt, ...) {
 // Queue counter of the theta rebuild's block bin: its own 64-byte line of the
 // counter array (slot 0 is the sampler's work queue).
 static int32_t *theta_queue(culda_ctx *ctx) { return ctx->d_counter + 16; }
+// Queue head of the items that the flat walk takes a warp each.
+static int32_t *warp_queue(const culda_ctx *ctx) { return ctx->d_counter + 48; }
 // CTAs finished, for kernels whose last CTA has more to do.
 static int32_t *done_counter(culda_ctx *ctx) { return ctx->d_counter + 32; }
 
@@ -165,12 +167,16 @@ SampleParams sample_params(const culda_ctx *ctx, int cur, uint32_t iteration, co
     p.rows = ctx->d_rows;
     p.nk = ctx->d_nk[cur];
     p.items = ctx->d_items;
+    p.inv = ctx->d_inv;
     p.seg_start = ctx->d_seg_start;
+    p.seg_doc = ctx->d_seg_doc;
     p.num_segs = ctx->num_segs;
     p.hot_phi = ctx->d_hot_phi;
     p.frozen_phi = ctx->d_frozen_phi;
     if (ctx->d_frozen_phi) p.nk = ctx->d_frozen_nk;
     p.item_counter = ctx->d_counter;
+    p.first_warp = ctx->first_warp;
+    p.warp_counter = warp_queue(ctx);
     p.item_ll = ctx->d_item_ll;
     p.seed = ctx->params.seed;
     p.iteration = iteration;
@@ -190,12 +196,16 @@ cudaError_t iteration_prologue(culda_ctx *ctx, int cur, bool uniforms, uint32_t 
     p.tok_index = ctx->d_tok_index;
     p.u = ctx->d_u;
     p.counter = ctx->d_counter;
+    p.warp_counter = warp_queue(ctx);
     p.theta_queue = theta_queue(ctx);
     p.done = done_counter(ctx);
     p.hot_phi = ctx->d_hot_phi;
     p.hot_n = ctx->d_frozen_phi ? 0 : (int64_t)ctx->num_hot * ctx->K;
     p.nk_next = ctx->d_nk[1 - cur];
     p.k = ctx->K;
+    p.nk = ctx->d_frozen_phi ? ctx->d_frozen_nk : ctx->d_nk[cur];
+    p.vbeta = ctx->params.beta * (float)ctx->V;
+    p.inv = ctx->d_inv;
     p.stats = ctx->d_stats;
     cudaError_t e = launch_prologue(p, ctx->stream);
     if (e == cudaSuccess && p.hot_n > 0)
@@ -328,6 +338,7 @@ int autotune_sampler(culda_ctx *ctx) {
         float t = 0.f;
         for (int rep = 0; rep < 3; ++rep) {
             CK(cudaMemsetAsync(ctx->d_counter, 0, sizeof(int32_t), s));
+            CK(cudaMemsetAsync(warp_queue(ctx), 0, sizeof(int32_t), s));
             CK(cudaEventRecord(ctx->ev0, s));
             CK(launch_sample(sp, c[0], c[1], grid, s));
             CK(cudaEventRecord(ctx->ev1, s));
@@ -545,9 +556,12 @@ __global__ void seg_flag_kernel(int64_t n, const int32_t *__restrict__ run_start
 }
 
 __global__ void seg_scatter_kernel(int64_t n, const int32_t *__restrict__ flag, const int32_t *__restrict__ index,
-                                   int32_t *seg_start) {
+                                   const int32_t *__restrict__ doc_ids, int32_t *seg_start, int32_t *seg_doc) {
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
-        if (flag[t]) seg_start[index[t]] = (int32_t)t;
+        if (flag[t]) {
+            seg_start[index[t]] = (int32_t)t;
+            seg_doc[index[t]] = doc_ids[t];
+        }
 }
 
 __global__ void item_segments_kernel(culda_item *items, int num_items, const int32_t *__restrict__ index) {
@@ -676,7 +690,7 @@ int build_segments_device(culda_ctx *ctx, SetupArena &arena) {
         CKS(cudaMemcpyAsync(&total, B + N, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
         CKS(cudaStreamSynchronize(s));
         ctx->num_segs = total;  // d_seg_start holds one entry per token, the most there can be
-        seg_scatter_kernel<<<grid(N), 256, 0, s>>>(N, A, B, ctx->d_seg_start);
+        seg_scatter_kernel<<<grid(N), 256, 0, s>>>(N, A, B, ctx->d_doc_ids, ctx->d_seg_start, ctx->d_seg_doc);
         item_segments_kernel<<<grid(ctx->num_items), 256, 0, s>>>(ctx->d_items, ctx->num_items, B);
         CKS(cudaGetLastError());
         CKS(cudaStreamSynchronize(s));
@@ -843,6 +857,7 @@ extern "C" int culda_create(const culda_corpus *c, const culda_params *p, culda_
         ctx->num_items = (int32_t)items.size();
         ctx->num_hot = nhot;
         ctx->num_hot_items = (int32_t)hot.size();
+        ctx->first_warp = first_warp_item(items.data(), ctx->num_items);
         ctx->num_long_items = (int32_t)long_items(items.data(), (int64_t)items.size());
     }
     ctx->sample_grid = std::max(1, std::min(ctx->num_items, sms * sbps));
@@ -902,10 +917,12 @@ extern "C" int culda_create(const culda_corpus *c, const culda_params *p, culda_
         const size_t o_stats = add(sizeof(DevStats));
         const size_t o_nk0 = add(sizeof(int32_t) * (size_t)K);
         const size_t o_nk1 = add(sizeof(int32_t) * (size_t)K);
+        const size_t o_inv = add(sizeof(float) * (size_t)K);
         const size_t o_partials = add(sizeof(double) * kMaxPartials);
         // the region set-up borrows, in the order it gives the buffers back
         const size_t o_doc_tok = add(sizeof(int32_t) * (size_t)N);
         const size_t o_seg_start = add(sizeof(int32_t) * (size_t)N);  // at most one segment per token
+        const size_t o_seg_doc = add(sizeof(int32_t) * (size_t)N);
         const size_t o_z0 = add(sizeof(uint16_t) * (size_t)N);
         const size_t o_z1 = add(sizeof(uint16_t) * (size_t)N);
         const size_t o_zx = add(sizeof(uint16_t) * (size_t)N);
@@ -935,11 +952,13 @@ extern "C" int culda_create(const culda_corpus *c, const culda_params *p, culda_
         ctx->d_hot_phi = reinterpret_cast<int32_t *>(b + o_hot_phi);
         ctx->d_item_ll = reinterpret_cast<double *>(b + o_item_ll);
         ctx->d_seg_start = reinterpret_cast<int32_t *>(b + o_seg_start);
+        ctx->d_seg_doc = reinterpret_cast<int32_t *>(b + o_seg_doc);
         ctx->d_counter = reinterpret_cast<int32_t *>(b + o_counter);
         ctx->d_iter = reinterpret_cast<uint32_t *>(b + o_iter);
         ctx->d_stats = reinterpret_cast<DevStats *>(b + o_stats);
         ctx->d_nk[0] = reinterpret_cast<int32_t *>(b + o_nk0);
         ctx->d_nk[1] = reinterpret_cast<int32_t *>(b + o_nk1);
+        ctx->d_inv = reinterpret_cast<float *>(b + o_inv);
         ctx->d_partials = reinterpret_cast<double *>(b + o_partials);
         ctx->d_z[0] = reinterpret_cast<uint16_t *>(b + o_z0);
         ctx->d_z[1] = reinterpret_cast<uint16_t *>(b + o_z1);

@@ -352,6 +352,7 @@ __global__ void __launch_bounds__(256) prologue_kernel(const PrologueParams p) {
     const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
     if (t0 == 0) {
         *p.counter = 0;
+        *p.warp_counter = 0;
         *p.theta_queue = 0;
         *p.done = 0;
         DevStats *st = p.stats;
@@ -362,11 +363,15 @@ __global__ void __launch_bounds__(256) prologue_kernel(const PrologueParams p) {
     }
     if (p.nk_next)
         for (int64_t i = t0; i < p.k; i += nt) p.nk_next[i] = 0;
+    for (int64_t i = t0; i < p.k; i += nt) p.inv[i] = 1.0f / ((float)p.nk[i] + p.vbeta);
     for (int64_t i = t0; i < p.hot_n; i += nt) p.hot_phi[i] = 0;
     const uint32_t iter = p.iteration_dev ? *p.iteration_dev : p.iteration;
-    for (int64_t i = t0; i < p.n; i += nt) {
-        const uint64_t t = p.tok_index ? (uint64_t)p.tok_index[i] : (uint64_t)i;
-        p.u[i] = uniform_from_bits(philox_token(p.seed, t, iter, kPurposeSample));
+    const int32_t *__restrict__ tok_index = p.tok_index;
+    float *__restrict__ u = p.u;
+    const int64_t n = p.n;
+    for (int64_t i = t0; i < n; i += nt) {
+        const uint64_t t = tok_index ? (uint64_t)__ldg(tok_index + i) : (uint64_t)i;
+        u[i] = uniform_from_bits(philox_token(p.seed, t, iter, kPurposeSample));
     }
 }
 

@@ -36,13 +36,18 @@ struct SampleParams {
     const ThetaEntry *theta;     // CSR rows
     const int2 *rows;            // [D] {start, end}
     const int32_t *nk;           // [K]
+    const float *inv;            // [K] 1 / (n_k + V beta), or null (formed where it is used)
     const culda_item *items;     // [num_items]
     const int32_t *seg_start;    // [num_segs] first token of every segment
+    const int32_t *seg_doc;      // [num_segs] its doc, or null (read at its first token)
     int32_t num_segs;
     const int32_t *hot_phi;      // [num_hot * K]
     const int32_t *frozen_phi;   // [V * K] word-topic counts held fixed (fold-in), or null; then nk
                                  // holds the matching topic totals
     int32_t *item_counter;       // work queue head, zeroed before the launch
+    int32_t first_warp;          // items [first_warp, num_items) are small: the flat walk takes them a warp
+                                 // each (first_warp_item)
+    int32_t *warp_counter;       // their queue head, zeroed before the launch; null: all items a CTA each
     double *item_ll;             // [num_items] sum of log(S+Q) per item
     uint64_t seed;
     uint32_t iteration;          // used when iteration_ptr is null
@@ -74,12 +79,16 @@ struct PrologueParams {
     const int32_t *tok_index;
     float *u;
     int32_t *counter;                // the sampler's queue head, cleared
+    int32_t *warp_counter;           // the queue head of the items a warp takes, cleared
     int32_t *theta_queue;            // the rebuild's queue head, cleared
     int32_t *done;                   // CTAs of the rebuild finished, cleared
     int32_t *hot_phi;                // cleared
     int64_t hot_n;
     int32_t *nk_next;                // topic totals the rebuild adds into, cleared (or null)
     int32_t k;
+    const int32_t *nk;               // topic totals the iteration samples against
+    float vbeta;
+    float *inv;                      // [K] receives 1 / (n_k + V beta)
     DevStats *stats;                 // counts cleared, clocks set to their neutral values
 };
 cudaError_t launch_prologue(const PrologueParams &p, cudaStream_t s);
@@ -114,9 +123,13 @@ constexpr int kSampleBlocksDefault = 8;
 constexpr int kSampleBlocksHigh = 10;
 constexpr int kFlatBlocks = 9;
 constexpr int kFlatLanes = -1;
+// Items of at most this many tokens are sampled a warp each (sampler.cu says why here).
+constexpr int kWarpItemTokens = 32;
 size_t sample_smem_bytes(int k, int group_lanes);
 bool sample_variant_exists(int group_lanes, int blocks_per_sm);
 int sample_blocks_per_sm(int k, int group_lanes, int blocks_per_sm);
+// The first item of a work list (largest first) that the flat walk gives to a warp.
+int32_t first_warp_item(const culda_item *items, int32_t n);
 cudaError_t launch_sample(const SampleParams &p, int group_lanes, int blocks_per_sm, int grid, cudaStream_t s);
 
 size_t theta_smem_bytes(int k);

@@ -25,6 +25,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 
 #include "device_util.cuh"
 #include "kernels.cuh"
@@ -599,6 +600,7 @@ struct FlatWalk {
 // the base prefix plus the cumulative corrections alpha * (phihat_wk - base_k)
 // of its topics, applied during the search.
 constexpr int kTinyTokens = 32;
+constexpr int kTinyMinK = 512;  // at K = 256 the full build is cheaper than the patch: 16.2 against 15.7 ms per iteration
 
 // The flat walk keeps the dense bucket as one prefix per block of 8 topics
 // (K is a multiple of 32): qb[b] = alpha * sum of ph[0 .. 8 (b + 1)).  A draw
@@ -607,12 +609,10 @@ constexpr int kTinyTokens = 32;
 // of 16 KB, which lets 7 CTAs share an SM instead of 5.
 constexpr int kDenseBlock = 8;
 
-// Each thread takes a run of blocks: a block's total is the running sum a
-// draw's pass over the block forms (the same operations, so the same bits),
-// the run's prefix is compensated, and add_run_offsets completes it.
-__device__ void dense_block_prefix(const float *ph, float *qb, int K, float alpha, float *s_warp) {
-    const int T = blockDim.x, nb = K / kDenseBlock, per = (nb + T - 1) / T;
-    const int b0 = min((int)threadIdx.x * per, nb), b1 = min(b0 + per, nb);
+// The local inclusive sums of blocks [b0, b1) into qb and their total.  A
+// block's total is the running sum a draw's pass over the block forms (the
+// same operations, so the same bits); the run's prefix is compensated.
+__device__ __forceinline__ float dense_block_run(const float *ph, float *qb, int b0, int b1, float alpha) {
     float s = 0.f, c = 0.f;
     for (int b = b0; b < b1; ++b) {
         const float4 x = reinterpret_cast<const float4 *>(ph)[2 * b];
@@ -628,8 +628,51 @@ __device__ void dense_block_prefix(const float *ph, float *qb, int K, float alph
         neumaier(s, c, part);
         qb[b] = s + c;
     }
-    add_run_offsets(s + c, qb, b0, b1, s_warp);
+    return s + c;
+}
+
+// Each thread takes a run of blocks; add_run_offsets completes the prefix.
+__device__ void dense_block_prefix(const float *ph, float *qb, int K, float alpha, float *s_warp) {
+    const int T = blockDim.x, nb = K / kDenseBlock, per = (nb + T - 1) / T;
+    const int b0 = min((int)threadIdx.x * per, nb), b1 = min(b0 + per, nb);
+    const float run = dense_block_run(ph, qb, b0, b1, alpha);
+    add_run_offsets(run, qb, b0, b1, s_warp);
     __syncthreads();
+}
+
+// One warp: writes the phihat of a tiny item's topics (lane l holds the topic
+// of token l, 0xFFFFFFFF past the item) over the base row in ph, and the
+// topics in ascending order (tk, 16-byte aligned) with the running sums of
+// their corrections to the dense prefix (tdc).  m is their number; lead marks the lane that wrote a
+// topic.  Ends with a warp barrier.
+__device__ __forceinline__ void tiny_patch(const SampleParams &p, float *ph, uint32_t z, int count, int lane, int *tk,
+                                           float *tdc, int &m, bool &lead) {
+    // the item's distinct topics (match groups), their counts and ranks
+    const unsigned grp = __match_any_sync(0xffffffffu, z);
+    lead = z != 0xFFFFFFFFu && __ffs(grp) - 1 == lane;
+    const uint32_t key = lead ? z : 0xFFFFFFFFu;
+    int rank = 0;
+#pragma unroll 4
+    for (int j = 0; j < count; ++j) rank += __shfl_sync(0xffffffffu, key, j) < key;
+    m = __popc(__ballot_sync(0xffffffffu, lead));
+    if (lane >= m && lane < 8) tk[lane] = INT_MAX;  // past the topics, for the searches that read 8 at a time
+    if (lead) {
+        const float v = ((float)__popc(grp) + p.beta) * (1.0f / ((float)__ldg(p.nk + z) + p.vbeta));
+        tdc[rank] = p.alpha * v - p.alpha * ph[z];  // ph[z] holds the base value here
+        ph[z] = v;
+        tk[rank] = (int)z;
+    }
+    // the corrections in topic order, then their running sums
+    __syncwarp();
+    float dc = lane < m ? tdc[lane] : 0.f;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float t = __shfl_up_sync(0xffffffffu, dc, o);
+        if (lane >= o) dc = fsum(dc, t);
+    }
+    __syncwarp();
+    if (lane < m) tdc[lane] = dc;
+    __syncwarp();
 }
 
 // Inside block b, from the prefix `base` before it: the first topic whose
@@ -667,6 +710,12 @@ __device__ __forceinline__ int dense_search_tiny_blocks(const float *ph, const f
     auto corrected = [&](int b) {
         const int last = b * kDenseBlock + kDenseBlock - 1;
         int a = 0, e = m;  // topics of the item up to the block's end
+        if (m <= 8) {      // most items: two 16-byte loads (tk is padded) instead of a chain of them
+            const int4 x = reinterpret_cast<const int4 *>(tk)[0], y = reinterpret_cast<const int4 *>(tk)[1];
+            a = (x.x <= last) + (x.y <= last) + (x.z <= last) + (x.w <= last) + (y.x <= last) + (y.y <= last) +
+                (y.z <= last) + (y.w <= last);
+            e = a;
+        }
         while (a < e) {
             const int c = (a + e) >> 1;
             if (tk[c] <= last)
@@ -700,7 +749,7 @@ __global__ void __launch_bounds__(kSampleThreads, MINB) sample_flat_kernel(const
     __shared__ double s_red[kSampleThreads / 32];
     // tiny items: whether ph / qb hold the base row, and the item's topics
     __shared__ int s_tiny, s_tm;
-    __shared__ int s_tk[kTinyTokens];
+    __shared__ __align__(16) int s_tk[kTinyTokens];
     __shared__ float s_tdc[kTinyTokens];
     __shared__ float s_tQ;
 
@@ -715,6 +764,8 @@ __global__ void __launch_bounds__(kSampleThreads, MINB) sample_flat_kernel(const
     float *m_S = reinterpret_cast<float *>(m_t0 + kFlatSegs);  // [n] S of the row
     float *m_lg = m_S + kFlatSegs;                               // [n] log(S + Q)
     const uint32_t iter = p.iteration_ptr ? *p.iteration_ptr : p.iteration;
+    // sample_warp_kernel, launched behind this kernel, may take the SMs' free room from now on
+    asm volatile("griddepcontrol.launch_dependents;");
 
     for (int j = K + tid; j < KP; j += blockDim.x) ph[j] = 0.f;
     if (tid == 0) {
@@ -743,8 +794,7 @@ __global__ void __launch_bounds__(kSampleThreads, MINB) sample_flat_kernel(const
         }
 
         // phi row of the word
-        // (at K = 256 the full build is cheaper than the patch: 16.2 against 15.7 ms per iteration)
-        const bool tiny = K >= 512 && !p.frozen_phi && item.hot < 0 && item.count <= kTinyTokens;
+        const bool tiny = K >= kTinyMinK && !p.frozen_phi && item.hot < 0 && item.count <= kTinyTokens;
         float Q;
         if (tiny) {
             if (!s_tiny) {  // the base row and its dense prefix, once per CTA
@@ -755,7 +805,6 @@ __global__ void __launch_bounds__(kSampleThreads, MINB) sample_flat_kernel(const
                 if (tid == 0) s_tiny = 1;
             }
             if (warp == 0) {
-                // the item's distinct topics (match groups), their counts and ranks
                 uint32_t z = 0xFFFFFFFFu;
                 if (lane < (int)item.count) {
                     z = p.topics_in[ibeg + lane];
@@ -764,35 +813,12 @@ __global__ void __launch_bounds__(kSampleThreads, MINB) sample_flat_kernel(const
                         z = 0xFFFFFFFFu;
                     }
                 }
-                const unsigned grp = __match_any_sync(0xffffffffu, z);
-                const bool lead = z != 0xFFFFFFFFu && __ffs(grp) - 1 == lane;
-                const uint32_t key = lead ? z : 0xFFFFFFFFu;
-                int rank = 0;
-#pragma unroll 8
-                for (int j = 0; j < 32; ++j) rank += __shfl_sync(0xffffffffu, key, j) < key;
-                const int m = __popc(__ballot_sync(0xffffffffu, lead));
-                float d = 0.f;
-                if (lead) {
-                    const float v = ((float)__popc(grp) + p.beta) * (1.0f / ((float)__ldg(p.nk + z) + p.vbeta));
-                    d = p.alpha * v - p.alpha * ph[z];  // ph[z] holds the base value here
-                    ph[z] = v;
-                    s_tk[rank] = (int)z;
-                    s_tdc[rank] = d;
-                }
-                // the corrections in topic order, then their running sums
-                __syncwarp();
-                float dc = lane < m ? s_tdc[lane] : 0.f;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const float t = __shfl_up_sync(0xffffffffu, dc, o);
-                    if (lane >= o) dc = fsum(dc, t);
-                }
-                __syncwarp();
-                if (lane < m) s_tdc[lane] = dc;
-                const float total = __shfl_sync(0xffffffffu, dc, m > 0 ? m - 1 : 0);
+                int m;
+                bool lead;
+                tiny_patch(p, ph, z, item.count, lane, s_tk, s_tdc, m, lead);
                 if (lane == 0) {
                     s_tm = m;
-                    s_tQ = fsum(qb[K / kDenseBlock - 1], m > 0 ? total : 0.f);
+                    s_tQ = fsum(qb[K / kDenseBlock - 1], m > 0 ? s_tdc[m - 1] : 0.f);
                 }
             }
             __syncthreads();
@@ -816,11 +842,10 @@ __global__ void __launch_bounds__(kSampleThreads, MINB) sample_flat_kernel(const
             } else {
                 src = p.hot_phi + (size_t)item.hot * K;
             }
-            // 1 / (n_k + V beta) is formed per item (the same operations, so the
-            // same bits, as a table would hold), which keeps the table's 4 KB
-            // out of each CTA's shared memory
+            // 1 / (n_k + V beta) comes from the iteration's table (through the L1,
+            // not 4 KB of each CTA's shared memory) or, with the same bits, from n_k
             for (int j = tid; j < K; j += blockDim.x)
-                ph[j] = ((float)src[j] + p.beta) * (1.0f / ((float)__ldg(p.nk + j) + p.vbeta));
+                ph[j] = ((float)src[j] + p.beta) * (p.inv ? __ldg(p.inv + j) : 1.0f / ((float)__ldg(p.nk + j) + p.vbeta));
             __syncthreads();
             dense_block_prefix(ph, qb, K, p.alpha, s_warp);
             Q = qb[K / kDenseBlock - 1];
@@ -846,11 +871,12 @@ __global__ void __launch_bounds__(kSampleThreads, MINB) sample_flat_kernel(const
             if (lane < nseg) {
                 const int sg = seg0 + lane;
                 const int64_t a0 = __ldg(p.seg_start + sg);
+                int d = p.seg_doc ? __ldg(p.seg_doc + sg) : -1;  // beside the start, not after it
                 const int64_t a1 = sg + 1 < sg_end ? (int64_t)__ldg(p.seg_start + sg + 1) : iend;
                 if (a0 < ibeg || a1 > iend || a0 >= a1) {
                     atomicOr(p.error, kErrRowRange);
                 } else {
-                    const int d = __ldg(p.doc_ids + a0);
+                    if (!p.seg_doc) d = __ldg(p.doc_ids + a0);
                     if ((unsigned)d < (unsigned)p.num_docs) {
                         const int2 r = __ldg(p.rows + d);
                         if (r.x >= 0 && r.x <= r.y && (int64_t)r.y <= p.theta_cap && ((r.x | r.y) & 31) == 0 &&
@@ -1003,6 +1029,447 @@ __global__ void __launch_bounds__(kSampleThreads, MINB) sample_flat_kernel(const
     if (tid == 0) clock_end(p.clock);
 }
 
+// The shared-memory arrays of one warp of the flat walk.
+struct FlatWarp {
+    const float *ph;  // [K] phihat of the word
+    const float *qb;  // [K / 8] dense-bucket prefix at the end of every 8-topic block
+    float *ub;        // [B] unit prefixes of the batch
+    int *m_cum;       // [n+1] first unit of each segment of the batch
+    int *m_tc;        // [n+1] first token (flat)
+    int *m_rs;        // [n] row start (entry index)
+    int *m_t0;        // [n] first token
+    float *m_S;       // [n] S of the row
+    float *m_lg;      // [n] log(S + Q)
+
+    __device__ __forceinline__ FlatWarp(const float *ph_, const float *qb_, float *ub_, int *meta)
+        : ph(ph_), qb(qb_), ub(ub_), m_cum(meta), m_tc(m_cum + (kFlatSegs + 1)), m_rs(m_tc + (kFlatSegs + 1)),
+          m_t0(m_rs + kFlatSegs), m_S(reinterpret_cast<float *>(m_t0 + kFlatSegs)), m_lg(m_S + kFlatSegs) {}
+};
+
+// A segment's theta row (start, units) and tokens; all zero past its item.
+struct SegMeta {
+    int rs, nu, t0, tcount;
+};
+
+// Its first and last token (plus one) and its doc, before the row is looked up.
+struct SegTokens {
+    int64_t a0, a1;
+    int d;
+};
+
+__device__ __forceinline__ SegTokens load_tokens(const SampleParams &p, bool valid, int sg, int sg_end, int64_t iend) {
+    SegTokens t{0, 0, -1};
+    if (!valid) return t;
+    t.a0 = __ldg(p.seg_start + sg);
+    t.a1 = sg + 1 < sg_end ? (int64_t)__ldg(p.seg_start + sg + 1) : iend;
+    if (p.seg_doc) t.d = __ldg(p.seg_doc + sg);  // beside the start, not after it
+    return t;
+}
+
+__device__ __forceinline__ SegMeta load_row(const SampleParams &p, bool valid, SegTokens t, int64_t ibeg, int64_t iend,
+                                            int B) {
+    SegMeta m{0, 0, 0, 0};
+    if (!valid) return m;
+    if (t.a0 < ibeg || t.a1 > iend || t.a0 >= t.a1) {
+        atomicOr(p.error, kErrRowRange);
+        return m;
+    }
+    if (!p.seg_doc) t.d = __ldg(p.doc_ids + t.a0);
+    if ((unsigned)t.d >= (unsigned)p.num_docs) {
+        atomicOr(p.error, kErrDocRange);
+        return m;
+    }
+    const int2 r = __ldg(p.rows + t.d);
+    if (r.x >= 0 && r.x <= r.y && (int64_t)r.y <= p.theta_cap && ((r.x | r.y) & 31) == 0 && r.y - r.x <= kUnit * B)
+        m = SegMeta{r.x, (r.y - r.x) / kUnit, (int)t.a0, (int)(t.a1 - t.a0)};
+    else
+        atomicOr(p.error, kErrRowRange);
+    return m;
+}
+
+__device__ __forceinline__ SegMeta load_segment(const SampleParams &p, bool valid, int sg, int sg_end, int64_t ibeg,
+                                                int64_t iend, int B) {
+    return load_row(p, valid, load_tokens(p, valid, sg, sg_end, iend), ibeg, iend, B);
+}
+
+// One walk group's range [gb, ge) of units, of a batch of n segments: every
+// unit's running prefix inside its row into w.ub (short of what enters the
+// range), the sum of the last row in gv, whether a row starts in the range in
+// gflag, and in lead_end the end of the units before that start.  sp is the
+// segment of unit gb.
+__device__ __forceinline__ void walk_range(const SampleParams &p, const FlatWarp &w, int sp, int gb, int ge, int wl,
+                                           unsigned wm, float &gv, int &gflag, int &lead_end) {
+    FlatWalk k{p.theta, w.ph, w.ub, w.m_cum, w.m_rs, ge, wl, wm, sp, w.m_cum[sp + 1], w.m_cum[sp], w.m_rs[sp], gb,
+               0.f, 0.f, 0};
+    k.gflag = gb == k.rowu;
+    lead_end = k.gflag ? gb : min(k.nxt, ge);
+    Step a = load_unit(p.theta, k.rbase + kUnit * (gb + wl - k.rowu)), b;
+    while (k.step(a, b) && k.step(b, a)) {
+    }
+    gflag = k.gflag;
+    gv = k.s + k.c;
+}
+
+// The segment and the token that lane f of a batch of n segments draws, and
+// its uniform.
+struct DrawToken {
+    int i, tok;
+    float um;
+};
+
+__device__ __forceinline__ DrawToken draw_token(const SampleParams &p, const FlatWarp &w, int n, int f, uint32_t iter) {
+    DrawToken t;
+    t.i = last_le(w.m_tc, n, f);
+    t.tok = w.m_t0[t.i] + (f - w.m_tc[t.i]);
+    if (p.uniforms) {
+        t.um = __ldg(p.uniforms + t.tok);
+    } else {
+        const int64_t key = p.tok_index ? (int64_t)__ldg(p.tok_index + t.tok) : (int64_t)t.tok;
+        t.um = uniform_from_bits(philox_token(p.seed, (uint64_t)key, iter, kPurposeSample));
+    }
+    return t;
+}
+
+// Draws one token of a walked batch; adds its log term to ll.
+__device__ __forceinline__ void draw_one(const SampleParams &p, const FlatWarp &w, const DrawToken &t, float Q,
+                                         bool tiny, const int *tk, const float *tdc, int tm, double &ll) {
+    const int K = p.k, i = t.i;
+    const float S = w.m_S[i];
+    const float T = t.um * (S + Q);
+    int z;
+    if (T < S) {
+        const int c0 = w.m_cum[i];
+        int lo = c0, hi = w.m_cum[i + 1] - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (w.ub[mid] > T)
+                hi = mid;
+            else
+                lo = mid + 1;
+        }
+        const float prev = lo > c0 ? w.ub[lo - 1] : 0.f;
+        z = resolve_unit(load_unit(p.theta, w.m_rs[i] + kUnit * (lo - c0)), prev, T, w.ph);
+        // a unit of the row's padding: T lies within a rounding of the
+        // prefix where that unit starts (a lane's carried-in sum can round
+        // one unit in the last place above the previous unit's prefix)
+        if (z < 0) z = row_last_nonzero(p.theta, w.m_rs[i], w.m_rs[i] + kUnit * (w.m_cum[i + 1] - c0));
+    } else {
+        z = tiny ? dense_search_tiny_blocks(w.ph, w.qb, K, p.alpha, T - S, tk, tdc, tm)
+                 : dense_search_blocks(w.ph, w.qb, K, p.alpha, T - S);
+    }
+    if (z < 0) {
+        atomicOr(p.error, kErrRowRange);
+        z = 0;
+    }
+    p.topics_out[t.tok] = (uint16_t)z;
+    ll += (double)w.m_lg[i];
+}
+
+// Draws the total_t tokens of a walked batch of n segments, one per lane: lane
+// f takes tokens f, f + 32, ...  Adds their log terms to ll.
+__device__ __forceinline__ void draw_batch(const SampleParams &p, const FlatWarp &w, int n, int total_t, float Q,
+                                           bool tiny, const int *tk, const float *tdc, int tm, uint32_t iter,
+                                           double &ll) {
+    for (int f = threadIdx.x & 31; f < total_t; f += 32)
+        draw_one(p, w, draw_token(p, w, n, f, iter), Q, tiny, tk, tdc, tm, ll);
+}
+
+// The batch's segments [0, n) (lane `first` + i holds segment i, incl and tincl
+// the inclusive sums of units and tokens from lane `first`) into the warp's
+// arrays; ends with a warp barrier.
+__device__ __forceinline__ void store_batch(const FlatWarp &w, const SegMeta &seg, int lane, int first, int last,
+                                            int incl, int tincl) {
+    if (lane >= first && lane <= last) {
+        const int i = lane - first;
+        w.m_cum[i] = incl - seg.nu;
+        w.m_tc[i] = tincl - seg.tcount;
+        w.m_rs[i] = seg.rs;
+        w.m_t0[i] = seg.t0;
+        if (lane == last) {
+            w.m_cum[i + 1] = incl;
+            w.m_tc[i + 1] = tincl;
+        }
+    }
+    __syncwarp();
+}
+
+// S and log(S + Q) of the walked batch's segments, one per lane; ends with a
+// warp barrier.
+__device__ __forceinline__ void store_sums(const FlatWarp &w, int i, int n, float Q) {
+    if (i >= 0 && i < n) {
+        const int c0 = w.m_cum[i], c1 = w.m_cum[i + 1];
+        const float S = c1 > c0 ? w.ub[c1 - 1] : 0.f;
+        w.m_S[i] = S;
+        w.m_lg[i] = logf(S + Q);
+    }
+    __syncwarp();
+}
+
+// Units per group range of a batch of total_u units: odd, so the 8 groups'
+// prefix stores hit distinct banks.
+__device__ __forceinline__ int range_steps(int total_u) { return ((total_u + 31) >> 5) | 1; }
+
+// A warp's own items: walks and draws n segments, held from lane `first` on,
+// as one batch that joins up to kJoinedParts parts of `part` segments.  A part
+// is what flat_batches walks at a time (a chunk, or as much of it as fits the
+// budget), and its units are cut into the same ranges, so every prefix has the
+// same bits; but the ranges of all parts share the 8 walk groups, and their
+// tokens one round of draws.  A small item's chunks are a few segments each:
+// one after the other they leave most lanes idle.
+constexpr int kJoinedParts = 4;
+
+struct JoinScratch {
+    float gv[32];
+    int lead[32], range[32];
+};
+
+__device__ __forceinline__ void joined_parts(const SampleParams &p, const FlatWarp &w, const SegMeta &seg, int first,
+                                             int n, int part, int incl, float Q, bool tiny, const int *tk,
+                                             const float *tdc, int tm, uint32_t iter, JoinScratch &js, double &ll) {
+    const int lane = threadIdx.x & 31;
+    const int wl = lane & (kWalkLanes - 1), wg = lane / kWalkLanes;
+    const unsigned wm = group_mask<kWalkLanes>(lane);
+    constexpr int G = 32 / kWalkLanes;  // ranges per part
+    const bool mine_seg = lane >= first && lane < first + n;
+    const int tincl = warp_incl_scan(mine_seg ? seg.tcount : 0, lane);
+    const int total_t = __shfl_sync(0xffffffffu, tincl, first + n - 1);
+    store_batch(w, seg, lane, first, first + n - 1, incl, tincl);
+    // the first round's uniforms are on their way during the walk
+    DrawToken mine{0, 0, 0.f};
+    if (lane < total_t) mine = draw_token(p, w, n, lane, iter);
+    // lane 8c + g stands for range g of part c
+    const int c = lane / G, g = lane % G;
+    const int u0 = w.m_cum[min(c * part, n)], u1 = w.m_cum[min((c + 1) * part, n)];
+    const int r = range_steps(u1 - u0);
+    const int gb = min(u0 + g * 4 * r, u1), ge = min(gb + 4 * r, u1);
+    // the non-empty ranges in a list: bounds (at most 512), first segment and place packed
+    const unsigned full = __ballot_sync(0xffffffffu, gb < ge);
+    const int ranges = __popc(full);
+    if (gb < ge) {
+        const int sp = last_le(w.m_cum, n, gb);
+        js.range[__popc(full & ((1u << lane) - 1u))] = gb | ge << 10 | sp << 20 | lane << 25;
+    }
+    __syncwarp();
+    for (int t = wg; t < ranges; t += G) {
+        const int x = js.range[t];
+        float gv;
+        int gflag, lead_end;
+        walk_range(p, w, (x >> 20) & 31, x & 1023, (x >> 10) & 1023, wl, wm, gv, gflag, lead_end);
+        if (wl == 0) {
+            js.gv[x >> 25] = gv;
+            js.lead[x >> 25] = lead_end << 1 | gflag;
+        }
+    }
+    __syncwarp();
+    const float my_v = gb < ge ? js.gv[lane] : 0.f;
+    const int my_flag = gb < ge ? js.lead[lane] & 1 : 0;
+    // the segmented scan over a part's ranges, as flat_batches makes it
+    double vd = (double)my_v;
+    int fl = my_flag;
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1) {
+        const double vo = __shfl_up_sync(0xffffffffu, vd, o, G);
+        const int fo = __shfl_up_sync(0xffffffffu, fl, o, G);
+        if (g >= o && !fl) {
+            vd += vo;
+            fl = fo;
+        }
+    }
+    double carry = __shfl_up_sync(0xffffffffu, vd, 1, G);
+    if (g == 0) carry = 0.0;
+    js.gv[lane] = (float)carry;  // a lane reads and rewrites its own place only
+    __syncwarp();
+    for (int t = wg; t < ranges; t += G) {
+        const int x = js.range[t], end = js.lead[x >> 25] >> 1;
+        const float cf = js.gv[x >> 25];
+        for (int u = (x & 1023) + wl; u < end; u += kWalkLanes) w.ub[u] = fsum(w.ub[u], cf);
+    }
+    __syncwarp();
+    store_sums(w, lane, n, Q);
+    for (int f = lane; f < total_t; f += 32) {
+        if (f >= 32) mine = draw_token(p, w, n, f, iter);
+        draw_one(p, w, mine, Q, tiny, tk, tdc, tm, ll);
+    }
+    __syncwarp();  // the batch's shared data is read before the next one is written
+}
+
+// ------------------------------------------------------ a warp per item
+// Items of at most kWarpItemTokens tokens, a warp (a CTA of 32 threads) each.
+// Such an item is a chain of dependent loads (queue, item, topics, segments,
+// rows, theta) around little walking.  A CTA of four warps with nine barriers
+// per item kept 9 items in flight per SM and gave each chunk of two or three
+// segments a round of draws of its own; here an SM holds as many items as fit
+// its registers and shared memory (20 at K = 1024, 16 at K = 2048), the next
+// item's loads are issued during the current one, and the chunks are walked
+// and drawn together.  Chunks, parts and every sum are those of
+// sample_flat_kernel, so an item's draws do not depend on which kernel takes
+// it.  A million words on 23.7M tokens at K = 2048 (957k of them this small,
+// 20% of the tokens): 7.28 -> 4.97 ms for the two kernels; 1M tokens at K =
+// 1024: 178 -> 136 us.  Limits of 64 and 128 tokens are no better (5.13 and
+// 5.18 ms; 140 and 144 us; 5.62 -> 5.63 and 5.75 ms at 61M tokens): past 32
+// tokens an item fills the CTA's four warps.  92 registers: held to 80 the build
+// spills (6.1 ms), at 122 it loses warps at K = 1024 (141 against 139 us).
+static_assert(kWarpItemTokens <= 32, "a lane holds a token and a segment of the item");
+
+// dense_block_prefix as its 128 threads compute it, by one warp: four rounds
+// of 32 runs, the same sums in the same order.
+__device__ __forceinline__ void dense_block_prefix_warp(const float *ph, float *qb, int K, float alpha, int lane) {
+    const int nb = K / kDenseBlock, per = (nb + kSampleThreads - 1) / kSampleThreads;
+    float tot[kSampleThreads / 32];
+#pragma unroll
+    for (int v = 0; v < kSampleThreads / 32; ++v) {
+        const int b0 = min((v * 32 + lane) * per, nb), b1 = min(b0 + per, nb);
+        const float run = dense_block_run(ph, qb, b0, b1, alpha);
+        float incl = run;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        float ex = __shfl_up_sync(0xffffffffu, incl, 1);
+        if (lane == 0) ex = 0.f;
+        tot[v] = __shfl_sync(0xffffffffu, incl, 31);
+        // the scan over the four warps' totals, step by step as add_run_offsets makes it
+        const float before = v == 0 ? 0.f : v == 1 ? tot[0] : v == 2 ? tot[1] + tot[0] : (tot[2] + tot[1]) + tot[0];
+        const float base = before + ex;
+        for (int j = b0; j < b1; ++j) qb[j] = base + qb[j];
+    }
+    __syncwarp();
+}
+
+__global__ void __launch_bounds__(32, 20) sample_warp_kernel(const SampleParams p, int first_item) {
+    extern __shared__ __align__(16) float smem_w[];
+    const int K = p.k, B = flat_unit_budget(K), lane = threadIdx.x;
+    float *ph = smem_w;             // [K] phihat of the item's word (the histogram before that)
+    float *qb = smem_w + K;         // [K / 8] dense-bucket prefix
+    const FlatWarp w(ph, qb, qb + K / kDenseBlock, reinterpret_cast<int *>(qb + K / kDenseBlock + B));
+    __shared__ __align__(16) int s_tk[kTinyTokens];
+    __shared__ float s_tdc[kTinyTokens];
+    __shared__ JoinScratch js;
+    const uint32_t iter = p.iteration_ptr ? *p.iteration_ptr : p.iteration;
+    if (lane == 0) clock_start(p.clock);
+    auto inverse = [&](int j) { return 1.0f / ((float)__ldg(p.nk + j) + p.vbeta); };
+    bool base_row = false;  // ph and qb hold the row of a word without tokens
+    auto claim = [&]() {
+        int it = 0;
+        if (lane == 0) it = first_item + atomicAdd(p.warp_counter, 1);
+        return __shfl_sync(0xffffffffu, it, 0);
+    };
+    auto in_list = [&](const culda_item &x) {
+        return x.begin >= 0 && x.count >= 0 && x.begin + x.count <= p.num_tokens && x.hot < p.num_hot &&
+               x.seg_begin >= 0 && x.seg_count >= 0 && (int64_t)x.seg_begin + x.seg_count <= p.num_segs &&
+               x.count <= kWarpItemTokens && x.seg_count <= x.count;
+    };
+    // what an item's first loads bring, issued while the item before it is drawn
+    auto load_first = [&](const culda_item &x) {
+        return load_tokens(p, lane < x.seg_count, x.seg_begin + lane, x.seg_begin + x.seg_count, x.begin + x.count);
+    };
+    int it = claim();
+    culda_item item{};
+    SegTokens tokens{0, 0, -1};
+    uint32_t z = 0u;
+    bool ok = false;
+    if (it < p.num_items) {
+        item = p.items[it];
+        ok = in_list(item);
+        if (ok) {
+            tokens = load_first(item);
+            if (lane < item.count) z = p.topics_in[item.begin + lane];
+        }
+    }
+    while (it < p.num_items) {
+        if (!ok && lane == 0) {
+            atomicOr(p.error, kErrRowRange);
+            p.item_ll[it] = 0.0;
+        }
+        const int next = claim();  // its latency passes under this item
+        const int64_t ibeg = item.begin, iend = item.begin + item.count;
+        const int held = ok ? item.seg_count : 0;
+        const int cs = max(1, (held + kFlatWarps - 1) / kFlatWarps);  // chunks of a quarter of the segments
+        const bool tiny = ok && K >= kTinyMinK && !p.frozen_phi && item.hot < 0 && item.count <= kTinyTokens;
+        const SegMeta seg = load_row(p, lane < held, tokens, ibeg, iend, B);
+        float Q = 0.f;
+        int tm = 0, tz = 0;
+        bool lead = false;
+        if (tiny) {
+            if (lane >= item.count) z = 0xFFFFFFFFu;
+            if (lane < item.count && z >= (uint32_t)K) {
+                atomicOr(p.error, kErrTopicRange);
+                z = 0xFFFFFFFFu;
+            }
+            if (!base_row) {
+                for (int j = lane; j < K; j += 32) ph[j] = (0.f + p.beta) * inverse(j);
+                __syncwarp();
+                dense_block_prefix_warp(ph, qb, K, p.alpha, lane);
+                base_row = true;
+            }
+            tiny_patch(p, ph, z, item.count, lane, s_tk, s_tdc, tm, lead);
+            tz = (int)z;
+            Q = fsum(qb[K / kDenseBlock - 1], tm > 0 ? s_tdc[tm - 1] : 0.f);
+        } else if (ok) {
+            const int *src = item.hot >= 0 ? p.hot_phi + (size_t)item.hot * K : reinterpret_cast<const int *>(ph);
+            if (p.frozen_phi) {
+                src = p.frozen_phi + (size_t)item.word * K;
+            } else if (item.hot < 0) {
+                int *hist = reinterpret_cast<int *>(ph);
+                for (int j = lane; j < K / 4; j += 32) reinterpret_cast<int4 *>(hist)[j] = make_int4(0, 0, 0, 0);
+                __syncwarp();
+                if (lane < item.count) {
+                    if (z < (uint32_t)K)
+                        atomicAdd(&hist[z], 1);
+                    else
+                        atomicOr(p.error, kErrTopicRange);
+                }
+                __syncwarp();
+            }
+            for (int j = lane; j < K; j += 32)
+                ph[j] = ((float)src[j] + p.beta) * (p.inv ? __ldg(p.inv + j) : inverse(j));
+            __syncwarp();
+            dense_block_prefix_warp(ph, qb, K, p.alpha, lane);
+            Q = qb[K / kDenseBlock - 1];
+            base_row = false;
+        }
+        const bool more = next < p.num_items;
+        culda_item nitem{};
+        if (more) nitem = p.items[next];
+
+        double ll = 0.0;
+        for (int lo = 0; lo < held;) {
+            // the part: the rest of lo's chunk, or its longest run of segments within the budget
+            const int chunk_end = min(lo / cs * cs + cs, held);
+            const bool act = lane >= lo && lane < held;
+            const int incl = warp_incl_scan(act ? seg.nu : 0, lane);
+            const unsigned fits = __ballot_sync(0xffffffffu, act && incl <= B);
+            int hi = min(32 - __clz(fits), chunk_end), part = hi - lo;  // lane lo always fits: nu <= B
+            // whole chunks go together while they fit
+            if (hi == chunk_end && lo % cs == 0) {
+                part = cs;
+                while (hi < held && hi - lo < kJoinedParts * cs && ((fits >> (min(hi + cs, held) - 1)) & 1u))
+                    hi = min(hi + cs, held);
+            }
+            joined_parts(p, w, seg, lo, hi - lo, part, incl, Q, tiny, s_tk, s_tdc, tm, iter, js, ll);
+            lo = hi;
+        }
+        const bool was_ok = ok;
+        ok = more && in_list(nitem);
+        if (ok) {
+            tokens = load_first(nitem);
+            z = lane < nitem.count ? (uint32_t)p.topics_in[nitem.begin + lane] : 0u;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ll += __shfl_down_sync(0xffffffffu, ll, o);
+        if (lane == 0 && was_ok) p.item_ll[it] = ll;
+        // a tiny item's topics back to the base row
+        if (tiny && lead) ph[tz] = (0.f + p.beta) * inverse(tz);
+        __syncwarp();
+        it = next;
+        item = nitem;
+    }
+    if (lane == 0) clock_end(p.clock);
+    // a kernel behind this one waits for this one only: do not end before sample_flat_kernel has
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 size_t sample_smem_bytes(int k, int group_lanes) {
     if (group_lanes == kFlatLanes)  // ph[pow2(K)] + qb[K/8] + per warp: unit prefixes and segment data
         return ((size_t)k / kDenseBlock + (size_t)pow2_ceil(k) + (size_t)kFlatWarps * flat_unit_budget(k) +
@@ -1055,14 +1522,52 @@ int sample_blocks_per_sm(int k, int group_lanes, int blocks_per_sm) {
     return n;
 }
 
+static size_t sample_warp_smem_bytes(int k) {
+    return ((size_t)k + (size_t)k / kDenseBlock + (size_t)flat_unit_budget(k) + (size_t)kFlatMeta) * sizeof(float);
+}
+
+int32_t first_warp_item(const culda_item *items, int32_t n) {
+    return (int32_t)(std::partition_point(items, items + n,
+                                          [](const culda_item &x) { return x.count > kWarpItemTokens; }) -
+                     items);
+}
+
 cudaError_t launch_sample(const SampleParams &p, int group_lanes, int blocks_per_sm, int grid, cudaStream_t s) {
     const size_t smem = sample_smem_bytes(p.k, group_lanes);
-    void *args[] = {const_cast<SampleParams *>(&p)};
     const void *fn = sample_kernel_for(group_lanes, blocks_per_sm);
     if (!fn) return cudaErrorInvalidValue;
     cudaError_t e = allow_smem(fn, smem, s);
     if (e != cudaSuccess) return e;
-    return cudaLaunchKernel(fn, dim3(grid), dim3(kSampleThreads), args, smem, s);
+    SampleParams head = p;
+    const int first = group_lanes == kFlatLanes && p.warp_counter ? std::min(p.first_warp, p.num_items) : p.num_items;
+    head.num_items = first;
+    if (first > 0) {
+        void *args[] = {&head};
+        e = cudaLaunchKernel(fn, dim3(std::min(grid, first)), dim3(kSampleThreads), args, smem, s);
+        if (e != cudaSuccess || first == p.num_items) return e;
+    }
+    // the small items: their CTAs start on what room the first kernel leaves
+    // and take over as its CTAs run out of items (neither reads what the other
+    // writes)
+    const size_t wsmem = sample_warp_smem_bytes(p.k);
+    const void *wfn = reinterpret_cast<const void *>(&sample_warp_kernel);
+    e = allow_smem(wfn, wsmem, s);
+    if (e != cudaSuccess) return e;
+    int dev = 0, bps = 0;
+    cudaGetDevice(&dev);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, wfn, 32, wsmem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(std::min(p.num_items - first, num_sms(dev) * std::max(bps, 1)));
+    cfg.blockDim = dim3(32);
+    cfg.dynamicSmemBytes = wsmem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = first > 0 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, sample_warp_kernel, p, first);
 }
 
 // ----------------------------------------------------------- hot-word rows
