@@ -989,7 +989,7 @@ extern "C" int culda_create(const culda_corpus *c, const culda_params *p, culda_
     // corpus upload
     CKB(cudaMemcpyAsync(ctx->d_word_ptr, c->word_ptr, sizeof(int64_t) * ((size_t)V + 1), cudaMemcpyHostToDevice, s));
     CKB(cudaMemcpyAsync(ctx->d_doc_ptr, c->doc_ptr, sizeof(int64_t) * ((size_t)D + 1), cudaMemcpyHostToDevice, s));
-    CKB(cudaMemcpyAsync(ctx->d_doc_ids, c->doc_ids, sizeof(int32_t) * (size_t)N, cudaMemcpyHostToDevice, s));
+    CKB(copy_to_device(ctx->d_doc_ids, c->doc_ids, sizeof(int32_t) * (size_t)N, s));
     CKB(cudaMemsetAsync(ctx->d_error, 0, 64 * sizeof(int32_t), s));
     // docs longest first for the theta rebuild's warps: a counting sort on
     // the length (below 65536), stable in doc id, on the host while the
@@ -1243,8 +1243,7 @@ int topics_to_host(culda_ctx *ctx, const uint16_t *d_src, uint16_t *host) {
         CK(launch_scatter<uint16_t>(ctx->N, ctx->d_tok_index, d_src, ctx->d_zx, s));
         d_src = ctx->d_zx;
     }
-    CK(cudaMemcpyAsync(host, d_src, sizeof(uint16_t) * (size_t)ctx->N, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+    CK(copy_to_host(host, d_src, sizeof(uint16_t) * (size_t)ctx->N, s));
     return CULDA_OK;
 }
 
@@ -1252,7 +1251,7 @@ extern "C" int culda_set_topics(culda_ctx *ctx, const uint16_t *topics) {
     if (!ctx || !topics) return fail(ctx, CULDA_ERR_INVALID_ARG, "culda_set_topics: null argument");
     CK(cudaSetDevice(ctx->device));
     cudaStream_t s = ctx->stream;
-    CK(cudaMemcpyAsync(ctx->d_zx, topics, sizeof(uint16_t) * (size_t)ctx->N, cudaMemcpyHostToDevice, s));
+    CK(copy_to_device(ctx->d_zx, topics, sizeof(uint16_t) * (size_t)ctx->N, s));
     int32_t *flag = ctx->d_error + 32;  // a spare word of the error buffer
     CK(cudaMemsetAsync(flag, 0, sizeof(int32_t), s));
     CK(launch_check_topics(ctx->N, ctx->K, ctx->d_zx, flag, s));
@@ -1284,8 +1283,7 @@ extern "C" int culda_get_phi(culda_ctx *ctx, int32_t *phi, int32_t *nk) {
         CK(dalloc(&d_nk2, (size_t)ctx->K));
         CK(cudaMemsetAsync(d_nk2, 0, sizeof(int32_t) * (size_t)ctx->K, s));
         CK(launch_update_phi(ctx->K, ctx->V, ctx->d_word_ptr, ctx->d_z[ctx->cur], d_phi, d_nk2, ctx->d_error, s));
-        CK(cudaMemcpyAsync(phi, d_phi, sizeof(int32_t) * (size_t)ctx->V * ctx->K, cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
+        CK(copy_to_host(phi, d_phi, sizeof(int32_t) * (size_t)ctx->V * ctx->K, s));
         cudaFree(d_phi);
         cudaFree(d_nk2);
     }
@@ -1480,6 +1478,7 @@ extern "C" int culda_trim_memory(int32_t device) {
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= 0) return CULDA_ERR_NO_DEVICE;
     if (device < 0 || device >= ndev) return CULDA_ERR_INVALID_ARG;
+    release_staging(device);
     cudaMemPool_t pool = nullptr;
     {
         std::lock_guard<std::mutex> lock(g_pool_mu);

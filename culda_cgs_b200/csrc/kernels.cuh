@@ -205,4 +205,13 @@ cudaError_t launch_check_topics(int64_t n, int k, const uint16_t *z, int32_t *er
 
 int num_sms(int device);
 
+// Copies between the host and the current device on stream s, through pinned
+// staging when the host memory is pageable and the copy is large (staging.cu).
+// copy_to_host returns when dst holds the bytes; copy_to_device when src has
+// been read (a pinned src: when the copy is queued, as cudaMemcpyAsync).
+cudaError_t copy_to_host(void *dst, const void *src, size_t bytes, cudaStream_t s);
+cudaError_t copy_to_device(void *dst, const void *src, size_t bytes, cudaStream_t s);
+// Frees the device's idle staging memory.
+void release_staging(int device);
+
 }  // namespace culda

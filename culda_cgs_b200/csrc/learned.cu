@@ -728,7 +728,8 @@ extern "C" int culda_set_frozen_phi(culda_ctx *ctx, const int32_t *phi, const in
                         (long long)sum[(size_t)k]);
     if (!ctx->d_frozen_phi) CK(dalloc(&ctx->d_frozen_phi, n));
     if (!ctx->d_frozen_nk) CK(dalloc(&ctx->d_frozen_nk, (size_t)ctx->K));
-    CK(cudaMemcpy(ctx->d_frozen_phi, phi, sizeof(int32_t) * n, cudaMemcpyHostToDevice));
+    CK(copy_to_device(ctx->d_frozen_phi, phi, sizeof(int32_t) * n, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
     CK(cudaMemcpy(ctx->d_frozen_nk, nk, sizeof(int32_t) * (size_t)ctx->K, cudaMemcpyHostToDevice));
     return build_graphs(ctx);
 }

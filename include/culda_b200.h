@@ -307,7 +307,9 @@ const char *culda_last_error(const culda_ctx *ctx);
 void culda_destroy(culda_ctx *ctx);
 
 /* Returns the pool's unused reserve on `device` to the driver (memory that
- * live contexts hold is untouched).  No reference counterpart. */
+ * live contexts hold is untouched), and the idle pinned memory that large
+ * copies from and to pageable host arrays pass through (at most 32 MB).  No
+ * reference counterpart. */
 int culda_trim_memory(int32_t device);
 
 /* ------------------------------------------------------------- kernel level */
