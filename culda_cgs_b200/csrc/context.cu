@@ -119,7 +119,7 @@ int fail(culda_ctx *c, int code, const char *fmt, ...) {
 // counter array (slot 0 is the sampler's work queue).
 static int32_t *theta_queue(culda_ctx *ctx) { return ctx->d_counter + 16; }
 // Queue head of the items that the flat walk takes a warp each.
-static int32_t *warp_queue(const culda_ctx *ctx) { return ctx->d_counter + 48; }
+int32_t *warp_queue(const culda_ctx *ctx) { return ctx->d_counter + 48; }
 // CTAs finished, for kernels whose last CTA has more to do.
 static int32_t *done_counter(culda_ctx *ctx) { return ctx->d_counter + 32; }
 
@@ -858,6 +858,9 @@ extern "C" int culda_create(const culda_corpus *c, const culda_params *p, culda_
         ctx->num_hot = nhot;
         ctx->num_hot_items = (int32_t)hot.size();
         ctx->first_warp = first_warp_item(items.data(), ctx->num_items);
+        ctx->num_mh_coop = (int32_t)(std::partition_point(items.begin(), items.end(),
+                                                          [](const culda_item &x) { return x.count >= kMHCoop; }) -
+                                     items.begin());
         ctx->num_long_items = (int32_t)long_items(items.data(), (int64_t)items.size());
     }
     ctx->sample_grid = std::max(1, std::min(ctx->num_items, sms * sbps));

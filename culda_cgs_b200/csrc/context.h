@@ -43,6 +43,7 @@ struct culda_ctx {
     int32_t *d_nk[2] = {nullptr, nullptr};  // topic totals of d_z[cur] in d_nk[cur]; the rebuild fills the other
     culda_item *d_items = nullptr, *d_hot_items = nullptr;
     int32_t num_items = 0, num_hot_items = 0, num_hot = 0;
+    int32_t num_mh_coop = 0;             // items whose MH steps a whole CTA runs
     int32_t num_long_items = 0;          // items counted by a whole CTA (long_items)
     double *d_partials = nullptr;        // [kMaxPartials] per-CTA sums of the reductions
     int32_t *d_seg_start = nullptr;  // first stored token of every segment
@@ -79,6 +80,7 @@ struct culda_ctx {
     int32_t *d_doc_words = nullptr;  // word id of every token in doc order (the doc_ptr CSR)
     float *d_acc = nullptr;          // [D x K] topic counts summed over the accumulated states
     int32_t n_acc = 0;               // states accumulated into d_acc
+    int2 *d_doc_span = nullptr;      // {first token, length} of every doc
     uint16_t *d_ndk = nullptr;       // [D x K] dense doc-topic counts of the current state
     float *d_cdf = nullptr;          // [D x K] inclusive prefix sums of each doc's encoder proposal
     float *d_cdf_blk = nullptr;      // [D x K/32] the prefix at the end of every 32 topics
@@ -114,6 +116,12 @@ cudaError_t dalloc(T **p, size_t n) {
 // Sampler parameters for topics d_z[cur] -> d_z[1-cur]; the Philox iteration
 // comes from the device counter when iteration_ptr is set (graph launches).
 culda::SampleParams sample_params(const culda_ctx *ctx, int cur, uint32_t iteration, const uint32_t *iteration_ptr);
+
+// Queue head of the items that a warp takes (cleared by the prologue).
+int32_t *warp_queue(const culda_ctx *ctx);
+// Items of at least this many tokens take a CTA in the MH kernel (351 us at 6M
+// tokens with 256 and with 512, 355 with 128; a warp on 512 tokens is the longer tail).
+constexpr int kMHCoop = 256;
 
 // The iteration's prologue kernel for topics d_z[cur]: counters, statistics
 // and d_nk[1-cur] cleared, hot rows cleared when they will be counted, and the

@@ -6,11 +6,11 @@
 // for new documents, and the encoder warm start of their topics.
 //
 // MH iteration (one launch per kernel, not graph-captured):
-//   memset(work counter, hot rows) -> hot_rows -> dense n_dk table from the
-//   theta CSR -> mh_kernel(z[c] -> z[1-c]) -> theta rebuild (as plain CGS).
-// mh_kernel reuses the sampler's work items: per item the word's phihat row is
-// built in shared memory from a histogram of the snapshot topics (or the hot
-// row, or the frozen counts), then one thread per token runs `steps` steps:
+//   prologue -> hot_rows -> dense n_dk table from the theta CSR (when a proposal
+//   is set) -> mh_kernel(z[c] -> z[1-c]) -> theta rebuild (as plain CGS).
+// mh_kernel reuses the sampler's work items: per item the word's counts come
+// from a histogram of the snapshot topics (or the hot row, or the frozen
+// counts), then a lane per token runs `steps` steps:
 //   doc step     k' ~ (n_dk + alpha): with probability L_d / (L_d + K alpha)
 //                the topic of a uniformly chosen token of the doc, else a
 //                uniform topic; accept with min(1, phihat_wk' / phihat_ws).
@@ -113,10 +113,12 @@ struct MHParams {
     const int32_t *tok_index;  // stored -> input index (Philox key), or null
     const uint16_t *topics_in;
     uint16_t *topics_out;
-    const int64_t *doc_ptr;
+    const int2 *doc_span;      // {first token, length} of every doc
     const int32_t *doc_tok;
     const int32_t *nk;
     const culda_item *items;
+    int num_coop;              // items [0, num_coop) take a CTA each, the others a warp
+    int32_t *warp_counter;     // queue head of the others
     const int32_t *hot_phi;
     const int32_t *frozen_phi;  // [V x K] fixed counts (fold-in) or null
     int32_t *item_counter;
@@ -179,79 +181,197 @@ __device__ __forceinline__ bool item_ok(const MHParams &p, const culda_item &ite
            item.word >= 0;
 }
 
-__global__ void __launch_bounds__(kMHThreads) mh_kernel(const MHParams p) {
+// ------------------------------------------------- Metropolis-Hastings steps
+// A token's steps are random reads behind one another (its document's span, a
+// token of it, that token's topic, the proposal's tables, n_dk), so the kernel
+// is bound by their latency (L1 at 36%, issue at 21% when a step followed the
+// other in program order: 561 us for two steps at 6M tokens and K = 512).  No
+// proposal depends on where the chain stands: the two of a pair of steps are
+// formed together, their reads in flight beside one another and beside those
+// of the next 32 tokens, and only the acceptances follow one another.  Words of
+// fewer than kMHCoop tokens take a warp each with the counts in 16 bits (phihat
+// is formed where it is read); a CTA per word left most lanes idle on them.
+// 351 us.  62 registers, 32 warps per SM: 363 us at 72 registers and 24 warps,
+// 413 us at 48 (spills); reading each search's 128-byte stretch with eight
+// lanes and probing comparison bits instead of memory takes 32 registers more
+// and was slower (497 us): the probes after the first hit the L1.
+constexpr int kMHStepThreads = 128;
+constexpr int kMHWarps = kMHStepThreads / 32;
+
+// A token before its steps: topic, document (-1: none), Philox key, the
+// document's first token and length.
+struct MHToken {
+    int s, d;
+    uint64_t key;
+    int2 span;
+};
+
+__device__ __forceinline__ MHToken mh_load(const MHParams &p, bool valid, int64_t t) {
+    MHToken x{0, -1, 0, make_int2(0, 1)};
+    if (!valid) return x;
+    x.s = p.topics_in[t];
+    x.d = p.doc_ids[t];
+    x.key = p.tok_index ? (uint64_t)__ldg(p.tok_index + t) : (uint64_t)t;
+    if ((unsigned)x.d >= (unsigned)p.num_docs || (unsigned)x.s >= (unsigned)p.k) {
+        atomicOr(p.error, kErrDocRange);
+        p.topics_out[t] = (uint16_t)min(max(x.s, 0), p.k - 1);
+        return MHToken{0, -1, 0, make_int2(0, 1)};
+    }
+    x.span = __ldg(p.doc_span + x.d);
+    return x;
+}
+
+// A doc proposal: a token of the document (its index in word order, else -1)
+// or, without one, the topic.
+__device__ __forceinline__ int doc_proposal(const MHParams &p, const MHToken &tok, const u32x4 &x, float ka, int &kp) {
+    const float L = (float)tok.span.y;
+    kp = (int)bounded_from_bits(x.y, (uint32_t)p.k);
+    if (tok.d >= 0 && uniform_from_bits(x.x) * (L + ka) < L)
+        return __ldg(p.doc_tok + tok.span.x + (int)bounded_from_bits(x.y, (uint32_t)tok.span.y));
+    return -1;
+}
+
+// The steps of up to 32 tokens, lane l's at t, against the word's phihat.  The
+// whole warp takes part.
+template <class PhiHat>
+__device__ __forceinline__ void mh_tokens(const MHParams &p, const MHToken &tok, int64_t t, const PhiHat &ph, int lane,
+                                          unsigned &acc_n, unsigned &prop_n) {
+    const int K = p.k, nb = K >> 5;
+    const float ka = (float)K * p.alpha;
+    const bool active = tok.d >= 0;
+    const int d = max(tok.d, 0);
+    int s = tok.s;
+    for (int step = 0; step < p.steps; step += 2) {
+        const bool two = step + 1 < p.steps, enc = two && p.cdf;
+        const u32x4 x0 = philox_token4(p.seed, tok.key, p.iteration, kPurposeMH + (uint32_t)step);
+        const u32x4 x1 = philox_token4(p.seed, tok.key, p.iteration, kPurposeMH + (uint32_t)step + 1u);
+        // both proposals: first what they read first, then what that leads to
+        int k0, k1 = 0, i1 = -1;
+        const int i0 = doc_proposal(p, tok, x0, ka, k0);
+        const float *blk = p.blk + (size_t)d * nb, *row = p.cdf + (size_t)d * K;
+        float total = 0.f;
+        if (enc)
+            total = __ldg(blk + nb - 1);
+        else if (two)
+            i1 = doc_proposal(p, tok, x1, ka, k1);
+        if (i0 >= 0) k0 = p.topics_in[i0];
+        if (i1 >= 0) k1 = p.topics_in[i1];
+        if (enc) {
+            const float T = uniform_from_bits(x1.y) * total;
+            k1 = first_above(row, 32 * first_above(blk, 0, nb, T), 32, T);
+        }
+        // the first acceptance
+        auto accept = [&](int k, float ratio, uint32_t bits) {
+            ++prop_n;
+            if (k != s && uniform_from_bits(bits) < ratio) {
+                s = k;
+                ++acc_n;
+            }
+        };
+        if (active) {
+            if ((unsigned)k0 >= (unsigned)K) k0 = s;
+            accept(k0, ph(k0) / ph(s), x0.z);
+        }
+        if (enc) {
+            const uint16_t *nd = p.ndk + (size_t)d * K;
+            const float at_s = __ldg(row + s), before_s = s > 0 ? __ldg(row + s - 1) : 0.f;
+            const float n_s = (float)nd[s];
+            const float qk = __ldg(row + k1) - (k1 > 0 ? __ldg(row + k1 - 1) : 0.f);
+            const float qs = at_s - before_s;
+            if (active) {
+                const float pk = ((float)nd[k1] + p.alpha) * ph(k1);
+                const float ps = (n_s + p.alpha) * ph(s);
+                accept(k1, (pk * qs) / (ps * qk), x1.z);
+            }
+        } else if (two && active) {
+            if ((unsigned)k1 >= (unsigned)K) k1 = s;
+            accept(k1, ph(k1) / ph(s), x1.z);
+        }
+    }
+    if (active) p.topics_out[t] = (uint16_t)s;
+}
+
+// Tokens [begin, end) of an item, 32 at a time `stride` apart, the next 32
+// loaded ahead.
+template <class PhiHat>
+__device__ __forceinline__ void mh_run(const MHParams &p, int64_t begin, int64_t end, int stride, const PhiHat &ph,
+                                       int lane, unsigned &acc_n, unsigned &prop_n) {
+    MHToken tok = mh_load(p, begin + lane < end, begin + lane);
+    for (int64_t t0 = begin; t0 < end; t0 += stride) {
+        const int64_t tn = t0 + stride + lane;
+        const MHToken next = mh_load(p, tn < end, tn);
+        mh_tokens(p, tok, t0 + lane, ph, lane, acc_n, prop_n);
+        tok = next;
+    }
+}
+
+__global__ void __launch_bounds__(kMHStepThreads, 8) mh_kernel(const MHParams p) {
     extern __shared__ float sm_mh[];
     const int K = p.k;
-    float *ph = sm_mh;                                   // [K]
-    float *inv = sm_mh + K;                              // [K]
-    int *hist = reinterpret_cast<int *>(sm_mh + 2 * K);  // [K]
+    float *inv = sm_mh;                              // [K] 1 / (n_k + V beta)
+    float *ph = sm_mh + K;                           // [K] phihat of the CTA's word (its histogram before that)
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint32_t *cnt = reinterpret_cast<uint32_t *>(sm_mh + 2 * K) + warp * (K / 2);  // the warp's word, 16-bit counts
     __shared__ int s_item;
-    const int tid = threadIdx.x;
-    const float ka = (float)K * p.alpha;
-    const int nb = K >> 5;
-    unsigned long long acc_n = 0, prop_n = 0;
+    unsigned acc_n = 0, prop_n = 0;
     if (tid == 0) clock_start(p.clock);
 
     for (int j = tid; j < K; j += blockDim.x) inv[j] = 1.0f / ((float)p.nk[j] + p.vbeta);
+    for (int j = lane; j < K / 2; j += 32) cnt[j] = 0u;
+    // the long items: a CTA each
     for (;;) {
         if (tid == 0) s_item = atomicAdd(p.item_counter, 1);
         __syncthreads();
         const int it = s_item;
-        if (it >= p.num_items) break;
+        if (it >= p.num_coop) break;
         const culda_item item = p.items[it];
         if (!item_ok(p, item)) {
             if (tid == 0) atomicOr(p.error, kErrRowRange);
             __syncthreads();
             continue;
         }
-        item_phi_row(p, item, ph, inv, hist);
+        item_phi_row(p, item, ph, inv, reinterpret_cast<int *>(ph));
         const int64_t iend = item.begin + item.count;
-        for (int64_t t = item.begin + tid; t < iend; t += blockDim.x) {
-            int s = p.topics_in[t];
-            const int d = p.doc_ids[t];
-            if ((unsigned)d >= (unsigned)p.num_docs || (unsigned)s >= (unsigned)K) {
-                atomicOr(p.error, kErrDocRange);
-                p.topics_out[t] = (uint16_t)min(max(s, 0), K - 1);
-                continue;
-            }
-            const uint64_t key = p.tok_index ? (uint64_t)__ldg(p.tok_index + t) : (uint64_t)t;
-            const int64_t d0 = p.doc_ptr[d];
-            const int L = (int)(p.doc_ptr[d + 1] - d0);
-            const uint16_t *nd = p.ndk + (size_t)d * K;
-            for (int step = 0; step < p.steps; ++step) {
-                const u32x4 x = philox_token4(p.seed, key, p.iteration, kPurposeMH + (uint32_t)step);
-                int kp;
-                float ratio;
-                if (!(p.cdf && (step & 1))) {  // doc proposal
-                    if (uniform_from_bits(x.x) * ((float)L + ka) < (float)L) {
-                        const int i = (int)bounded_from_bits(x.y, (uint32_t)L);
-                        kp = p.topics_in[p.doc_tok[d0 + i]];
-                        if ((unsigned)kp >= (unsigned)K) kp = s;
-                    } else {
-                        kp = (int)bounded_from_bits(x.y, (uint32_t)K);
-                    }
-                    ratio = ph[kp] / ph[s];
-                } else {  // encoder proposal
-                    const float *row = p.cdf + (size_t)d * K;
-                    const float total = __ldg(p.blk + (size_t)d * nb + nb - 1);
-                    const float T = uniform_from_bits(x.y) * total;
-                    const int b = first_above(p.blk + (size_t)d * nb, 0, nb, T);
-                    kp = first_above(row, 32 * b, 32, T);
-                    const float qk = __ldg(row + kp) - (kp > 0 ? __ldg(row + kp - 1) : 0.f);
-                    const float qs = __ldg(row + s) - (s > 0 ? __ldg(row + s - 1) : 0.f);
-                    const float pk = ((float)nd[kp] + p.alpha) * ph[kp];
-                    const float ps = ((float)nd[s] + p.alpha) * ph[s];
-                    ratio = (pk * qs) / (ps * qk);
-                }
-                ++prop_n;
-                if (kp != s && uniform_from_bits(x.z) < ratio) {
-                    s = kp;
-                    ++acc_n;
-                }
-            }
-            p.topics_out[t] = (uint16_t)s;
+        mh_run(p, item.begin + 32 * warp, iend, kMHStepThreads, [ph](int k) { return ph[k]; }, lane, acc_n, prop_n);
+        __syncthreads();  // ph is rebuilt for the next item
+    }
+    // the others: a warp each
+    for (;;) {
+        int it = 0;
+        if (lane == 0) it = p.num_coop + atomicAdd(p.warp_counter, 1);
+        it = __shfl_sync(0xffffffffu, it, 0);
+        if (it >= p.num_items) break;
+        const culda_item item = p.items[it];
+        if (!item_ok(p, item)) {
+            if (lane == 0) atomicOr(p.error, kErrRowRange);
+            continue;
         }
-        __syncthreads();  // ph / hist are rebuilt for the next item
+        const int64_t iend = item.begin + item.count;
+        const int32_t *fixed = p.frozen_phi ? p.frozen_phi + (size_t)item.word * K
+                               : item.hot >= 0 ? p.hot_phi + (size_t)item.hot * K : nullptr;
+        if (fixed) {
+            auto phihat = [&](int k) { return ((float)__ldg(fixed + k) + p.beta) * inv[k]; };
+            mh_run(p, item.begin, iend, 32, phihat, lane, acc_n, prop_n);
+            continue;
+        }
+        for (int64_t t = item.begin + lane; t < iend; t += 32) {
+            const uint32_t z = p.topics_in[t];
+            if (z < (uint32_t)K)
+                atomicAdd(&cnt[z >> 1], 1u << ((z & 1u) << 4));
+            else
+                atomicOr(p.error, kErrTopicRange);
+        }
+        __syncwarp();
+        auto phihat = [&](int k) {
+            return ((float)((cnt[k >> 1] >> ((k & 1) << 4)) & 0xFFFFu) + p.beta) * inv[k];
+        };
+        mh_run(p, item.begin, iend, 32, phihat, lane, acc_n, prop_n);
+        __syncwarp();
+        for (int64_t t = item.begin + lane; t < iend; t += 32) {
+            const uint32_t z = p.topics_in[t];
+            if (z < (uint32_t)K) cnt[z >> 1] = 0u;
+        }
+        __syncwarp();
     }
     if (p.stats) {
 #pragma unroll
@@ -259,12 +379,18 @@ __global__ void __launch_bounds__(kMHThreads) mh_kernel(const MHParams p) {
             acc_n += __shfl_xor_sync(0xffffffffu, acc_n, o);
             prop_n += __shfl_xor_sync(0xffffffffu, prop_n, o);
         }
-        if ((tid & 31) == 0 && prop_n) {
-            atomicAdd(&p.stats[0], acc_n);
-            atomicAdd(&p.stats[1], prop_n);
+        if (lane == 0 && prop_n) {
+            atomicAdd(&p.stats[0], (unsigned long long)acc_n);
+            atomicAdd(&p.stats[1], (unsigned long long)prop_n);
         }
     }
     if (tid == 0) clock_end(p.clock);
+}
+
+// {first token, length} of every document (tokens are below 2^31).
+__global__ void doc_span_kernel(int D, const int64_t *__restrict__ doc_ptr, int2 *span) {
+    for (int d = blockIdx.x * blockDim.x + threadIdx.x; d < D; d += gridDim.x * blockDim.x)
+        span[d] = make_int2((int)doc_ptr[d], (int)(doc_ptr[d + 1] - doc_ptr[d]));
 }
 
 // Warm start: warp per token; the token's topic is drawn from
@@ -419,7 +545,9 @@ MHParams mh_params(culda_ctx *ctx, int cur, uint32_t iteration, int steps) {
     p.tok_index = ctx->d_tok_index;
     p.topics_in = ctx->d_z[cur];
     p.topics_out = ctx->d_z[1 - cur];
-    p.doc_ptr = ctx->d_doc_ptr;
+    p.doc_span = ctx->d_doc_span;
+    p.num_coop = ctx->num_mh_coop;
+    p.warp_counter = warp_queue(ctx);
     p.doc_tok = ctx->d_doc_tok;
     p.nk = ctx->d_frozen_phi ? ctx->d_frozen_nk : ctx->d_nk[cur];
     p.items = ctx->d_items;
@@ -449,10 +577,10 @@ int hot_rows_if_needed(culda_ctx *ctx, int cur) {
 }
 
 template <class Kernel>
-int persistent_grid(culda_ctx *ctx, Kernel kernel, size_t smem, int *grid) {
+int persistent_grid(culda_ctx *ctx, Kernel kernel, int threads, size_t smem, int *grid) {
     CK(allow_smem(reinterpret_cast<const void *>(kernel), smem, ctx->stream));
     int bps = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kernel, kMHThreads, smem));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kernel, threads, smem));
     *grid = std::max(1, std::min(ctx->num_items, num_sms(ctx->device) * std::max(bps, 1)));
     return CULDA_OK;
 }
@@ -461,13 +589,19 @@ int persistent_grid(culda_ctx *ctx, Kernel kernel, size_t smem, int *grid) {
 int launch_mh_pass(culda_ctx *ctx, int cur, uint32_t iteration, int steps) {
     cudaStream_t s = ctx->stream;
     CK(iteration_prologue(ctx, cur, false, iteration, nullptr));
-    int rc = build_dense_theta(ctx);
+    int rc = CULDA_OK;
+    if (ctx->has_proposal) rc = build_dense_theta(ctx);  // the doc proposal reads no n_dk
     if (rc) return rc;
-    const size_t smem = 3 * (size_t)ctx->K * sizeof(float);
+    if (!ctx->d_doc_span) {
+        CK(dalloc(&ctx->d_doc_span, (size_t)ctx->D));
+        doc_span_kernel<<<grid_for(ctx->D), 256, 0, s>>>(ctx->D, ctx->d_doc_ptr, ctx->d_doc_span);
+        CK(cudaGetLastError());
+    }
+    const size_t smem = ((size_t)2 * ctx->K + (size_t)kMHWarps * (size_t)(ctx->K / 2)) * sizeof(float);
     int grid = 1;
-    rc = persistent_grid(ctx, mh_kernel, smem, &grid);
+    rc = persistent_grid(ctx, mh_kernel, kMHStepThreads, smem, &grid);
     if (rc) return rc;
-    mh_kernel<<<grid, kMHThreads, smem, s>>>(mh_params(ctx, cur, iteration, steps));
+    mh_kernel<<<grid, kMHStepThreads, smem, s>>>(mh_params(ctx, cur, iteration, steps));
     CK(cudaGetLastError());
     return CULDA_OK;
 }
@@ -484,7 +618,7 @@ int check_device_error(culda_ctx *ctx, const char *what) {
 
 void free_learned_state(culda_ctx *ctx) {
     void *bufs[] = {ctx->d_doc_words, ctx->d_acc,    ctx->d_ndk,        ctx->d_cdf,        ctx->d_cdf_blk,
-                    ctx->d_probs,     ctx->frozen_borrowed ? nullptr : ctx->d_frozen_phi,
+                    ctx->d_doc_span,  ctx->d_probs,     ctx->frozen_borrowed ? nullptr : ctx->d_frozen_phi,
                     ctx->frozen_borrowed ? nullptr : ctx->d_frozen_nk};
     for (void *b : bufs)
         if (b) cudaFree(b);
@@ -492,6 +626,7 @@ void free_learned_state(culda_ctx *ctx) {
     ctx->d_doc_words = nullptr;
     ctx->d_acc = nullptr;
     ctx->d_ndk = nullptr;
+    ctx->d_doc_span = nullptr;
     ctx->d_cdf = nullptr;
     ctx->d_cdf_blk = nullptr;
     ctx->d_probs = nullptr;
@@ -745,7 +880,7 @@ extern "C" int culda_warm_start(culda_ctx *ctx) {
     if (rc) return rc;
     const size_t smem = 3 * (size_t)ctx->K * sizeof(float);
     int grid = 1;
-    rc = persistent_grid(ctx, warm_start_kernel, smem, &grid);
+    rc = persistent_grid(ctx, warm_start_kernel, kMHThreads, smem, &grid);
     if (rc) return rc;
     warm_start_kernel<<<grid, kMHThreads, smem, s>>>(mh_params(ctx, cur, 0u, 0));
     CK(cudaGetLastError());
