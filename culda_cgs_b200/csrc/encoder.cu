@@ -79,16 +79,37 @@ __device__ __forceinline__ void unpack8(const uint4 &v, float f[8]) {
     for (int i = 0; i < 8; ++i) f[i] = __bfloat162float(h[i]);
 }
 
-// Warp per batch row; lane l owns embedding columns 8l .. 8l+7.
+// 16 bytes from global to shared memory, asynchronously (zeros when !valid).
+__device__ __forceinline__ void copy16_async(void *dst, const void *src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                     static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+                 "l"(src), "r"(valid ? 16 : 0)
+                 : "memory");
+}
+
+// One CTA per batch row: its 8 warps take contiguous eighths of the document's
+// tokens, then the partial sums are added in warp order.  Lane l owns columns
+// 8l .. 8l+7.  The 512-byte rows come from all over the L2, so what counts is
+// how many are in flight: each warp keeps kBagRows of them on their way into a
+// ring in shared memory (a lane reads only the bytes it copied itself, so the
+// ring needs no barrier), 196 KB per SM.  For 4000 documents of 204 tokens (the
+// longest 3200), 418 MB of rows: 134 us with 8 rows in registers at 91
+// registers and 16 warps per SM, 98 us with 8 at 64 registers, 81 us with 16
+// at 128 registers, 64 us in this form (71 us with 16 rows and 24 warps).  A
+// grid of one CTA per row, so a long document holds back no row behind it.
+constexpr int kBagRows = 12, kBagGroup = 4;  // rows on their way per warp, rows per commit group
+constexpr int kBagGroups = kBagRows / kBagGroup;
+constexpr size_t kBagSmem = (size_t)8 * kBagRows * kE * sizeof(bf16);
+
 __global__ void __launch_bounds__(256) embbag_fwd_kernel(int batch, int rows, const int32_t *__restrict__ docs,
                                                          const int64_t *__restrict__ doc_ptr,
                                                          const int32_t *__restrict__ words, int V,
                                                          const bf16 *__restrict__ emb, bf16 *X0, int32_t *error) {
-    // one CTA per batch row: its 8 warps take contiguous eighths of the
-    // document's tokens (a long document is no longer one warp's serial loop),
-    // then the partial sums are added in warp order
-    __shared__ float part[8][kE];
+    extern __shared__ __align__(16) uint4 bag_ring[];
+    __shared__ __align__(16) float part[8][kE];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint4 *table = reinterpret_cast<const uint4 *>(emb) + lane;
+    uint4 *ring = bag_ring + warp * kBagRows * 32 + lane;  // row r of the ring: ring[32 r]
     for (int b = blockIdx.x; b < rows; b += gridDim.x) {
         float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         int64_t t0 = 0, t1 = 0;
@@ -97,49 +118,53 @@ __global__ void __launch_bounds__(256) embbag_fwd_kernel(int batch, int rows, co
             t0 = doc_ptr[d];
             t1 = doc_ptr[d + 1];
             const int64_t per = (t1 - t0 + 7) / 8;
-            const int64_t w0 = t0 + per * warp, w1 = min(t1, w0 + per);
-            for (int64_t tb = w0; tb < w1; tb += 32) {
-                const int wl = tb + lane < w1 ? words[tb + lane] : 0;
-                const int n = (int)min((int64_t)32, w1 - tb);
-                // eight embedding rows in flight, then added in token order
-                for (int j0 = 0; j0 < n; j0 += 8) {
-                    uint4 v[8];
-                    bool ok[8];
+            const int64_t w0 = min(t1, t0 + per * warp);
+            const int n = (int)(min(t1, w0 + per) - w0);
+            const int32_t *ids = words + w0;
+            const int groups = (n + kBagGroup - 1) / kBagGroup;
+            int cur = 0, next = lane < n ? ids[lane] : 0;  // the word ids of 32 tokens, and of the 32 after them
+            unsigned ok = 0u;
+            for (int g = 0; g < groups + kBagGroups; ++g) {
+                uint4 *slot = ring + (g % kBagGroups) * kBagGroup * 32;
+                if (g >= kBagGroups) {
+                    // rows are added in token order; one that was left out adds zero, which keeps a sum's bits
+                    asm volatile("cp.async.wait_group %0;" ::"n"(kBagGroups - 1) : "memory");
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        const int w = __shfl_sync(0xffffffffu, wl, (j0 + u) & 31);
-                        const bool in = j0 + u < n;
-                        ok[u] = in && (unsigned)w < (unsigned)V;
-                        if (in && !ok[u] && lane == 0) atomicOr(error, kErrWordRange);
-                        v[u] = ok[u] ? __ldg(reinterpret_cast<const uint4 *>(emb + (size_t)w * kE) + lane)
-                                     : make_uint4(0u, 0u, 0u, 0u);
-                    }
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        if (!ok[u]) continue;
+                    for (int u = 0; u < kBagGroup; ++u) {
                         float f[8];
-                        unpack8(v[u], f);
+                        unpack8(slot[32 * u], f);
 #pragma unroll
                         for (int i = 0; i < 8; ++i) acc[i] += f[i];
                     }
                 }
+                if (g < groups) {
+                    const int j = g * kBagGroup;
+                    if (j % 32 == 0) {
+                        cur = next;
+                        next = j + 32 + lane < n ? ids[j + 32 + lane] : 0;
+                        const bool in = j + lane < n, good = in && (unsigned)cur < (unsigned)V;
+                        if (in && !good) atomicOr(error, kErrWordRange);
+                        ok = __ballot_sync(0xffffffffu, good);
+                    }
+#pragma unroll
+                    for (int u = 0; u < kBagGroup; ++u) {
+                        const int w = __shfl_sync(0xffffffffu, cur, (j + u) & 31);
+                        const bool good = (ok >> ((j + u) & 31)) & 1u;
+                        copy16_async(slot + 32 * u, table + (size_t)(good ? w : 0) * (kE / 8), good);
+                    }
+                }
+                asm volatile("cp.async.commit_group;" ::: "memory");
             }
         }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) part[warp][8 * lane + i] = acc[i];
+        reinterpret_cast<float4 *>(part[warp])[2 * lane] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        reinterpret_cast<float4 *>(part[warp])[2 * lane + 1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
         __syncthreads();
-        if (warp == 0) {
-            float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            for (int w = 0; w < 8; ++w)
+        // column threadIdx.x of the row: the partial sums in warp order
+        float sum = 0.f;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) sum[i] += part[w][8 * lane + i];
-            const float inv = t1 > t0 ? 1.0f / (float)(t1 - t0) : 0.f;
-            uint4 q;
-            __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&q);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(sum[2 * i] * inv, sum[2 * i + 1] * inv);
-            reinterpret_cast<uint4 *>(X0 + (size_t)b * kE)[lane] = q;
-        }
+        for (int w = 0; w < 8; ++w) sum += part[w][threadIdx.x];
+        const float inv = t1 > t0 ? 1.0f / (float)(t1 - t0) : 0.f;
+        X0[(size_t)b * kE + threadIdx.x] = __float2bfloat16_rn(sum * inv);
         __syncthreads();  // part is rewritten by the next row
     }
 }
@@ -445,7 +470,8 @@ int encoder_pass(culda_encoder *e, int batch, const int32_t *docs, const int64_t
     const int Bp = (batch + 127) & ~127, K = e->K;
     int32_t *err = e->d_error;
     // forward
-    embbag_fwd_kernel<<<std::min(Bp, 148 * 16), 256, 0, s>>>(batch, Bp, docs, doc_ptr, words, e->V, e->emb_bf,
+    ECK(allow_smem(reinterpret_cast<const void *>(&embbag_fwd_kernel), kBagSmem, s));
+    embbag_fwd_kernel<<<Bp, 256, kBagSmem, s>>>(batch, Bp, docs, doc_ptr, words, e->V, e->emb_bf,
                                                                  e->X0, err);
     ECK(cudaGetLastError());
     GemmEpilogue ep;
