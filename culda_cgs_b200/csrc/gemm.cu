@@ -5,12 +5,12 @@
 // stored in BF16 both as is and transposed), and the GELU backward (times
 // GELU'(pre), BF16 out and transposed, bias-gradient column sums).
 //
-// One CTA of 128 threads per 128 x 128 output tile (and per K slice when the
-// K range is split), two CTAs resident per SM so one tile's epilogue runs
-// while the other's MMAs do.  Warp 0 lane 0 streams
-// 128 x 64 tiles of A and B into a 3-stage shared-memory ring with TMA
-// (128-byte swizzle); warp 1 lane 0 issues tcgen05.mma (M = 128, N = 128,
-// K = 16 per instruction) into 128 TMEM columns and frees each stage with
+// One CTA of 128 threads per output tile of 128 x 128, 64 or 32 (and per K
+// slice when the K range is split), two or more CTAs resident per SM so one
+// tile's epilogue runs while the other's MMAs do.  Warp 0 lane 0 streams
+// tiles of A and B, 64 deep, into a 3-stage shared-memory ring with TMA
+// (128-byte swizzle); warp 1 lane 0 issues tcgen05.mma (M = 128, N = the tile's,
+// K = 16 per instruction) into as many TMEM columns and frees each stage with
 // tcgen05.commit; when the last MMA has landed all four warps read their 32
 // TMEM lanes back with tcgen05.ld into a shared-memory copy of the tile, and
 // the epilogue writes it out row by row (coalesced) and, for the transposed
@@ -31,10 +31,19 @@ namespace culda {
 
 namespace {
 
-constexpr int kBM = 128, kBN = 128, kBK = 64, kStages = 3;
-constexpr int kTileBytes = kBM * kBK * 2;  // 16 KB; the B tile (kBN rows) is the same size
+constexpr int kBM = 128, kBK = 64, kStages = 3;
 constexpr int kGemmThreads = 128;
-constexpr size_t kGemmSmem = (size_t)kStages * 2 * kTileBytes + 1024;  // + alignment slack
+
+// The output tile is kBM x BN, BN = 128, 64 or 32.
+template <int BN>
+struct Tile {
+    static constexpr int kA = kBM * kBK * 2, kB = BN * kBK * 2;  // bytes of a stage's operands
+    // the ring (operand A's stages, then B's), which later holds the accumulator copy, + alignment slack
+    static constexpr size_t kRing = (size_t)kStages * (kA + kB);
+    static constexpr size_t kSmem = kRing + 1024;
+    static constexpr int kSP = BN + 1;  // row stride of the accumulator copy in floats
+    static_assert((size_t)kBM * kSP * sizeof(float) <= kSmem - 1023, "the accumulator copy fits the ring and the slack");
+};
 
 __device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
 
@@ -45,20 +54,21 @@ __device__ __forceinline__ float gelu_grad(float x) {
 }
 
 // The accumulator tile is staged in shared memory (the operand ring is free
-// once the last MMA has landed) as S[128][kSP] floats, row = output row; the
-// stride of 129 keeps both a lane-per-row write and a lane-per-row column read
-// free of bank conflicts.  Phase 1 (rows): each warp takes rows w, w+4, ...,
-// each lane 4 consecutive columns, so every global row store or load is one
-// 512-byte (FP32) or 256-byte (BF16) run.  Phase 2 (columns, BF16 epilogues):
-// each warp takes columns, each lane rows l, l+32, l+64, l+96 of the column,
-// for the transposed copy and the bias-gradient column sums.
-constexpr int kSP = kBN + 1;
-
-template <int EPI>
+// once the last MMA has landed) as S[128][BN + 1] floats, row = output row; the
+// odd stride keeps both a lane-per-row write and a lane-per-row column read
+// free of bank conflicts.  Phase 1 (rows): BN / 4 lanes take a row, 4
+// consecutive columns each, so every global row store or load is one run of 4
+// BN (FP32) or 2 BN (BF16) bytes.  Phase 2 (columns, BF16 epilogues): each warp
+// takes columns, each lane rows l, l+32, l+64, l+96 of the column, for the
+// transposed copy and the bias-gradient column sums.
+template <int EPI, int BN>
 __device__ __forceinline__ void epilogue_rows(const GemmEpilogue &ep, float *S, int m0, int n0, int warp, int lane) {
-    const int c = 4 * lane;
-    constexpr int kRowStep = kGemmThreads / 32, kAhead = 8;
-    for (int r0 = warp; r0 < kBM; r0 += kRowStep * kAhead) {
+    constexpr int kSP = Tile<BN>::kSP;
+    constexpr int kLanes = BN / 4, kRows = 32 / kLanes;  // lanes per row, rows per warp at a time
+    constexpr int kRowStep = kRows * kGemmThreads / 32, kAhead = 8;
+    static_assert(kBM % (kRowStep * kAhead) == 0, "whole groups of rows");
+    const int c = 4 * (lane % kLanes);
+    for (int r0 = warp * kRows + lane / kLanes; r0 < kBM; r0 += kRowStep * kAhead) {
         // the pre-activations of the next 8 rows are loaded before any of them
         // is stored: the stores below could alias them for all the compiler knows
         float4 pv[kAhead];
@@ -111,10 +121,11 @@ __device__ __forceinline__ void epilogue_rows(const GemmEpilogue &ep, float *S, 
     }
 }
 
-template <int EPI>
+template <int EPI, int BN>
 __device__ __forceinline__ void epilogue_cols(const GemmEpilogue &ep, const float *S, int m0, int n0, int warp,
                                               int lane) {
-    for (int cc = warp; cc < kBN; cc += kGemmThreads / 32) {
+    constexpr int kSP = Tile<BN>::kSP;
+    for (int cc = warp; cc < BN; cc += kGemmThreads / 32) {
         float s = 0.f;
         __nv_bfloat16 *dst = ep.out_bf16_t + (size_t)(n0 + cc) * ep.ld_t + m0;
 #pragma unroll
@@ -132,11 +143,12 @@ __device__ __forceinline__ void epilogue_cols(const GemmEpilogue &ep, const floa
     }
 }
 
-template <int EPI>
+template <int EPI, int BN>
 __global__ void __launch_bounds__(kGemmThreads, 2)
     gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, int K,
                      const GemmEpilogue ep, int32_t *error) {
     extern __shared__ uint8_t gsm_raw[];
+    constexpr int kA = Tile<BN>::kA, kB = Tile<BN>::kB, kSP = Tile<BN>::kSP;
     __shared__ __align__(8) uint64_t full[kStages], empty[kStages], done;
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
@@ -144,7 +156,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2)
     const uint32_t raw = umma::smem_u32(gsm_raw);
     uint8_t *base = gsm_raw + ((1024u - (raw & 1023u)) & 1023u);  // 1024-byte aligned for the swizzle
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * kBN;
+    const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * BN;
     // this CTA's K slice: k-blocks [kb0, kb0 + nk)
     const int nk_all = K / kBK;
     const int kb0 = (int)(((int64_t)nk_all * blockIdx.z) / gridDim.z);
@@ -162,7 +174,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2)
         umma::tma_prefetch_map(&tma_b);
     }
     if (warp == 0) {
-        umma::tmem_alloc(&tmem_slot, kBN);
+        umma::tmem_alloc(&tmem_slot, BN);
         umma::tmem_relinquish();
     }
     umma::tc_fence_before();
@@ -179,15 +191,15 @@ __global__ void __launch_bounds__(kGemmThreads, 2)
                     atomicExch(&abort_flag, 1);
                     break;
                 }
-                umma::mbar_arrive_expect_tx(&full[s], 2u * kTileBytes);
-                umma::tma_load_2d(base + (size_t)s * kTileBytes, &tma_a, (kb0 + kb) * kBK, m0, &full[s]);
-                umma::tma_load_2d(base + (size_t)(kStages + s) * kTileBytes, &tma_b, (kb0 + kb) * kBK, n0, &full[s]);
+                umma::mbar_arrive_expect_tx(&full[s], (uint32_t)(kA + kB));
+                umma::tma_load_2d(base + (size_t)s * kA, &tma_a, (kb0 + kb) * kBK, m0, &full[s]);
+                umma::tma_load_2d(base + (size_t)kStages * kA + (size_t)s * kB, &tma_b, (kb0 + kb) * kBK, n0, &full[s]);
             }
         }
         __syncwarp();
     } else if (warp == 1) {
         if (lane == 0) {  // MMA issuer
-            constexpr uint32_t idesc = umma::idesc_bf16_f32(kBM, kBN);
+            constexpr uint32_t idesc = umma::idesc_bf16_f32(kBM, BN);
             for (int kb = 0; kb < nk; ++kb) {
                 const int s = kb % kStages;
                 if (!umma::mbar_wait(&full[s], (uint32_t)(kb / kStages) & 1u)) {
@@ -196,8 +208,8 @@ __global__ void __launch_bounds__(kGemmThreads, 2)
                     break;
                 }
                 umma::tc_fence_after();
-                const uint64_t ad = umma::sdesc_k_sw128(base + (size_t)s * kTileBytes);
-                const uint64_t bd = umma::sdesc_k_sw128(base + (size_t)(kStages + s) * kTileBytes);
+                const uint64_t ad = umma::sdesc_k_sw128(base + (size_t)s * kA);
+                const uint64_t bd = umma::sdesc_k_sw128(base + (size_t)kStages * kA + (size_t)s * kB);
 #pragma unroll
                 for (int j = 0; j < kBK / 16; ++j)  // 16 BF16 = 32 bytes = 2 descriptor units per step
                     umma::mma_bf16(tmem, ad + 2u * j, bd + 2u * j, idesc, (kb | j) != 0 ? 1u : 0u);
@@ -217,22 +229,22 @@ __global__ void __launch_bounds__(kGemmThreads, 2)
     if (go) {
         float *S = reinterpret_cast<float *>(base);  // the operand ring, free now: every MMA has landed
         const int r = warp * 32 + lane;
-        for (int c = 0; c < kBN; c += 16) {
+        for (int c = 0; c < BN; c += 16) {
             float v[16];
             umma::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
 #pragma unroll
             for (int i = 0; i < 16; ++i) S[r * kSP + c + i] = v[i];
         }
         __syncthreads();
-        epilogue_rows<EPI>(ep, S, m0, n0, warp, lane);
+        epilogue_rows<EPI, BN>(ep, S, m0, n0, warp, lane);
         if (EPI != kEpiF32) {
             __syncthreads();
-            epilogue_cols<EPI>(ep, S, m0, n0, warp, lane);
+            epilogue_cols<EPI, BN>(ep, S, m0, n0, warp, lane);
         }
     }
     umma::tc_fence_before();
     __syncthreads();
-    if (warp == 0) umma::tmem_dealloc(tmem, kBN);
+    if (warp == 0) umma::tmem_dealloc(tmem, BN);
 }
 
 // ------------------------------------------------------------ tensor maps
@@ -254,13 +266,13 @@ EncodeTiledFn encode_fn() {
 }
 
 // A row-major BF16 matrix [rows x cols] with row stride ld elements, read in
-// boxes of 128 rows x 64 columns with 128-byte swizzle.
-cudaError_t make_map(CUtensorMap *map, const void *ptr, int rows, int cols, int ld) {
+// boxes of box_rows rows x 64 columns with 128-byte swizzle.
+cudaError_t make_map(CUtensorMap *map, const void *ptr, int rows, int cols, int ld, int box_rows) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return cudaErrorNotSupported;
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)ld * 2u};
-    const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)kBM};
+    const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)box_rows};
     const cuuint32_t estr[2] = {1u, 1u};
     const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(ptr), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -268,18 +280,46 @@ cudaError_t make_map(CUtensorMap *map, const void *ptr, int rows, int cols, int 
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-template <int EPI>
+template <int EPI, int BN>
 cudaError_t launch(const CUtensorMap &a, const CUtensorMap &b, int M, int N, int K, const GemmEpilogue &ep,
                    int32_t *error, cudaStream_t s) {
     static std::once_flag once;
     static cudaError_t attr = cudaSuccess;
     std::call_once(once, [] {
-        attr = cudaFuncSetAttribute(gemm_bf16_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)kGemmSmem);
+        attr = cudaFuncSetAttribute(gemm_bf16_kernel<EPI, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)Tile<BN>::kSmem);
     });
     if (attr != cudaSuccess) return attr;
-    gemm_bf16_kernel<EPI><<<dim3(N / kBN, M / kBM, ep.k_splits), kGemmThreads, kGemmSmem, s>>>(a, b, K, ep, error);
+    gemm_bf16_kernel<EPI, BN>
+        <<<dim3(N / BN, M / kBM, ep.k_splits), kGemmThreads, Tile<BN>::kSmem, s>>>(a, b, K, ep, error);
     return cudaGetLastError();
+}
+
+template <int EPI>
+cudaError_t launch_tile(int bn, const CUtensorMap &a, const CUtensorMap &b, int M, int N, int K,
+                        const GemmEpilogue &ep, int32_t *error, cudaStream_t s) {
+    return bn == 128  ? launch<EPI, 128>(a, b, M, N, K, ep, error, s)
+           : bn == 64 ? launch<EPI, 64>(a, b, M, N, K, ep, error, s)
+                      : launch<EPI, 32>(a, b, M, N, K, ep, error, s);
+}
+
+// Columns per tile: the narrowest tile that needs at most two CTAs per SM.  A
+// launch's time is its CTAs' fixed costs and epilogues (the MMAs of a 128 x 128
+// tile take 0.5 to 2 us), so a product of few tiles is cut finer until the chip
+// is full: 1024 x 512 outputs with the GELU epilogues 13.2 us (32 CTAs of 128
+// columns), 9.2 (64) and 7.2 us (128 CTAs of 32); 4096 x 512 14.4, 11.7 and
+// 14.3 us; 4096 x 1024 13.9, 15.3 and 18.9 us.  Every width adds an output's
+// products in the same order.
+int tile_columns(int M, int N, int splits) {
+    static const int sms = [] {
+        int dev = 0, n = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+            n = 148;
+        return n;
+    }();
+    const int64_t wide = (int64_t)(M / kBM) * (N / 128) * splits;
+    return wide * 4 <= 2 * sms ? 32 : wide * 2 <= 2 * sms ? 64 : 128;
 }
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -288,7 +328,7 @@ bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 
 const char *gemm_check(int M, int N, int K, const void *A, int lda, const void *B, int ldb, int epi,
                        const GemmEpilogue &ep) {
-    if (M <= 0 || N <= 0 || K <= 0 || M % kBM || N % kBN || K % kBK) return "M, N must be multiples of 128, K of 64";
+    if (M <= 0 || N <= 0 || K <= 0 || M % kBM || N % 128 || K % kBK) return "M, N must be multiples of 128, K of 64";
     if (!A || !B || !aligned16(A) || !aligned16(B)) return "A and B must be 16-byte aligned device pointers";
     if (lda < K || ldb < K || lda % 8 || ldb % 8) return "lda, ldb must be >= K and multiples of 8";
     if (ep.ldo < N || ep.ldo % 4) return "ldo must be >= N and a multiple of 4";
@@ -317,15 +357,16 @@ const char *gemm_check(int M, int N, int K, const void *A, int lda, const void *
 cudaError_t gemm_bf16_nt(int M, int N, int K, const void *A, int lda, const void *B, int ldb, int epi,
                          const GemmEpilogue &ep, int32_t *error, cudaStream_t s) {
     if (gemm_check(M, N, K, A, lda, B, ldb, epi, ep)) return cudaErrorInvalidValue;
+    const int bn = tile_columns(M, N, ep.k_splits);
     CUtensorMap ma, mb;
-    cudaError_t e = make_map(&ma, A, M, K, lda);
+    cudaError_t e = make_map(&ma, A, M, K, lda, kBM);
     if (e != cudaSuccess) return e;
-    e = make_map(&mb, B, N, K, ldb);
+    e = make_map(&mb, B, N, K, ldb, bn);
     if (e != cudaSuccess) return e;
     switch (epi) {
-        case kEpiF32: return launch<kEpiF32>(ma, mb, M, N, K, ep, error, s);
-        case kEpiBiasGelu: return launch<kEpiBiasGelu>(ma, mb, M, N, K, ep, error, s);
-        default: return launch<kEpiGeluBwd>(ma, mb, M, N, K, ep, error, s);
+        case kEpiF32: return launch_tile<kEpiF32>(bn, ma, mb, M, N, K, ep, error, s);
+        case kEpiBiasGelu: return launch_tile<kEpiBiasGelu>(bn, ma, mb, M, N, K, ep, error, s);
+        default: return launch_tile<kEpiGeluBwd>(bn, ma, mb, M, N, K, ep, error, s);
     }
 }
 
