@@ -15,16 +15,12 @@
 //             dW2 = dP2^T H1,  dP1 = (dP2 W2) * GELU'(P1), db1
 //             dW1 = dP1^T X0,  dX0 = dP1 W1          FP32
 //             dE[w] = sum of dX0[b] / L_b over the tokens of w in the batch
-//                   (tokens grouped by word, one write per embedding row)
 // The weight gradients split their K range (the batch) over several CTAs
 // per tile.  Every GEMM is C = A B^T with both operands K-major, so each weight is kept
 // in BF16 twice (W and W^T) and each activation that feeds a weight gradient
 // is written transposed by the epilogue that produces it.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
-
-#include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_scan.cuh>
 
 #include <algorithm>
 #include <cmath>
@@ -104,7 +100,7 @@ constexpr size_t kBagSmem = (size_t)8 * kBagRows * kE * sizeof(bf16);
 __global__ void __launch_bounds__(256) embbag_fwd_kernel(int batch, int rows, const int32_t *__restrict__ docs,
                                                          const int64_t *__restrict__ doc_ptr,
                                                          const int32_t *__restrict__ words, int V,
-                                                         const bf16 *__restrict__ emb, bf16 *X0, int32_t *error) {
+                                                         const bf16 *__restrict__ emb, bf16 *X0, bf16 *X0t, int32_t *error) {
     extern __shared__ __align__(16) uint4 bag_ring[];
     __shared__ __align__(16) float part[8][kE];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -164,112 +160,86 @@ __global__ void __launch_bounds__(256) embbag_fwd_kernel(int batch, int rows, co
 #pragma unroll
         for (int w = 0; w < 8; ++w) sum += part[w][threadIdx.x];
         const float inv = t1 > t0 ? 1.0f / (float)(t1 - t0) : 0.f;
-        X0[(size_t)b * kE + threadIdx.x] = __float2bfloat16_rn(sum * inv);
+        const bf16 mean = __float2bfloat16_rn(sum * inv);
+        X0[(size_t)b * kE + threadIdx.x] = mean;
+        if (X0t) X0t[(size_t)threadIdx.x * rows + b] = mean;  // for the weight gradient
         __syncthreads();  // part is rewritten by the next row
     }
 }
 
-// The embedding gradient: the batch's (word, row) pairs are laid out in row
-// order (a scan of the row lengths), sorted by word (a radix sort, stable, so
-// a word's tokens stay in row order), and the sorted list is cut into chunks
-// of 32 tokens.  A warp walks its chunk in order, summing dX0[b] / L_b per
-// word in registers.  A word whose tokens all lie in the chunk is written with
-// plain stores; a word whose run crosses the chunk's first or last token (the
-// frequent ones) adds each chunk's partial sum with one vector atomic per
-// lane.  gE holds zeros before the pass; words outside [0, V) sort last under
-// the key V and are skipped.
+// The embedding gradient: dX0[b] / L_b goes to the row of each of row b's
+// words with one vector reduction per 4 columns; a run of one word (documents
+// list their words in order) takes one for the whole run.  gE holds zeros
+// before.  A CTA per batch row; documents of more than kBagLong tokens, which
+// would hold one SM's reductions long after the others' are done, are shared
+// by kBagHelpers more CTAs.  (Laying out (word, row) pairs, sorting them by word
+// and walking the sorted list was 9 launches and a read-back of the batch's
+// token count: 79 us and a 20 us wait for 102k tokens, 230 us for 836k; the
+// reductions take 24 and 159 us.)
+constexpr int kBagLong = 4096, kBagHelpers = 148;
 
-// len[b] = L_b (for the scan of row offsets) and inv_len[b] = 1 / L_b.
-__global__ void bag_rows_kernel(int batch, const int32_t *__restrict__ docs, const int64_t *__restrict__ doc_ptr,
-                                int32_t *len, float *inv_len) {
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < batch; b += gridDim.x * blockDim.x) {
-        const int d = docs ? docs[b] : b;
-        const int64_t L = doc_ptr[d + 1] - doc_ptr[d];
-        len[b] = (int32_t)L;
-        inv_len[b] = L > 0 ? 1.0f / (float)L : 0.f;
+// Tokens [q0, q1) of a row: warps 2q and 2q + 1 take the two halves of the
+// columns for a quarter of them; g is the warp's part of dX0[b] / L_b.
+__device__ __forceinline__ void bag_scatter(int64_t q0, int64_t q1, const int32_t *__restrict__ words, int V, float4 g,
+                                            float *dst, int lane) {
+    for (int64_t tb = q0; tb < q1; tb += 32) {
+        const int w = tb + lane < q1 ? words[tb + lane] : -1;
+        const int prev = __shfl_up_sync(0xffffffffu, w, 1);
+        const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || w != prev);
+        for (unsigned m = __ballot_sync(0xffffffffu, (unsigned)w < (unsigned)V) & heads; m; m &= m - 1u) {
+            const int j = __ffs(m) - 1;
+            const unsigned after = heads & ~((2u << j) - 1u);  // the next run's start, if any
+            const float c = (float)((after ? __ffs(after) - 1 : 32) - j);
+            const int wj = __shfl_sync(0xffffffffu, w, j);
+            atomicAdd(reinterpret_cast<float4 *>(dst + (size_t)wj * kE),
+                      make_float4(c * g.x, c * g.y, c * g.z, c * g.w));
+        }
     }
 }
 
-// key[off[b] + j] = word of the j-th token of row b (V when out of range), val = b.
-__global__ void __launch_bounds__(256) bag_pairs_kernel(int batch, const int32_t *__restrict__ docs,
-                                                        const int64_t *__restrict__ doc_ptr,
-                                                        const int32_t *__restrict__ words, int V,
-                                                        const int32_t *__restrict__ off, int32_t *key, int32_t *val) {
-    for (int b = blockIdx.x; b < batch; b += gridDim.x) {
-        const int d = docs ? docs[b] : b;
+__global__ void __launch_bounds__(256) embbag_bwd_kernel(int batch, const int32_t *__restrict__ docs,
+                                                         const int64_t *__restrict__ doc_ptr,
+                                                         const int32_t *__restrict__ words, int V,
+                                                         const float *__restrict__ dX0, float *gE) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int col = (warp & 1) * 128 + 4 * lane;
+    // part s of `parts` of row b's tokens [t0, t1)
+    auto scatter = [&](int b, int64_t t0, int64_t t1, int s, int parts) {
+        const float inv = 1.0f / (float)(t1 - t0);
+        float4 g = *reinterpret_cast<const float4 *>(dX0 + (size_t)b * kE + col);
+        g = make_float4(g.x * inv, g.y * inv, g.z * inv, g.w * inv);
+        const int64_t per = (t1 - t0 + 4 * parts - 1) / (4 * parts);
+        const int64_t q0 = min(t1, t0 + per * (4 * s + (warp >> 1))), q1 = min(t1, q0 + per);
+        bag_scatter(q0, q1, words, V, g, gE + col, lane);
+    };
+    if ((int)blockIdx.x < batch) {
+        const int b = blockIdx.x, d = docs ? docs[b] : b;
         const int64_t t0 = doc_ptr[d], t1 = doc_ptr[d + 1];
-        const int o = off[b];
-        for (int64_t t = t0 + threadIdx.x; t < t1; t += blockDim.x) {
-            const int w = words[t];
-            key[o + (t - t0)] = (unsigned)w < (unsigned)V ? w : V;
-            val[o + (t - t0)] = b;
-        }
+        if (t1 > t0 && t1 - t0 <= kBagLong) scatter(b, t0, t1, 0, 1);
+        return;
     }
-}
-
-// Warp per chunk of 32 sorted tokens; each lane holds 8 of the 256 columns.
-__global__ void embbag_bwd_grouped_kernel(int64_t n, int V, const int32_t *__restrict__ wid,
-                                          const int32_t *__restrict__ rows, const float *__restrict__ inv_len,
-                                          const float *__restrict__ dX0, float *gE) {
-    const int lane = threadIdx.x & 31;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t c0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; c0 < n; c0 += nw * 32) {
-        const int cn = (int)min((int64_t)32, n - c0);
-        const int my_w = lane < cn ? wid[c0 + lane] : V;
-        const int my_b = lane < cn ? rows[c0 + lane] : 0;
-        const float my_s = lane < cn ? inv_len[my_b] : 0.f;
-        // does the chunk's first (last) run continue from the chunk before (after) it?
-        const int w_before = c0 > 0 ? wid[c0 - 1] : -1;
-        const int w_after = c0 + cn < n ? wid[c0 + cn] : -1;
-        const int first_w = __shfl_sync(0xffffffffu, my_w, 0), last_w = __shfl_sync(0xffffffffu, my_w, cn - 1);
-        // the chunk's dX0 rows, 2 x 16 bytes per lane each, loaded 8 at a time ahead of their use
-        float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
-        float4 r0[8], r1[8];
-        for (int j = 0; j < cn; ++j) {
-            if ((j & 7) == 0) {
+    // the long documents, 8 rows per thread at a time
+    constexpr int kAhead = 8;
+    __shared__ int found[256 * kAhead], num_found;
+    for (int b0 = 0; b0 < batch; b0 += 256 * kAhead) {
+        if (threadIdx.x == 0) num_found = 0;
+        __syncthreads();
+        int64_t len[kAhead];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const int bj = __shfl_sync(0xffffffffu, my_b, (j + u) & 31);
-                    const float4 *q = reinterpret_cast<const float4 *>(dX0 + (size_t)bj * kE) + 2 * lane;
-                    const bool in = j + u < cn;
-                    r0[u] = in ? q[0] : make_float4(0.f, 0.f, 0.f, 0.f);
-                    r1[u] = in ? q[1] : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-            }
-            const int w = __shfl_sync(0xffffffffu, my_w, j);
-            const float sc = __shfl_sync(0xffffffffu, my_s, j);
-            float4 g0 = r0[0], g1 = r1[0];
-#pragma unroll
-            for (int u = 1; u < 8; ++u)
-                if ((j & 7) == u) {
-                    g0 = r0[u];
-                    g1 = r1[u];
-                }
-            a0.x += g0.x * sc;
-            a0.y += g0.y * sc;
-            a0.z += g0.z * sc;
-            a0.w += g0.w * sc;
-            a1.x += g1.x * sc;
-            a1.y += g1.y * sc;
-            a1.z += g1.z * sc;
-            a1.w += g1.w * sc;
-            const int wn = __shfl_sync(0xffffffffu, my_w, (j + 1) & 31);
-            if (j + 1 == cn || wn != w) {  // the end of this word's run in the chunk
-                if (w < V) {
-                    float4 *dst = reinterpret_cast<float4 *>(gE + (size_t)w * kE) + 2 * lane;
-                    const bool shared = (w == first_w && w == w_before) || (w == last_w && w == w_after);
-                    if (!shared) {  // the whole word: no other chunk adds to it
-                        dst[0] = a0;
-                        dst[1] = a1;
-                    } else {
-                        atomicAdd(dst, a0);
-                        atomicAdd(dst + 1, a1);
-                    }
-                }
-                a0 = make_float4(0.f, 0.f, 0.f, 0.f);
-                a1 = a0;
-            }
+        for (int u = 0; u < kAhead; ++u) {
+            const int b = b0 + 256 * u + threadIdx.x;
+            const int d = b < batch ? (docs ? docs[b] : b) : -1;
+            len[u] = d >= 0 ? doc_ptr[d + 1] - doc_ptr[d] : 0;
         }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            if (len[u] > kBagLong) found[atomicAdd(&num_found, 1)] = b0 + 256 * u + threadIdx.x;
+        __syncthreads();
+        for (int i = 0; i < num_found; ++i) {
+            const int b = found[i], d = docs ? docs[b] : b;
+            scatter(b, doc_ptr[d], doc_ptr[d + 1], blockIdx.x - batch, kBagHelpers);
+        }
+        __syncthreads();  // the list is rewritten
     }
 }
 
@@ -372,15 +342,83 @@ __global__ void __launch_bounds__(256) softmax_xent_kernel(int batch, int rows, 
     }
 }
 
-__global__ void adam_kernel(int64_t n, float *p, const float *g, float *m, float *v, float lr, float b1, float b2,
-                            float eps, float c1, float c2) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float gi = g[i];
-        const float mi = b1 * m[i] + (1.0f - b1) * gi;
-        const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        p[i] -= lr * (mi * c1) / (sqrtf(vi * c2) + eps);
+// ------------------------------------------------------------------- Adam
+struct AdamStep {
+    float lr, b1, b2, eps, c1, c2;
+
+    __device__ __forceinline__ float operator()(float p, float g, float &m, float &v) const {
+        m = b1 * m + (1.0f - b1) * g;
+        v = b2 * v + (1.0f - b2) * g * g;
+        return p - lr * (m * c1) / (sqrtf(v * c2) + eps);
+    }
+};
+
+// One Adam step on every weight and the BF16 copies the next pass reads, in one
+// pass over memory (30 bytes a weight).  The first flat_blocks CTAs take the
+// embeddings, then the biases, 16 bytes per access; the others a 32 x 32 tile
+// of W1, W2 or W3 each, whose transposed copy goes through shared memory.  (An
+// Adam kernel of scalar accesses, four conversions and three transposes after
+// it: 70 us and 8 launches at 6M weights; this form 32 us.)
+struct AdamParams {
+    float *p;
+    const float *g;
+    float *m, *v;
+    int64_t embed;          // elements of E, the first in the blocks
+    int64_t bias[3];        // offsets of b1, b2, b3
+    int bias_n[3];
+    bf16 *emb_bf;
+    int64_t w[3];           // offsets of W1, W2, W3
+    int rows[3], cols[3];   // multiples of 32
+    bf16 *wb[3], *wt[3];
+    int flat_blocks;
+};
+
+__global__ void __launch_bounds__(256) adam_kernel(const AdamParams a, const AdamStep step) {
+    __shared__ float tile[32][33];
+    const int tid = threadIdx.x;
+    if ((int)blockIdx.x < a.flat_blocks) {
+        const int64_t n4 = a.embed / 4, stride = (int64_t)a.flat_blocks * 256;
+        for (int64_t i = (int64_t)blockIdx.x * 256 + tid; i < n4; i += stride) {
+            float4 p = reinterpret_cast<const float4 *>(a.p)[i], m = reinterpret_cast<const float4 *>(a.m)[i],
+                   v = reinterpret_cast<const float4 *>(a.v)[i];
+            const float4 g = reinterpret_cast<const float4 *>(a.g)[i];
+            p.x = step(p.x, g.x, m.x, v.x);
+            p.y = step(p.y, g.y, m.y, v.y);
+            p.z = step(p.z, g.z, m.z, v.z);
+            p.w = step(p.w, g.w, m.w, v.w);
+            reinterpret_cast<float4 *>(a.p)[i] = p;
+            reinterpret_cast<float4 *>(a.m)[i] = m;
+            reinterpret_cast<float4 *>(a.v)[i] = v;
+            uint2 h;
+            reinterpret_cast<__nv_bfloat162 *>(&h)[0] = __floats2bfloat162_rn(p.x, p.y);
+            reinterpret_cast<__nv_bfloat162 *>(&h)[1] = __floats2bfloat162_rn(p.z, p.w);
+            reinterpret_cast<uint2 *>(a.emb_bf)[i] = h;
+        }
+        for (int t = 0; t < 3; ++t)
+            for (int i = blockIdx.x * 256 + tid; i < a.bias_n[t]; i += (int)stride) {
+                const int64_t o = a.bias[t] + i;
+                a.p[o] = step(a.p[o], a.g[o], a.m[o], a.v[o]);
+            }
+        return;
+    }
+    int x = blockIdx.x - a.flat_blocks, t = 0;
+    while (x >= (a.rows[t] / 32) * (a.cols[t] / 32)) x -= (a.rows[t] / 32) * (a.cols[t] / 32), ++t;
+    const int R = a.rows[t], C = a.cols[t], r0 = x / (C / 32) * 32, c0 = x % (C / 32) * 32;
+    const int c = tid & 31;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = (tid >> 5) + 8 * i;
+        const int64_t e = (int64_t)(r0 + r) * C + c0 + c, o = a.w[t] + e;
+        const float p = step(a.p[o], a.g[o], a.m[o], a.v[o]);
+        a.p[o] = p;
+        a.wb[t][e] = __float2bfloat16_rn(p);
+        tile[r][c] = p;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = (tid >> 5) + 8 * i;  // column of the tile
+        a.wt[t][(int64_t)(c0 + r) * R + r0 + c] = __float2bfloat16_rn(tile[c][r]);
     }
 }
 
@@ -404,15 +442,6 @@ struct culda_encoder {
     float *P1 = nullptr, *P2 = nullptr, *Z = nullptr, *dX0 = nullptr;
     double *d_loss = nullptr;
     int32_t *d_error = nullptr;
-    // the batch's (word, row) pairs sorted by word, for the embedding gradient
-    int32_t *bag_len = nullptr, *bag_off = nullptr;  // [Bmax + 1] row lengths and their exclusive scan
-    float *bag_inv_len = nullptr;                    // [Bmax] 1 / L of every batch row
-    int32_t *bag_key = nullptr, *bag_val = nullptr;  // [bag_cap] pairs in row order
-    int32_t *bag_wid = nullptr, *bag_rows = nullptr; // [bag_cap] the pairs sorted by word
-    int64_t bag_cap = 0;
-    void *scan_tmp = nullptr, *sort_tmp = nullptr;
-    size_t scan_tmp_bytes = 0, sort_tmp_bytes = 0;
-    int key_bits = 1;                                // bits of the keys 0..V
     std::vector<void *> allocs;
 
     float *tensor(int t) { return params + off[t]; }
@@ -443,11 +472,6 @@ int fail_enc(int code, const char *fmt, const char *what) {
 
 cudaError_t transpose_to_bf16(int R, int C, const float *in, bf16 *out, cudaStream_t s) {
     transpose_bf16_kernel<float><<<dim3((C + 31) / 32, (R + 31) / 32), dim3(32, 8), 0, s>>>(R, C, in, C, out, R);
-    return cudaGetLastError();
-}
-
-cudaError_t transpose_bf16(int R, int C, const bf16 *in, bf16 *out, cudaStream_t s) {
-    transpose_bf16_kernel<bf16><<<dim3((C + 31) / 32, (R + 31) / 32), dim3(32, 8), 0, s>>>(R, C, in, C, out, R);
     return cudaGetLastError();
 }
 
@@ -519,7 +543,7 @@ int encoder_max_batch(const culda_encoder *e) { return e->Bmax; }
 int32_t *encoder_error_word(culda_encoder *e) { return e->d_error; }
 
 int encoder_pass(culda_encoder *e, int batch, const int32_t *docs, const int64_t *doc_ptr, const int32_t *words,
-                 const EncoderTarget *target, bool update, float *probs, cudaStream_t s, int64_t batch_tokens) {
+                 const EncoderTarget *target, bool update, float *probs, cudaStream_t s) {
     if (batch <= 0 || batch > e->Bmax || !doc_ptr || !words)
         return fail_enc(CULDA_ERR_INVALID_ARG, "encoder: %s", "batch outside 1..max_batch or null CSR");
     if (target && !target->dense && !target->acc)
@@ -530,7 +554,7 @@ int encoder_pass(culda_encoder *e, int batch, const int32_t *docs, const int64_t
     // forward
     ECK(allow_smem(reinterpret_cast<const void *>(&embbag_fwd_kernel), kBagSmem, s));
     embbag_fwd_kernel<<<Bp, 256, kBagSmem, s>>>(batch, Bp, docs, doc_ptr, words, e->V, e->emb_bf,
-                                                                 e->X0, err);
+                                                                 e->X0, target ? e->X0t : nullptr, err);
     ECK(cudaGetLastError());
     GemmEpilogue ep;
     ep.out_f32 = e->P1;
@@ -559,7 +583,6 @@ int encoder_pass(culda_encoder *e, int batch, const int32_t *docs, const int64_t
     ECK(cudaMemsetAsync(e->grads, 0, sizeof(float) * (size_t)e->off[kNumTensors], s));
     ECK(softmax_xent(batch, Bp, K, e->Z, *target, docs, doc_ptr, probs, e->dZ, e->dZt, e->grad(CULDA_ENC_B3),
                      e->d_loss, s));
-    ECK(transpose_bf16(Bp, kE, e->X0, e->X0t, s));
     GemmEpilogue gw;
     gw.ldo = kH;
     gw.out_f32 = e->grad(CULDA_ENC_W3);
@@ -585,70 +608,52 @@ int encoder_pass(culda_encoder *e, int batch, const int32_t *docs, const int64_t
     ECK(gemm_wgrad(kH, kE, Bp, e->dP1t, e->X0t, g1, err, s));  // dW1 = dP1^T X0
     g1.out_f32 = e->dX0;
     ECK(gemm(Bp, kE, kH, e->dP1, e->W1t, kEpiF32, g1, err, s));  // dX0 = dP1 W1
-    // the batch's (word, row) pairs sorted by word, then one pass over them
-    bag_rows_kernel<<<(batch + 255) / 256, 256, 0, s>>>(batch, docs, doc_ptr, e->bag_len, e->bag_inv_len);
+    embbag_bwd_kernel<<<batch + kBagHelpers, 256, 0, s>>>(batch, docs, doc_ptr, words, e->V, e->dX0,
+                                                          e->grad(CULDA_ENC_E));
     ECK(cudaGetLastError());
-    ECK(cub::DeviceScan::ExclusiveSum(e->scan_tmp, e->scan_tmp_bytes, e->bag_len, e->bag_off, batch + 1, s));
-    if (batch_tokens < 0) {  // the caller did not count the batch's tokens: read the scan's total
-        int32_t n = 0;
-        ECK(cudaMemcpyAsync(&n, e->bag_off + batch, sizeof n, cudaMemcpyDeviceToHost, s));
-        ECK(cudaStreamSynchronize(s));
-        batch_tokens = n;
-    }
-    if (batch_tokens > e->bag_cap) {
-        ECK(cudaStreamSynchronize(s));
-        for (void **q : {(void **)&e->bag_key, (void **)&e->bag_val, (void **)&e->bag_wid, (void **)&e->bag_rows,
-                         &e->sort_tmp}) {
-            if (*q) {
-                cudaFree(*q);
-                e->allocs.erase(std::find(e->allocs.begin(), e->allocs.end(), *q));
-                *q = nullptr;
-            }
-        }
-        const int64_t cap = std::max<int64_t>(batch_tokens, 2 * e->bag_cap);
-        ECK(ealloc(e, &e->bag_key, (size_t)cap));
-        ECK(ealloc(e, &e->bag_val, (size_t)cap));
-        ECK(ealloc(e, &e->bag_wid, (size_t)cap));
-        ECK(ealloc(e, &e->bag_rows, (size_t)cap));
-        e->sort_tmp_bytes = 0;
-        ECK(cub::DeviceRadixSort::SortPairs(nullptr, e->sort_tmp_bytes, e->bag_key, e->bag_wid, e->bag_val,
-                                            e->bag_rows, (int)cap, 0, e->key_bits));
-        uint8_t *tmp = nullptr;
-        ECK(ealloc(e, &tmp, e->sort_tmp_bytes));
-        e->sort_tmp = tmp;
-        e->bag_cap = cap;
-    }
-    if (batch_tokens > 0) {
-        bag_pairs_kernel<<<std::min(batch, 148 * 16), 256, 0, s>>>(batch, docs, doc_ptr, words, e->V, e->bag_off,
-                                                                   e->bag_key, e->bag_val);
-        ECK(cudaGetLastError());
-        ECK(cub::DeviceRadixSort::SortPairs(e->sort_tmp, e->sort_tmp_bytes, e->bag_key, e->bag_wid, e->bag_val,
-                                            e->bag_rows, (int)batch_tokens, 0, e->key_bits, s));
-        embbag_bwd_grouped_kernel<<<grid_for(batch_tokens), 256, 0, s>>>(batch_tokens, e->V, e->bag_wid, e->bag_rows,
-                                                                         e->bag_inv_len, e->dX0,
-                                                                         e->grad(CULDA_ENC_E));
-        ECK(cudaGetLastError());
-    }
     if (update) {
         e->steps += 1;
         const float c1 = 1.0f / (1.0f - powf(e->b1, (float)e->steps));
         const float c2 = 1.0f / (1.0f - powf(e->b2, (float)e->steps));
-        const int64_t n = e->off[kNumTensors];
-        adam_kernel<<<grid_for(n), 256, 0, s>>>(n, e->params, e->grads, e->adam_m, e->adam_v, e->lr, e->b1, e->b2,
-                                                e->eps, c1, c2);
+        AdamParams a{};
+        a.p = e->params;
+        a.g = e->grads;
+        a.m = e->adam_m;
+        a.v = e->adam_v;
+        a.embed = e->off[CULDA_ENC_E + 1];
+        a.emb_bf = e->emb_bf;
+        const int bias[3] = {CULDA_ENC_B1, CULDA_ENC_B2, CULDA_ENC_B3};
+        const int weight[3] = {CULDA_ENC_W1, CULDA_ENC_W2, CULDA_ENC_W3};
+        const int rows[3] = {kH, kH, K}, cols[3] = {kE, kH, kH};
+        bf16 *wb[3] = {e->W1, e->W2, e->W3}, *wt[3] = {e->W1t, e->W2t, e->W3t};
+        int tiles = 0;
+        for (int t = 0; t < 3; ++t) {
+            a.bias[t] = e->off[bias[t]];
+            a.bias_n[t] = (int)(e->off[bias[t] + 1] - e->off[bias[t]]);
+            a.w[t] = e->off[weight[t]];
+            a.rows[t] = rows[t];
+            a.cols[t] = cols[t];
+            a.wb[t] = wb[t];
+            a.wt[t] = wt[t];
+            tiles += (rows[t] / 32) * (cols[t] / 32);
+        }
+        a.flat_blocks = (int)std::min<int64_t>(148 * 8, (a.embed / 4 + 255) / 256);
+        adam_kernel<<<a.flat_blocks + tiles, 256, 0, s>>>(a, AdamStep{e->lr, e->b1, e->b2, e->eps, c1, c2});
         ECK(cudaGetLastError());
-        ECK(refresh_bf16(e, s));
     }
     return CULDA_OK;
 }
 
 int encoder_take_loss(culda_encoder *e, int batch_rows, double *loss, cudaStream_t s) {
-    double h = 0.0;
-    int32_t err = 0;
-    ECK(cudaMemcpyAsync(&h, e->d_loss, sizeof(double), cudaMemcpyDeviceToHost, s));
-    ECK(cudaMemcpyAsync(&err, e->d_error, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-    ECK(cudaMemsetAsync(e->d_loss, 0, sizeof(double), s));
+    struct {
+        double loss;
+        int32_t err;
+    } got = {0.0, 0};
+    ECK(cudaMemcpyAsync(&got, e->d_loss, sizeof got, cudaMemcpyDeviceToHost, s));
     ECK(cudaStreamSynchronize(s));
+    ECK(cudaMemsetAsync(e->d_loss, 0, sizeof(double), s));
+    const double h = got.loss;
+    const int32_t err = got.err;
     if (err) {
         cudaMemsetAsync(e->d_error, 0, sizeof(int32_t), s);
         char msg[96];
@@ -754,19 +759,8 @@ extern "C" int culda_encoder_create(const culda_encoder_params *p, culda_encoder
     EALLOC(e->P2, B * kH);
     EALLOC(e->Z, B * K);
     EALLOC(e->dX0, B * kE);
-    EALLOC(e->d_loss, 1);
-    EALLOC(e->d_error, 1);
-    EALLOC(e->bag_len, (size_t)B + 1);
-    EALLOC(e->bag_off, (size_t)B + 1);
-    EALLOC(e->bag_inv_len, B);
-    while ((1u << e->key_bits) <= (unsigned)e->V) ++e->key_bits;  // keys 0..V
-    r = cub::DeviceScan::ExclusiveSum(nullptr, e->scan_tmp_bytes, e->bag_len, e->bag_off, B + 1);
-    if (r != cudaSuccess) return bail(r);
-    {
-        uint8_t *tmp = nullptr;
-        EALLOC(tmp, e->scan_tmp_bytes);
-        e->scan_tmp = tmp;
-    }
+    EALLOC(e->d_loss, 2);  // the error word follows the loss, so one copy reads both
+    e->d_error = reinterpret_cast<int32_t *>(e->d_loss + 1);
 #undef EALLOC
     cudaStream_t s = nullptr;
     r = cudaMemsetAsync(e->grads, 0, sizeof(float) * np, s);

@@ -44,3 +44,71 @@ def test_forward_at_the_bag_limits(batch):
         assert np.abs(probs.cpu().numpy() - ora["q"]).max() < 2e-3
         d_words[int(doc_ptr[batch]) - 1] = V  # the last token of the last document with tokens
         assert forward() == _ffi.CULDA_ERR_DEVICE_STATE
+
+
+def _batch(rng, V, lens):
+    """Documents of the given lengths, each with its words in order, so runs of one word occur."""
+    doc_ptr = np.concatenate([[0], np.cumsum(lens)])
+    words = np.concatenate([np.sort((V * rng.random(n) ** 3).astype(np.int64)) for n in lens] + [np.zeros(0, int)])
+    return doc_ptr, words
+
+
+def _grads(enc, batch, doc_ptr, words, target, fn):
+    import torch
+
+    d = [torch.from_numpy(a).cuda() for a in (doc_ptr.astype(np.int64), words.astype(np.int32), target.astype(np.float32))]
+    loss = C.c_double()
+    assert fn(enc.handle, batch, None, *[C.c_void_p(x.data_ptr()) for x in d], C.byref(loss), None) == 0
+    return {n: enc.get(n, grad=True).astype(np.float64).ravel() for n in EO.NAMES}
+
+
+def _rel(a, b):
+    return np.linalg.norm(a - b) / np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("lens", [[0, 1, 31, 32, 33, 64, 65, 2], [4096, 4097, 0, 20_000, 5], [4097]])
+def test_embedding_gradient_at_the_length_limits(lens):
+    """dE against the oracle (2e-2 relative Frobenius, as the other gradients):
+    documents of one CTA, those its helpers share, runs of one word."""
+    rng = np.random.default_rng(len(lens))
+    V, K, batch = 300, 128, len(lens)
+    doc_ptr, words = _batch(rng, V, lens)
+    t = {k: v.astype(np.float32).astype(np.float64) for k, v in EO.random_tensors(rng, V, K).items()}
+    target = EO.random_target(rng, batch, K).astype(np.float32).astype(np.float64)
+    with cb.Encoder(V, K, max_batch=batch) as enc:
+        for k, v in t.items():
+            enc.set(k, v)
+        got = _grads(enc, batch, doc_ptr, words, target, cb.lib().culda_encoder_backward)
+        want = EO.EncoderOracle(t).run(doc_ptr, words, np.arange(batch), target)["grads"]
+        for n in EO.NAMES:
+            assert _rel(got[n], want[n].ravel()) < 2e-2, n
+
+
+@pytest.mark.parametrize("V,K", [(37, 128), (1000, 640)])
+def test_training_step_refreshes_every_copy(V, K):
+    """After a step, an encoder given the same weights anew (whose BF16 copies and
+    transposes come from the plain conversion) has the same forward pass bit for
+    bit and the same gradients up to the order of FP32 sums (1e-5)."""
+    import torch
+
+    rng = np.random.default_rng(V)
+    batch = 150
+    doc_ptr, words = _batch(rng, V, rng.integers(1, 40, batch))
+    target = EO.random_target(rng, batch, K)
+    with cb.Encoder(V, K, max_batch=batch, lr=1e-2) as a, cb.Encoder(V, K, max_batch=batch) as b:
+        before = a.get("W3")
+        _grads(a, batch, doc_ptr, words, target, cb.lib().culda_encoder_train_step)
+        assert (a.get("W3") != before).mean() > 0.9
+        for n in EO.NAMES:
+            b.set(n, a.get(n))
+        probs = []
+        for enc in (a, b):
+            q = torch.zeros(batch, K, device="cuda")
+            d = [torch.from_numpy(x).cuda() for x in (doc_ptr.astype(np.int64), words.astype(np.int32))]
+            assert cb.lib().culda_encoder_forward(enc.handle, batch, None, *[C.c_void_p(x.data_ptr()) for x in d],
+                                                  C.c_void_p(q.data_ptr()), None) == 0
+            probs.append(q.cpu().numpy())
+        assert np.array_equal(*probs)
+        ga, gb = (_grads(e, batch, doc_ptr, words, target, cb.lib().culda_encoder_backward) for e in (a, b))
+        for n in EO.NAMES:
+            assert _rel(ga[n], gb[n]) < 1e-5, n
