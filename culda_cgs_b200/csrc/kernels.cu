@@ -1043,20 +1043,22 @@ extern "C" int culda_sample(const culda_sample_args *a, void *d_workspace, size_
     int32_t *hot_phi = (int32_t *)(ws + 256 + ((size_t)a->num_items * sizeof(double) + 255) / 256 * 256);
     int rc = cuda_status(cudaMemsetAsync(counter, 0, 256, s));
     if (rc) return rc;
+    int32_t first_warp = a->num_items;  // items from here on are small
     // the sampler indexes shared memory with each entry's topic: reject a
     // theta array whose rows or topics are out of range before launching it
     {
-        int32_t *flag = counter + 2, bad = 0;
-        rc = cuda_status(launch_check_theta(a->num_docs, a->k, reinterpret_cast<const int2 *>(a->theta_rows),
-                                            reinterpret_cast<const ThetaEntry *>(a->theta), a->theta_capacity, flag,
-                                            s));
-        if (!rc) rc = cuda_status(cudaMemcpyAsync(&bad, flag, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+        int32_t *out = counter + 40, got[3] = {0, 0, 0};
+        rc = cuda_status(launch_check_sample(a->num_docs, a->k, reinterpret_cast<const int2 *>(a->theta_rows),
+                                             reinterpret_cast<const ThetaEntry *>(a->theta), a->theta_capacity,
+                                             a->items, a->num_items, out, s));
+        if (!rc) rc = cuda_status(cudaMemcpyAsync(got, out, sizeof got, cudaMemcpyDeviceToHost, s));
         if (!rc) rc = cuda_status(cudaStreamSynchronize(s));
         if (rc) return rc;
-        if (bad) {
-            set_global_error("culda_sample: theta rows or topics out of range (flags 0x%x)", bad);
+        if (got[0]) {
+            set_global_error("culda_sample: theta rows or topics out of range (flags 0x%x)", got[0]);
             return CULDA_ERR_INVALID_ARG;
         }
+        if (got[1] + got[2] <= a->num_items) first_warp = a->num_items - got[1];
     }
     if (a->num_hot > 0) {
         rc = cuda_status(cudaMemsetAsync(hot_phi, 0, (size_t)a->num_hot * a->k * sizeof(int32_t), s));
@@ -1088,6 +1090,8 @@ extern "C" int culda_sample(const culda_sample_args *a, void *d_workspace, size_
     p.num_segs = a->num_segs;
     p.hot_phi = hot_phi;
     p.item_counter = counter;
+    p.first_warp = first_warp;
+    p.warp_counter = counter + 48;
     p.item_ll = item_ll;
     p.seed = a->seed;
     p.iteration = a->iteration;

@@ -150,9 +150,12 @@ cudaError_t launch_hot_rows(int k, const culda_item *hot_items, int num_hot_item
 cudaError_t launch_finalize_ll(double *item_ll, int num_items, DevStats *st, int32_t *done, cudaStream_t s);
 
 // Flags theta rows outside the array or misaligned, and entries whose topic
-// is not below K (the kernel-level sampler checks a caller's theta with it).
-cudaError_t launch_check_theta(int num_docs, int k, const int2 *rows, const ThetaEntry *theta, int64_t cap,
-                               int32_t *error, cudaStream_t s);
+// is not below K (the kernel-level sampler checks a caller's theta with it),
+// and looks the work list over: out[0] the flags, out[1] num_items minus the
+// first item of at most kWarpItemTokens tokens, out[2] one past the last larger
+// one (all zero before; the list is in order when out[1] + out[2] <= num_items).
+cudaError_t launch_check_sample(int num_docs, int k, const int2 *rows, const ThetaEntry *theta, int64_t cap,
+                                const culda_item *items, int num_items, int32_t *out, cudaStream_t s);
 
 cudaError_t launch_init_topics(int64_t n, int k, uint64_t seed, const int32_t *tok_index, uint16_t *z,
                                cudaStream_t s);

@@ -56,7 +56,7 @@ __device__ __forceinline__ float fsum(float a, float b) { return __fadd_rn(a, b)
 // total `tot`; adds to the run the totals of all earlier threads (Kogge-Stone
 // shuffles inside a warp, then across the warps).  Ends without a barrier.
 __device__ __forceinline__ void add_run_offsets(float tot, float *out, int b, int e, float *s_warp) {
-    const int T = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = T >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = kSampleThreads / 32;
     float incl = tot;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -65,7 +65,7 @@ __device__ __forceinline__ void add_run_offsets(float tot, float *out, int b, in
     }
     float ex = __shfl_up_sync(0xffffffffu, incl, 1);
     if (lane == 0) ex = 0.f;
-    if (lane == 31) s_warp[warp] = incl;
+    if (lane == 31 && warp < nwarps) s_warp[warp] = incl;
     __syncthreads();
     if (warp == 0) {
         float w = lane < nwarps ? s_warp[lane] : 0.f;
@@ -79,6 +79,7 @@ __device__ __forceinline__ void add_run_offsets(float tot, float *out, int b, in
         if (lane < nwarps) s_warp[lane] = wex;
     }
     __syncthreads();
+    if (warp >= nwarps) return;  // threads past the first kSampleThreads hold no run
     const float base = s_warp[warp] + ex;
     for (int j = b; j < e; ++j) out[j] = base + out[j];
 }
@@ -461,6 +462,14 @@ __global__ void __launch_bounds__(kSampleThreads, MINB) sample_kernel(const Samp
 // another token's draw.
 constexpr int kUnit = kLaneEntries;               // entries per unit: two 16-byte loads
 constexpr int kFlatWarps = kSampleThreads / 32;
+// The wide form of the flat kernel, for work lists that leave most SMs idle: the
+// launch lasts as long as its longest item, whose chunks go to 16 warps instead
+// of 4.  8k tokens, K = 64, 33 items past the warp kernel's: 25.9 -> 15.5 us; 36k
+// tokens, K = 256, 134 items: 33.5 -> 21.5; 90k tokens, K = 256, 326 items: 44.5
+// -> 32.0.  From K = 512 on the row builds count for more: 332 items at K = 1024
+// take 47 us in the narrow form, 49 in the wide one.
+constexpr int kWideThreads = 512, kWideBlocks = 2;
+static bool wide_form(int k, int items, int sms) { return items <= (k < 512 ? 4 : 1) * sms; }
 constexpr int kFlatSegs = 32;                     // segments a warp takes at a time
 constexpr int kFlatMeta = 2 * (kFlatSegs + 1) + 4 * kFlatSegs;  // ints of per-warp segment data
 constexpr int kWalkLanes = 4;                     // lanes walking one range: 4 units, 128 bytes, per step
@@ -631,9 +640,10 @@ __device__ __forceinline__ float dense_block_run(const float *ph, float *qb, int
     return s + c;
 }
 
-// Each thread takes a run of blocks; add_run_offsets completes the prefix.
+// Each of the first kSampleThreads threads takes a run of blocks (so the sums do
+// not depend on the CTA's width); add_run_offsets completes the prefix.
 __device__ void dense_block_prefix(const float *ph, float *qb, int K, float alpha, float *s_warp) {
-    const int T = blockDim.x, nb = K / kDenseBlock, per = (nb + T - 1) / T;
+    const int T = kSampleThreads, nb = K / kDenseBlock, per = (nb + T - 1) / T;
     const int b0 = min((int)threadIdx.x * per, nb), b1 = min(b0 + per, nb);
     const float run = dense_block_run(ph, qb, b0, b1, alpha);
     add_run_offsets(run, qb, b0, b1, s_warp);
@@ -736,8 +746,8 @@ __device__ __forceinline__ int dense_search_tiny_blocks(const float *ph, const f
     return dense_block_scan(ph, lo, lo > 0 ? corrected(lo - 1) : 0.f, alpha, tq);
 }
 
-template <int MINB>
-__global__ void __launch_bounds__(kSampleThreads, MINB) sample_flat_kernel(const SampleParams p) {
+template <int MINB, int THREADS>
+__global__ void __launch_bounds__(THREADS, MINB) sample_flat_kernel(const SampleParams p) {
     extern __shared__ float smem[];
     const int K = p.k, KP = p.kmask + 1, B = flat_unit_budget(K);
     float *ph = smem;               // [KP] phihat of the current word (zero past K), at offset 0
@@ -746,7 +756,7 @@ __global__ void __launch_bounds__(kSampleThreads, MINB) sample_flat_kernel(const
     int *hist = reinterpret_cast<int *>(ph);
     __shared__ int s_item, s_chunk;
     __shared__ float s_warp[kSampleThreads / 32];
-    __shared__ double s_red[kSampleThreads / 32];
+    __shared__ double s_red[THREADS / 32];
     // tiny items: whether ph / qb hold the base row, and the item's topics
     __shared__ int s_tiny, s_tm;
     __shared__ __align__(16) int s_tk[kTinyTokens];
@@ -757,7 +767,7 @@ __global__ void __launch_bounds__(kSampleThreads, MINB) sample_flat_kernel(const
     const int wl = lane & (kWalkLanes - 1), wg = lane / kWalkLanes;  // lane in its walk group, group
     const unsigned wm = group_mask<kWalkLanes>(lane);
     float *ub = qb + K / kDenseBlock + warp * B;  // [B] unit prefixes of the warp's batch
-    int *m_cum = reinterpret_cast<int *>(qb + K / kDenseBlock + kFlatWarps * B) + warp * kFlatMeta;
+    int *m_cum = reinterpret_cast<int *>(qb + K / kDenseBlock + (THREADS / 32) * B) + warp * kFlatMeta;
     int *m_tc = m_cum + (kFlatSegs + 1);  // [n+1] first unit / first token (flat) of each segment
     int *m_rs = m_tc + (kFlatSegs + 1);   // [n] row start (entry index)
     int *m_t0 = m_rs + kFlatSegs;         // [n] first token
@@ -1019,7 +1029,7 @@ __global__ void __launch_bounds__(kSampleThreads, MINB) sample_flat_kernel(const
         __syncthreads();
         if (tid == 0) {
             double s = 0.0;
-            for (int w = 0; w < kSampleThreads / 32; ++w) s += s_red[w];
+            for (int w = 0; w < THREADS / 32; ++w) s += s_red[w];
             p.item_ll[it] = s;
         }
         // a tiny item's topics back to the base row (every draw of it is done)
@@ -1470,11 +1480,14 @@ __global__ void __launch_bounds__(32, 20) sample_warp_kernel(const SampleParams 
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// ph[pow2(K)] + qb[K/8] + per warp: unit prefixes and segment data
+static size_t flat_smem_bytes(int k, int warps) {
+    return ((size_t)k / kDenseBlock + (size_t)pow2_ceil(k) + (size_t)warps * (flat_unit_budget(k) + kFlatMeta)) *
+           sizeof(float);
+}
+
 size_t sample_smem_bytes(int k, int group_lanes) {
-    if (group_lanes == kFlatLanes)  // ph[pow2(K)] + qb[K/8] + per warp: unit prefixes and segment data
-        return ((size_t)k / kDenseBlock + (size_t)pow2_ceil(k) + (size_t)kFlatWarps * flat_unit_budget(k) +
-                (size_t)kFlatWarps * kFlatMeta) *
-               sizeof(float);
+    if (group_lanes == kFlatLanes) return flat_smem_bytes(k, kFlatWarps);
     // ph[pow2(K)] + inv[K] + qc[K] + the per-group running sums
     return ((size_t)2 * k + (size_t)pow2_ceil(k) + (size_t)SampleShape<1>::kPrefixFloats) * sizeof(float);
 }
@@ -1486,8 +1499,10 @@ static const void *sample_fn() {
 
 static const void *sample_kernel_for(int g, int minb) {
     if (g == kFlatLanes) {
-        if (minb == kSampleBlocksDefault) return reinterpret_cast<const void *>(&sample_flat_kernel<kSampleBlocksDefault>);
-        if (minb == kFlatBlocks) return reinterpret_cast<const void *>(&sample_flat_kernel<kFlatBlocks>);
+        if (minb == kSampleBlocksDefault)
+            return reinterpret_cast<const void *>(&sample_flat_kernel<kSampleBlocksDefault, kSampleThreads>);
+        if (minb == kFlatBlocks)
+            return reinterpret_cast<const void *>(&sample_flat_kernel<kFlatBlocks, kSampleThreads>);
         return nullptr;
     }
     if (minb == kSampleBlocksDefault) switch (g) {
@@ -1517,6 +1532,11 @@ int sample_blocks_per_sm(int k, int group_lanes, int blocks_per_sm) {
     if (!fn) return 0;
     const size_t smem = sample_smem_bytes(k, group_lanes);
     if (allow_smem(fn, smem, nullptr) != cudaSuccess) return 0;
+    // launch_sample may choose the wide form, also while a stream is captured
+    if (group_lanes == kFlatLanes &&
+        allow_smem(reinterpret_cast<const void *>(&sample_flat_kernel<kWideBlocks, kWideThreads>),
+                   flat_smem_bytes(k, kWideThreads / 32), nullptr) != cudaSuccess)
+        return 0;
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kSampleThreads, smem) != cudaSuccess) return 0;
     return n;
@@ -1533,17 +1553,25 @@ int32_t first_warp_item(const culda_item *items, int32_t n) {
 }
 
 cudaError_t launch_sample(const SampleParams &p, int group_lanes, int blocks_per_sm, int grid, cudaStream_t s) {
-    const size_t smem = sample_smem_bytes(p.k, group_lanes);
+    size_t smem = sample_smem_bytes(p.k, group_lanes);
     const void *fn = sample_kernel_for(group_lanes, blocks_per_sm);
     if (!fn) return cudaErrorInvalidValue;
-    cudaError_t e = allow_smem(fn, smem, s);
-    if (e != cudaSuccess) return e;
     SampleParams head = p;
     const int first = group_lanes == kFlatLanes && p.warp_counter ? std::min(p.first_warp, p.num_items) : p.num_items;
     head.num_items = first;
+    int dev = 0, bps = 0, threads = kSampleThreads;
+    cudaGetDevice(&dev);
+    if (group_lanes == kFlatLanes && wide_form(p.k, first, num_sms(dev))) {
+        fn = reinterpret_cast<const void *>(&sample_flat_kernel<kWideBlocks, kWideThreads>);
+        threads = kWideThreads;
+        smem = flat_smem_bytes(p.k, kWideThreads / 32);
+        grid = first;
+    }
+    cudaError_t e = allow_smem(fn, smem, s);
+    if (e != cudaSuccess) return e;
     if (first > 0) {
         void *args[] = {&head};
-        e = cudaLaunchKernel(fn, dim3(std::min(grid, first)), dim3(kSampleThreads), args, smem, s);
+        e = cudaLaunchKernel(fn, dim3(std::min(grid, first)), dim3(threads), args, smem, s);
         if (e != cudaSuccess || first == p.num_items) return e;
     }
     // the small items: their CTAs start on what room the first kernel leaves
@@ -1553,8 +1581,6 @@ cudaError_t launch_sample(const SampleParams &p, int group_lanes, int blocks_per
     const void *wfn = reinterpret_cast<const void *>(&sample_warp_kernel);
     e = allow_smem(wfn, wsmem, s);
     if (e != cudaSuccess) return e;
-    int dev = 0, bps = 0;
-    cudaGetDevice(&dev);
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, wfn, 32, wsmem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
@@ -1644,29 +1670,45 @@ cudaError_t launch_finalize_ll(double *item_ll, int num_items, DevStats *st, int
     return cudaGetLastError();
 }
 
-// ------------------------------------------------- theta entry validation
+// ------------------------------------------------- theta and list validation
 // Every entry of every row must carry a topic below K (as a byte offset) and
 // rows must be 32-aligned inside the array: checked before the kernel-level
-// entry point samples a caller's theta.
-__global__ void check_theta_kernel(int num_docs, int K, const int2 *__restrict__ rows,
-                                   const ThetaEntry *__restrict__ theta, int64_t cap, int32_t *error) {
+// entry point samples a caller's theta.  The caller's work list may be in any
+// order; where its small items come last, as culda_build_items orders them, a
+// warp each takes them.
+__global__ void check_sample_kernel(int num_docs, int K, const int2 *__restrict__ rows,
+                                    const ThetaEntry *__restrict__ theta, int64_t cap,
+                                    const culda_item *__restrict__ items, int num_items, int32_t *out) {
     const int lane = threadIdx.x & 31;
-    for (int d = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; d < num_docs; d += (gridDim.x * blockDim.x) >> 5) {
+    const int t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+    int small = 0, large = 0;
+    for (int i = t0; i < num_items; i += nt) {
+        if (items[i].count <= kWarpItemTokens)
+            small = max(small, num_items - i);
+        else
+            large = max(large, i + 1);
+    }
+    small = __reduce_max_sync(0xffffffffu, small);
+    large = __reduce_max_sync(0xffffffffu, large);
+    if (lane == 0 && small) atomicMax(&out[1], small);
+    if (lane == 0 && large) atomicMax(&out[2], large);
+    for (int d = t0 >> 5; d < num_docs; d += nt >> 5) {
         const int2 r = rows[d];
         if (r.x < 0 || r.y < r.x || (int64_t)r.y > cap || ((r.x | r.y) & 31)) {
-            if (lane == 0) atomicOr(error, kErrRowRange);
+            if (lane == 0) atomicOr(&out[0], kErrRowRange);
             continue;
         }
         for (int i = r.x + lane; i < r.y; i += 32) {
             const ThetaEntry e = theta[i];
-            if ((e & 0x30000u) || (e >> 18) >= (uint32_t)K) atomicOr(error, kErrTopicRange);
+            if ((e & 0x30000u) || (e >> 18) >= (uint32_t)K) atomicOr(&out[0], kErrTopicRange);
         }
     }
 }
 
-cudaError_t launch_check_theta(int num_docs, int k, const int2 *rows, const ThetaEntry *theta, int64_t cap,
-                               int32_t *error, cudaStream_t s) {
-    check_theta_kernel<<<grid_for((int64_t)num_docs * 32), 256, 0, s>>>(num_docs, k, rows, theta, cap, error);
+cudaError_t launch_check_sample(int num_docs, int k, const int2 *rows, const ThetaEntry *theta, int64_t cap,
+                                const culda_item *items, int num_items, int32_t *out, cudaStream_t s) {
+    check_sample_kernel<<<grid_for((int64_t)num_docs * 32), 256, 0, s>>>(num_docs, k, rows, theta, cap, items,
+                                                                        num_items, out);
     return cudaGetLastError();
 }
 

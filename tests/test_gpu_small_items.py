@@ -1,7 +1,8 @@
 """Work items of at most 32 tokens are sampled by a kernel of their own (a warp
-per item).  Its draws must equal, bit for bit, those of the CTA-per-item kernel
-that the kernel-level entry point uses for every item: the same corpus in the
-same token order, topics, uniforms and work list on both sides."""
+per item) when they come last in the work list, and short lists by CTAs of 16
+warps instead of 4.  The draws must equal, bit for bit, those of the narrow CTAs
+that the kernel-level entry point uses for every item of a long list in another
+order: the same corpus in the same token order, topics, uniforms and items."""
 from __future__ import annotations
 
 import ctypes as C
@@ -31,12 +32,14 @@ def corpus(rng, lens, docs, long_docs):
 
 
 @pytest.mark.parametrize("k", [32, 64, 512, 1024, 2048, 4096])
-@pytest.mark.parametrize("long_docs", [1, 12])
-def test_small_items_draw_as_the_cta_kernel(k, long_docs):
+@pytest.mark.parametrize("long_docs,large", [(1, 0), (12, 150), (12, 700)])
+@pytest.mark.parametrize("shuffled", [False, True])
+def test_small_items_draw_as_the_cta_kernel(k, long_docs, large, shuffled):
     import torch
 
     rng = np.random.default_rng(k + long_docs)
-    lens = np.concatenate([np.arange(0, 70), rng.integers(1, 33, 3000), [1500], np.full(300, 1), [33, 32, 31]])
+    lens = np.concatenate([np.arange(0, 70), rng.integers(1, 33, 3000), [1500], np.full(300, 1), [33, 32, 31],
+                           rng.integers(33, 90, large)])
     c = corpus(rng, lens, 400, long_docs)
     z = O.init_topics(c.num_tokens, k, 5)
     with cb.LDA(c, k, 0.05, 0.01, seed=9, flags=cb.CULDA_FLAG_NO_REORDER) as m:
@@ -45,6 +48,9 @@ def test_small_items_draw_as_the_cta_kernel(k, long_docs):
         item_tokens = m.info()["item_tokens"]
     p = prepare(c, k, 0.05, 0.01, z, item_tokens=item_tokens)
     assert update_theta(p) == 0
+    if shuffled:  # a small item first: every item takes a CTA
+        items = np.frombuffer(bytes(p.items), dtype=np.uint8).reshape(p.num_items, -1)
+        p.d["items"] = torch.from_numpy(np.ascontiguousarray(items[::-1])).cuda()
     a = sample_args(p, seed=9, iteration=4, group_lanes=_ffi.CULDA_SAMPLER_FLAT)
     ws = torch.zeros(cb.lib().culda_sample_workspace(k, p.num_items, p.num_hot) // 4 + 64, dtype=torch.int32,
                      device="cuda")
