@@ -55,8 +55,11 @@ __device__ __forceinline__ float fsum(float a, float b) { return __fadd_rn(a, b)
 // Each thread holds the local inclusive sums of its run out[b, e) and their
 // total `tot`; adds to the run the totals of all earlier threads (Kogge-Stone
 // shuffles inside a warp, then across the warps).  Ends without a barrier.
+// wide: only the first kSampleThreads threads of the CTA hold runs.
+template <bool wide = false>
 __device__ __forceinline__ void add_run_offsets(float tot, float *out, int b, int e, float *s_warp) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = kSampleThreads / 32;
+    const int T = wide ? kSampleThreads : blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5,
+              nwarps = T >> 5;
     float incl = tot;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -65,7 +68,7 @@ __device__ __forceinline__ void add_run_offsets(float tot, float *out, int b, in
     }
     float ex = __shfl_up_sync(0xffffffffu, incl, 1);
     if (lane == 0) ex = 0.f;
-    if (lane == 31 && warp < nwarps) s_warp[warp] = incl;
+    if (lane == 31 && (!wide || warp < nwarps)) s_warp[warp] = incl;
     __syncthreads();
     if (warp == 0) {
         float w = lane < nwarps ? s_warp[lane] : 0.f;
@@ -79,7 +82,7 @@ __device__ __forceinline__ void add_run_offsets(float tot, float *out, int b, in
         if (lane < nwarps) s_warp[lane] = wex;
     }
     __syncthreads();
-    if (warp >= nwarps) return;  // threads past the first kSampleThreads hold no run
+    if (wide && warp >= nwarps) return;
     const float base = s_warp[warp] + ex;
     for (int j = b; j < e; ++j) out[j] = base + out[j];
 }
@@ -640,13 +643,15 @@ __device__ __forceinline__ float dense_block_run(const float *ph, float *qb, int
     return s + c;
 }
 
-// Each of the first kSampleThreads threads takes a run of blocks (so the sums do
-// not depend on the CTA's width); add_run_offsets completes the prefix.
+// Each thread takes a run of blocks, in a wide CTA each of the first
+// kSampleThreads (so the sums do not depend on the width); add_run_offsets
+// completes the prefix.
+template <bool wide>
 __device__ void dense_block_prefix(const float *ph, float *qb, int K, float alpha, float *s_warp) {
-    const int T = kSampleThreads, nb = K / kDenseBlock, per = (nb + T - 1) / T;
+    const int T = wide ? kSampleThreads : blockDim.x, nb = K / kDenseBlock, per = (nb + T - 1) / T;
     const int b0 = min((int)threadIdx.x * per, nb), b1 = min(b0 + per, nb);
     const float run = dense_block_run(ph, qb, b0, b1, alpha);
-    add_run_offsets(run, qb, b0, b1, s_warp);
+    add_run_offsets<wide>(run, qb, b0, b1, s_warp);
     __syncthreads();
 }
 
@@ -811,7 +816,7 @@ __global__ void __launch_bounds__(THREADS, MINB) sample_flat_kernel(const Sample
                 for (int j = tid; j < K; j += blockDim.x)
                     ph[j] = (0.f + p.beta) * (1.0f / ((float)__ldg(p.nk + j) + p.vbeta));
                 __syncthreads();
-                dense_block_prefix(ph, qb, K, p.alpha, s_warp);
+                dense_block_prefix<(THREADS > kSampleThreads)>(ph, qb, K, p.alpha, s_warp);
                 if (tid == 0) s_tiny = 1;
             }
             if (warp == 0) {
@@ -857,7 +862,7 @@ __global__ void __launch_bounds__(THREADS, MINB) sample_flat_kernel(const Sample
             for (int j = tid; j < K; j += blockDim.x)
                 ph[j] = ((float)src[j] + p.beta) * (p.inv ? __ldg(p.inv + j) : 1.0f / ((float)__ldg(p.nk + j) + p.vbeta));
             __syncthreads();
-            dense_block_prefix(ph, qb, K, p.alpha, s_warp);
+            dense_block_prefix<(THREADS > kSampleThreads)>(ph, qb, K, p.alpha, s_warp);
             Q = qb[K / kDenseBlock - 1];
             if (tid == 0) s_tiny = 0;  // read by every thread before the barrier above
         }
