@@ -1364,15 +1364,17 @@ extern "C" int culda_loglik_joint(culda_ctx *ctx, double *ll) {
     p.items = ctx->d_items;
     p.hot_phi = ctx->d_hot_phi;
     p.topics = ctx->d_z[ctx->cur];
-    p.rows = ctx->d_rows;
     p.theta = ctx->d_theta;
+    p.theta_cap = ctx->theta_cap;
     p.doc_ptr = ctx->d_doc_ptr;
     p.nk = ctx->d_nk[ctx->cur];
     p.partials = ctx->d_partials;
-    p.done = done_counter(ctx);
+    p.lg_alpha = std::lgamma(p.alpha);
+    p.lg_beta = std::lgamma(p.beta);
+    p.counts = reinterpret_cast<uint32_t *>(ctx->d_partials + kMaxPartials - 512);  // past the CTAs' sums
     p.result = &ctx->h_stats->joint;  // pinned, mapped
     p.error = ctx->d_error;
-    CK(launch_loglik_joint(p, kMaxPartials, s));
+    CK(launch_loglik_joint(p, kMaxPartials - 512, s));
     CK(cudaStreamSynchronize(s));
     const double a = ctx->params.alpha, b = ctx->params.beta;
     *ll = ctx->h_stats->joint + (double)ctx->K * std::lgamma((double)ctx->V * b) +

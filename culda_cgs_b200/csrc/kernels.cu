@@ -780,27 +780,29 @@ cudaError_t launch_phi_head(int k, float beta, int num_words, const int32_t *phi
 // FP64 sum of  sum_{w,k: n>0} [lgamma(n_wk + beta) - lgamma(beta)]
 //            + sum_{d,k: n>0} [lgamma(n_dk + alpha) - lgamma(alpha)]
 //            - sum_d lgamma(L_d + K alpha) - sum_k lgamma(n_k + V beta).
-// Nearly all counts are small, so each CTA tabulates the two bracketed terms
-// for counts below kJointTable once; what remains is reading the topics and
-// theta (74 MB at 12.2M tokens: 11 us at the measured copy bandwidth).  Words
-// come as the sampler's work items, largest first: a warp counts an item in
-// packed 16-bit counts, a whole CTA the first num_long items (kPhiLong tokens
-// or more), and a word split over several items is read from its hot row.
-// Items, docs and topics go to fixed threads and the last CTA adds the CTAs'
-// sums in order, so the result is reproducible.  (An lgamma per non-zero, a
-// CTA per word, and one thread for the docs' terms took 1305 us at 12.2M
-// tokens and K = 1024; this form takes 101 us.)
+// A term depends on its count alone and nearly all counts are small, so the
+// kernel counts how often each count below kJointTable occurs (1, 2 and 3 in
+// registers, the others in shared memory) and multiplies at the end; what
+// remains is reading the topics and theta (74 MB at 12.2M tokens: 11 us at the
+// measured copy bandwidth).  Words come as the sampler's work items, largest
+// first: a warp counts an item's topics in packed 16-bit counts, a whole CTA the
+// first num_long items (kPhiLong tokens or more), and a word split over several
+// items is read from its hot row.  Items, theta, docs and topics go to fixed
+// threads and the last CTA adds the CTAs' sums in order, so the result is
+// reproducible.  (An lgamma per non-zero, a CTA per word, and one thread for the
+// docs' terms took 1305 us at 12.2M tokens and K = 1024; a table of the terms
+// and an FP64 sum per non-zero, few lanes at a time, 101 us; this form 71 us.)
 constexpr int kJointTable = 256;
+static_assert(kJointTable == kPhiThreads && 2 * kJointTable < kJointCounters, "a thread per tabulated count");
 
 __global__ void __launch_bounds__(kPhiThreads) loglik_joint_kernel(const JointParams p) {
-    extern __shared__ double sm_f64[];
-    double *fb = sm_f64, *fa = sm_f64 + kJointTable;  // the bracketed terms by count
-    int *coop = reinterpret_cast<int *>(sm_f64 + 2 * kJointTable);  // [K] whole-CTA histogram
+    extern __shared__ int sm_joint[];
+    int *coop = sm_joint;  // [K] whole-CTA histogram
     const int K = p.k, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     uint32_t *hist = reinterpret_cast<uint32_t *>(coop + K) + warp * (K / 2);  // this warp's packed counts
     __shared__ double red[kPhiThreads];
+    __shared__ unsigned word_of[kJointTable], doc_of[kJointTable];  // how often a count occurs
     __shared__ bool s_last;
-    const double lg_b = lgamma(p.beta), lg_a = lgamma(p.alpha);
     double s = 0.0, c = 0.0;
     auto add = [&](double x) {
         const double t = s + x;
@@ -810,21 +812,38 @@ __global__ void __launch_bounds__(kPhiThreads) loglik_joint_kernel(const JointPa
             c += (x - t) + s;
         s = t;
     };
-    auto word_term = [&](uint32_t n) { add(n < kJointTable ? fb[n] : lgamma((double)n + p.beta) - lg_b); };
-    for (int i = tid; i < kJointTable; i += kPhiThreads) {
-        fb[i] = lgamma((double)i + p.beta) - lg_b;
-        fa[i] = lgamma((double)i + p.alpha) - lg_a;
-    }
+    unsigned w1 = 0, w2 = 0, w3 = 0, d1 = 0, d2 = 0, d3 = 0;
+    auto word_term = [&](uint32_t n) {
+        w1 += n == 1u;
+        w2 += n == 2u;
+        w3 += n == 3u;
+        if (n > 3u) {
+            if (n < kJointTable)
+                atomicAdd(&word_of[n], 1u);
+            else
+                add(lgamma((double)n + p.beta) - p.lg_beta);
+        }
+    };
+    auto doc_term = [&](uint32_t e) {
+        const uint32_t n = e & 0xFFFFu;
+        d1 += n == 1u;
+        d2 += n == 2u;
+        d3 += n == 3u;
+        if (n > 3u) {
+            if (n < kJointTable)
+                atomicAdd(&doc_of[n], 1u);
+            else
+                add(lgamma((double)n + p.alpha) - p.lg_alpha);
+        }
+    };
+    word_of[tid] = doc_of[tid] = 0u;
     for (int j = tid; j < K + kPhiWarps * (K / 2); j += kPhiThreads) coop[j] = 0;
     __syncthreads();
     for (int i = blockIdx.x; i < p.num_long; i += gridDim.x) {
         const culda_item it = p.items[i];
         if (it.hot >= 0) {
             if (it.first)
-                for (int j = tid; j < K; j += kPhiThreads) {
-                    const uint32_t n = (uint32_t)p.hot_phi[(size_t)it.hot * K + j];
-                    if (n) word_term(n);
-                }
+                for (int j = tid; j < K; j += kPhiThreads) word_term((uint32_t)p.hot_phi[(size_t)it.hot * K + j]);
             continue;  // the same branch in every thread
         }
         const int64_t e = it.begin + it.count;
@@ -843,53 +862,98 @@ __global__ void __launch_bounds__(kPhiThreads) loglik_joint_kernel(const JointPa
         }
         __syncthreads();
         for (int j = tid; j < K; j += kPhiThreads) {
-            const uint32_t n = (uint32_t)coop[j];
-            if (n) word_term(n);
+            word_term((uint32_t)coop[j]);
             coop[j] = 0;
         }
         __syncthreads();
     }
-    for (int i = p.num_long + blockIdx.x * kPhiWarps + warp; i < p.num_items; i += gridDim.x * kPhiWarps) {
-        const culda_item it = p.items[i];
+    // a warp's items, the topics of the next one's first 128 tokens on their way
+    // while the current one is counted, and the item after it
+    const int stride = gridDim.x * kPhiWarps;
+    auto load_item = [&](int i) { return i < p.num_items ? p.items[i] : culda_item{0, 0, 0, -1, 0, 0, 0}; };
+    auto load_topics = [&](const culda_item &it, uint32_t z[4]) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            z[u] = it.hot < 0 && lane + 32 * u < it.count ? p.topics[it.begin + lane + 32 * u] : 0u;
+    };
+    const int i0 = p.num_long + blockIdx.x * kPhiWarps + warp;
+    culda_item it = load_item(i0), ahead = load_item(i0 + stride);
+    uint32_t z[4], next_z[4];
+    load_topics(it, z);
+    for (int i = i0; i < p.num_items; i += stride) {
+        const culda_item after = load_item(i + 2 * stride);
+        load_topics(ahead, next_z);
         if (it.hot >= 0) {
             if (it.first)
-                for (int j = lane; j < K; j += 32) {
-                    const uint32_t n = (uint32_t)p.hot_phi[(size_t)it.hot * K + j];
-                    if (n) word_term(n);
-                }
-            continue;
-        }
-        const int64_t e = it.begin + it.count;
-        for (int64_t t0 = it.begin + lane; t0 < e; t0 += 4 * 32) {
-            uint32_t z[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) z[u] = t0 + 32 * u < e ? p.topics[t0 + 32 * u] : 0u;
+                for (int j = lane; j < K; j += 32) word_term((uint32_t)p.hot_phi[(size_t)it.hot * K + j]);
+        } else if (it.count <= 128) {
+            // the tokens are few: the lane whose token came first to its topic reads the
+            // topic's count, instead of a pass over K counts
+            bool first[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                if (t0 + 32 * u >= e) continue;
-                if (z[u] < (uint32_t)K)
-                    atomicAdd(&hist[z[u] >> 1], 1u << ((z[u] & 1u) << 4));
-                else
+                const bool in = lane + 32 * u < it.count;
+                first[u] = false;
+                if (in && z[u] < (uint32_t)K) {
+                    const uint32_t sh = (z[u] & 1u) << 4;
+                    first[u] = ((atomicAdd(&hist[z[u] >> 1], 1u << sh) >> sh) & 0xFFFFu) == 0u;
+                } else if (in) {
                     atomicOr(p.error, kErrTopicRange);
+                }
             }
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (first[u]) word_term((hist[z[u] >> 1] >> ((z[u] & 1u) << 4)) & 0xFFFFu);
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (first[u]) hist[z[u] >> 1] = 0u;
+            __syncwarp();
+        } else {
+            for (int t0 = 0; t0 < it.count; t0 += 128) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int t = t0 + lane + 32 * u;
+                    if (t >= it.count) continue;
+                    const uint32_t x = t0 == 0 ? z[u] : (uint32_t)p.topics[it.begin + t];
+                    if (x < (uint32_t)K)
+                        atomicAdd(&hist[x >> 1], 1u << ((x & 1u) << 4));
+                    else
+                        atomicOr(p.error, kErrTopicRange);
+                }
+            }
+            __syncwarp();
+            for (int j = lane; j < K / 4; j += 32) {
+                const uint2 q = reinterpret_cast<const uint2 *>(hist)[j];
+                if ((q.x | q.y) == 0u) continue;
+                reinterpret_cast<uint2 *>(hist)[j] = make_uint2(0u, 0u);
+                word_term(q.x & 0xFFFFu);
+                word_term(q.x >> 16);
+                word_term(q.y & 0xFFFFu);
+                word_term(q.y >> 16);
+            }
+            __syncwarp();
         }
-        __syncwarp();
-        for (int j = lane; j < K / 4; j += 32) {
-            const uint2 q = reinterpret_cast<const uint2 *>(hist)[j];
-            if ((q.x | q.y) == 0u) continue;
-            reinterpret_cast<uint2 *>(hist)[j] = make_uint2(0u, 0u);
-            if (q.x & 0xFFFFu) word_term(q.x & 0xFFFFu);
-            if (q.x >> 16) word_term(q.x >> 16);
-            if (q.y & 0xFFFFu) word_term(q.y & 0xFFFFu);
-            if (q.y >> 16) word_term(q.y >> 16);
-        }
-        __syncwarp();
+        it = ahead;
+        ahead = after;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) z[u] = next_z[u];
     }
-    for (int d = blockIdx.x * kPhiWarps + warp; d < p.num_docs; d += gridDim.x * kPhiWarps) {
-        const int2 r = p.rows[d];
-        for (int i = r.x + lane; i < r.y; i += 32) {
-            const uint32_t n = p.theta[i] & 0xFFFFu;
-            if (n) add(n < kJointTable ? fa[n] : lgamma((double)n + p.alpha) - lg_a);
+    // theta as one array: past the end of a row it holds zeros
+    const int64_t n4 = p.theta_cap / 4, threads = (int64_t)gridDim.x * kPhiThreads;  // capacity: a multiple of 32
+    for (int64_t i = (int64_t)blockIdx.x * kPhiThreads + tid; i < n4; i += 4 * threads) {
+        uint4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            v[u] = i + u * threads < n4 ? __ldg(reinterpret_cast<const uint4 *>(p.theta) + i + u * threads)
+                                        : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            doc_term(v[u].x);
+            doc_term(v[u].y);
+            doc_term(v[u].z);
+            doc_term(v[u].w);
         }
     }
     const double ka = (double)K * p.alpha, vb = (double)p.num_words * p.beta;
@@ -897,6 +961,22 @@ __global__ void __launch_bounds__(kPhiThreads) loglik_joint_kernel(const JointPa
         add(-lgamma((double)(p.doc_ptr[d + 1] - p.doc_ptr[d]) + ka));
     for (int k = blockIdx.x * kPhiThreads + tid; k < K; k += gridDim.x * kPhiThreads)
         add(-lgamma((double)p.nk[k] + vb));
+    // how often each count occurred, over all CTAs (the last one multiplies)
+    if (w1 | d1) {
+        atomicAdd(&word_of[1], w1);
+        atomicAdd(&doc_of[1], d1);
+    }
+    if (w2 | d2) {
+        atomicAdd(&word_of[2], w2);
+        atomicAdd(&doc_of[2], d2);
+    }
+    if (w3 | d3) {
+        atomicAdd(&word_of[3], w3);
+        atomicAdd(&doc_of[3], d3);
+    }
+    __syncthreads();
+    if (word_of[tid]) atomicAdd(&p.counts[tid], word_of[tid]);
+    if (doc_of[tid]) atomicAdd(&p.counts[kJointTable + tid], doc_of[tid]);
     auto block_sum = [&](double x) {
         red[tid] = x;
         __syncthreads();
@@ -909,29 +989,32 @@ __global__ void __launch_bounds__(kPhiThreads) loglik_joint_kernel(const JointPa
     if (tid == 0) {
         p.partials[blockIdx.x] = red[0];
         __threadfence();
-        s_last = atomicAdd(p.done, 1) == (int)gridDim.x - 1;
+        s_last = atomicAdd(&p.counts[2 * kJointTable], 1u) == gridDim.x - 1;
     }
     __syncthreads();
     if (!s_last) return;
     __threadfence();
     s = c = 0.0;
     for (int i = tid; i < (int)gridDim.x; i += kPhiThreads) add(__ldcg(p.partials + i));
+    // count tid's terms, for the words and for the docs
+    const unsigned nw = __ldcg(p.counts + tid), nd = __ldcg(p.counts + kJointTable + tid);
+    if (nw) add((double)nw * (lgamma((double)tid + p.beta) - p.lg_beta));
+    if (nd) add((double)nd * (lgamma((double)tid + p.alpha) - p.lg_alpha));
     block_sum(s + c);
     if (tid == 0) *p.result = red[0];
 }
 
 cudaError_t launch_loglik_joint(const JointParams &p, int max_partials, cudaStream_t s) {
-    const size_t smem = 2 * kJointTable * sizeof(double) +
-                        ((size_t)p.k + (size_t)kPhiWarps * (size_t)(p.k / 2)) * sizeof(int);
+    const size_t smem = ((size_t)p.k + (size_t)kPhiWarps * (size_t)(p.k / 2)) * sizeof(int);
     cudaError_t e = allow_smem(reinterpret_cast<const void *>(&loglik_joint_kernel), smem, s);
     if (e != cudaSuccess) return e;
     int dev = 0, bps = 0;
     cudaGetDevice(&dev);
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, loglik_joint_kernel, kPhiThreads, smem);
     if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(p.done, 0, sizeof(int32_t), s);
+    e = cudaMemsetAsync(p.counts, 0, kJointCounters * sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
-    // no more CTAs than have a warp's worth of words or docs each: every CTA forms its own tables
+    // no more CTAs than have a warp's worth of words or docs each
     const int64_t need = ((int64_t)std::max(p.num_items, p.num_docs) + kPhiWarps - 1) / kPhiWarps;
     const int grid = (int)std::max<int64_t>(
         1, std::min<int64_t>(std::min(max_partials, num_sms(dev) * std::max(bps, 1)), need));

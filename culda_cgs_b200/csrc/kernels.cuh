@@ -171,19 +171,20 @@ cudaError_t launch_doc_check(int64_t n, int num_docs, const int32_t *doc_ids, in
 
 // Joint log-likelihood (see kernels.cu): items are the sampler's work list,
 // largest first, with the hot rows of the current topics.
+constexpr int kJointCounters = 513;
 struct JointParams {
     int32_t k, num_words, num_docs;
     int32_t num_items, num_long;  // num_long: long_items() of the list
-    double alpha, beta;
+    double alpha, beta, lg_alpha, lg_beta;  // and their lgamma
     const culda_item *items;
     const int32_t *hot_phi;
     const uint16_t *topics;
-    const int2 *rows;
     const ThetaEntry *theta;
+    int64_t theta_cap;  // entries; those past the end of a row are zero
     const int64_t *doc_ptr;
     const int32_t *nk;
     double *partials;  // one per CTA
-    int32_t *done;     // CTAs finished (cleared by the launch)
+    uint32_t *counts;  // [kJointCounters], cleared by the launch
     double *result;    // receives the sum; may be mapped host memory
     int32_t *error;
 };
