@@ -1397,8 +1397,11 @@ extern "C" int culda_get_info(const culda_ctx *ctx, culda_info *info) {
     info->theta_long_docs = ctx->theta_long;
     info->theta_tune_ms = ctx->theta_tune_ms;
     info->theta_grid = ctx->theta_grid;
-    // hot_rows (when words are split), prologue, sample, theta_rebuild
-    info->kernels_per_iteration = (ctx->num_hot > 0 ? 1 : 0) + 3;
+    // hot_rows (when words are split), prologue, the sampler (two kernels when the
+    // flat walk has items for both), theta_rebuild
+    info->kernels_per_iteration =
+        (ctx->num_hot > 0 ? 1 : 0) + 3 +
+        (ctx->group_lanes == kFlatLanes && ctx->first_warp > 0 && ctx->first_warp < ctx->num_items ? 1 : 0);
     info->theta_capacity = ctx->theta_cap;
     const int64_t N = ctx->N, D = ctx->D, V = ctx->V, K = ctx->K;
     (void)N;

@@ -704,7 +704,8 @@ __global__ void __launch_bounds__(kPhiThreads) update_phi_kernel(int K, int V, c
 cudaError_t launch_update_phi(int k, int num_words, const int64_t *word_ptr, const uint16_t *topics, int32_t *phi,
                               int32_t *nk, int32_t *error, cudaStream_t s) {
     const size_t smem = (2 * (size_t)k + (size_t)kPhiWarps * (size_t)(k / 2)) * sizeof(int);
-    cudaError_t e = allow_smem(reinterpret_cast<const void *>(&update_phi_kernel), smem, s);
+    // set also while s is being captured: the entry point may be captured at any K
+    cudaError_t e = allow_smem(reinterpret_cast<const void *>(&update_phi_kernel), smem, nullptr);
     if (e != cudaSuccess) return e;
     int dev = 0, bps = 0;
     cudaGetDevice(&dev);

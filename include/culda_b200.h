@@ -221,7 +221,7 @@ typedef struct culda_iter_stats {
     int64_t row_entries;    /* sum over tokens of the padded theta row length of the rebuilt state */
     int64_t theta_nnz;      /* non-zeros in theta after the rebuild */
     int64_t token_nnz;      /* sum over tokens of the non-zeros in their doc's rebuilt row */
-    double sample_seconds;  /* device time of the sampler kernel */
+    double sample_seconds;  /* device time of the sampler kernels (the GPU's timer) */
     double rebuild_seconds; /* device time of the theta / n_k rebuild */
     double accept_rate;     /* Metropolis-Hastings iterations: accepted moves / proposals (else 0) */
 } culda_iter_stats;
@@ -238,7 +238,9 @@ int culda_create(const culda_corpus *c, const culda_params *p, culda_ctx **out);
 
 /* Run n iterations (sample, log-likelihood, rebuild counts), one CUDA graph
  * launch each, writing one culda_iter_stats per iteration into stats (may be
- * NULL).  Replaces the loop body SingleChunkSingleGPU.h:70-127. */
+ * NULL).  A few iterations are queued ahead of the host; when one reports a
+ * device error, those behind it have run too.  Replaces the loop body
+ * SingleChunkSingleGPU.h:70-127. */
 int culda_iterate(culda_ctx *ctx, int n, culda_iter_stats *stats);
 
 /* Replace all topics from a host array and rebuild the counts. */

@@ -49,3 +49,29 @@ def test_update_phi_and_phi_head(k, shift):
         assert (head[:shift] == -1).all() and (head[shift + v * k:] == -1).all()
         den = want.sum(0).astype(np.float32) + np.float32(beta * np.float32(v))
         assert np.array_equal(head[shift:shift + v * k].reshape(v, k), (want.astype(np.float32) + beta) / den)
+
+
+@pytest.mark.parametrize("k", [4096])
+def test_tables_in_a_captured_stream(k):
+    """The two entry points can be captured into a graph, at any K."""
+    import torch
+
+    rng = np.random.default_rng(1)
+    lens = rng.integers(0, 40, 200)
+    v, n = len(lens), int(lens.sum())
+    z = rng.integers(0, k, n).astype(np.uint16)
+    d_ptr = torch.from_numpy(np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)).cuda()
+    d_z = torch.from_numpy(z.view(np.int16)).cuda()
+    phi, head = torch.zeros(v, k, dtype=torch.int32, device="cuda"), torch.zeros(v, k, device="cuda")
+    nk = torch.zeros(k, dtype=torch.int32, device="cuda")
+    g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(g, stream=s):
+        assert cb.lib().culda_update_phi(k, v, d_ptr.data_ptr(), d_z.data_ptr(), phi.data_ptr(), nk.data_ptr(),
+                                         s.cuda_stream) == 0
+        assert cb.lib().culda_compute_phi_head(k, 0.01, v, phi.data_ptr(), nk.data_ptr(), head.data_ptr(),
+                                               s.cuda_stream) == 0
+    g.replay()
+    torch.cuda.synchronize()
+    want = np.bincount(np.repeat(np.arange(v), lens) * k + z, minlength=v * k).reshape(v, k)
+    assert np.array_equal(phi.cpu().numpy(), want) and np.array_equal(nk.cpu().numpy(), want.sum(0))
+    assert (head.cpu().numpy() > 0).all()
