@@ -195,6 +195,17 @@ __device__ __forceinline__ bool item_ok(const MHParams &p, const culda_item &ite
 // 413 us at 48 (spills); reading each search's 128-byte stretch with eight
 // lanes and probing comparison bits instead of memory takes 32 registers more
 // and was slower (497 us): the probes after the first hit the L1.
+// They do while the L1 holds a warp's 32 stretches from probe to probe.  Once
+// the tables are well past the L2, the reads' latency keeps so many stretches
+// alive that they drive one another out, and fewer warps are faster: from
+// kMHTableL2 times the L2 on an SM takes kMHTableBlocks CTAs.  Two steps at 61M
+// tokens: K = 1024 (1.8 GB) 7.98 ms with 8 CTAs, 7.03 with 6, 7.05 with 5; K =
+// 512 (0.9 GB) 6.84, 6.14, 6.24; but at 12M tokens, K = 1024 (0.37 GB) 1.08,
+// 1.11, 1.20.  For the same room cnt lies in ph's place (8.44 -> 7.85 ms at 8
+// CTAs).  With such tables a chain of more than two steps also keeps what it
+// read of its topic while it stays there (kKeep; eight steps 25.7 -> 22.4 ms;
+// it costs 3% at two steps and gives nothing at 12M tokens).
+constexpr int kMHTableL2 = 4, kMHTableBlocks = 6;
 constexpr int kMHStepThreads = 128;
 constexpr int kMHWarps = kMHStepThreads / 32;
 
@@ -233,7 +244,7 @@ __device__ __forceinline__ int doc_proposal(const MHParams &p, const MHToken &to
 
 // The steps of up to 32 tokens, lane l's at t, against the word's phihat.  The
 // whole warp takes part.
-template <class PhiHat>
+template <bool kKeep, class PhiHat>
 __device__ __forceinline__ void mh_tokens(const MHParams &p, const MHToken &tok, int64_t t, const PhiHat &ph, int lane,
                                           unsigned &acc_n, unsigned &prop_n) {
     const int K = p.k, nb = K >> 5;
@@ -241,6 +252,9 @@ __device__ __forceinline__ void mh_tokens(const MHParams &p, const MHToken &tok,
     const bool active = tok.d >= 0;
     const int d = max(tok.d, 0);
     int s = tok.s;
+    // q_d and n_dk of the topic s_read, where the chain stood when they were read
+    float q_s = 0.f, n_s = 0.f;
+    int s_read = -1;
     for (int step = 0; step < p.steps; step += 2) {
         const bool two = step + 1 < p.steps, enc = two && p.cdf;
         const u32x4 x0 = philox_token4(p.seed, tok.key, p.iteration, kPurposeMH + (uint32_t)step);
@@ -254,6 +268,14 @@ __device__ __forceinline__ void mh_tokens(const MHParams &p, const MHToken &tok,
             total = __ldg(blk + nb - 1);
         else if (two)
             i1 = doc_proposal(p, tok, x1, ka, k1);
+        const uint16_t *nd = p.ndk + (size_t)d * K;
+        auto read_s = [&] {
+            if (!kKeep || s != s_read) {
+                q_s = __ldg(row + s) - (s > 0 ? __ldg(row + s - 1) : 0.f);
+                n_s = (float)nd[s];
+                s_read = s;
+            }
+        };
         if (i0 >= 0) k0 = p.topics_in[i0];
         if (i1 >= 0) k1 = p.topics_in[i1];
         if (enc) {
@@ -273,15 +295,14 @@ __device__ __forceinline__ void mh_tokens(const MHParams &p, const MHToken &tok,
             accept(k0, ph(k0) / ph(s), x0.z);
         }
         if (enc) {
-            const uint16_t *nd = p.ndk + (size_t)d * K;
-            const float at_s = __ldg(row + s), before_s = s > 0 ? __ldg(row + s - 1) : 0.f;
-            const float n_s = (float)nd[s];
             const float qk = __ldg(row + k1) - (k1 > 0 ? __ldg(row + k1 - 1) : 0.f);
-            const float qs = at_s - before_s;
+            const float n_k = (float)nd[k1];
+            read_s();
             if (active) {
-                const float pk = ((float)nd[k1] + p.alpha) * ph(k1);
+                const float pk = (n_k + p.alpha) * ph(k1);
                 const float ps = (n_s + p.alpha) * ph(s);
-                accept(k1, (pk * qs) / (ps * qk), x1.z);
+                accept(k1, (pk * q_s) / (ps * qk), x1.z);
+                if (kKeep && s == k1) q_s = qk, n_s = n_k, s_read = k1;
             }
         } else if (two && active) {
             if ((unsigned)k1 >= (unsigned)K) k1 = s;
@@ -293,31 +314,31 @@ __device__ __forceinline__ void mh_tokens(const MHParams &p, const MHToken &tok,
 
 // Tokens [begin, end) of an item, 32 at a time `stride` apart, the next 32
 // loaded ahead.
-template <class PhiHat>
+template <bool kKeep, class PhiHat>
 __device__ __forceinline__ void mh_run(const MHParams &p, int64_t begin, int64_t end, int stride, const PhiHat &ph,
                                        int lane, unsigned &acc_n, unsigned &prop_n) {
     MHToken tok = mh_load(p, begin + lane < end, begin + lane);
     for (int64_t t0 = begin; t0 < end; t0 += stride) {
         const int64_t tn = t0 + stride + lane;
         const MHToken next = mh_load(p, tn < end, tn);
-        mh_tokens(p, tok, t0 + lane, ph, lane, acc_n, prop_n);
+        mh_tokens<kKeep>(p, tok, t0 + lane, ph, lane, acc_n, prop_n);
         tok = next;
     }
 }
 
+template <bool kKeep>
 __global__ void __launch_bounds__(kMHStepThreads, 8) mh_kernel(const MHParams p) {
     extern __shared__ float sm_mh[];
     const int K = p.k;
     float *inv = sm_mh;                              // [K] 1 / (n_k + V beta)
     float *ph = sm_mh + K;                           // [K] phihat of the CTA's word (its histogram before that)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    uint32_t *cnt = reinterpret_cast<uint32_t *>(sm_mh + 2 * K) + warp * (K / 2);  // the warp's word, 16-bit counts
+    uint32_t *cnt = reinterpret_cast<uint32_t *>(sm_mh + K) + warp * (K / 2);  // in ph's place later: the warp's word, 16-bit counts
     __shared__ int s_item;
     unsigned acc_n = 0, prop_n = 0;
     if (tid == 0) clock_start(p.clock);
 
     for (int j = tid; j < K; j += blockDim.x) inv[j] = 1.0f / ((float)p.nk[j] + p.vbeta);
-    for (int j = lane; j < K / 2; j += 32) cnt[j] = 0u;
     // the long items: a CTA each
     for (;;) {
         if (tid == 0) s_item = atomicAdd(p.item_counter, 1);
@@ -332,10 +353,12 @@ __global__ void __launch_bounds__(kMHStepThreads, 8) mh_kernel(const MHParams p)
         }
         item_phi_row(p, item, ph, inv, reinterpret_cast<int *>(ph));
         const int64_t iend = item.begin + item.count;
-        mh_run(p, item.begin + 32 * warp, iend, kMHStepThreads, [ph](int k) { return ph[k]; }, lane, acc_n, prop_n);
+        mh_run<kKeep>(p, item.begin + 32 * warp, iend, kMHStepThreads, [ph](int k) { return ph[k]; }, lane, acc_n, prop_n);
         __syncthreads();  // ph is rebuilt for the next item
     }
-    // the others: a warp each
+    // the others: a warp each (behind the barrier of the loop's last turn)
+    for (int j = lane; j < K / 2; j += 32) cnt[j] = 0u;
+    __syncwarp();
     for (;;) {
         int it = 0;
         if (lane == 0) it = p.num_coop + atomicAdd(p.warp_counter, 1);
@@ -351,7 +374,7 @@ __global__ void __launch_bounds__(kMHStepThreads, 8) mh_kernel(const MHParams p)
                                : item.hot >= 0 ? p.hot_phi + (size_t)item.hot * K : nullptr;
         if (fixed) {
             auto phihat = [&](int k) { return ((float)__ldg(fixed + k) + p.beta) * inv[k]; };
-            mh_run(p, item.begin, iend, 32, phihat, lane, acc_n, prop_n);
+            mh_run<kKeep>(p, item.begin, iend, 32, phihat, lane, acc_n, prop_n);
             continue;
         }
         for (int64_t t = item.begin + lane; t < iend; t += 32) {
@@ -365,7 +388,7 @@ __global__ void __launch_bounds__(kMHStepThreads, 8) mh_kernel(const MHParams p)
         auto phihat = [&](int k) {
             return ((float)((cnt[k >> 1] >> ((k & 1) << 4)) & 0xFFFFu) + p.beta) * inv[k];
         };
-        mh_run(p, item.begin, iend, 32, phihat, lane, acc_n, prop_n);
+        mh_run<kKeep>(p, item.begin, iend, 32, phihat, lane, acc_n, prop_n);
         __syncwarp();
         for (int64_t t = item.begin + lane; t < iend; t += 32) {
             const uint32_t z = p.topics_in[t];
@@ -597,11 +620,16 @@ int launch_mh_pass(culda_ctx *ctx, int cur, uint32_t iteration, int steps) {
         doc_span_kernel<<<grid_for(ctx->D), 256, 0, s>>>(ctx->D, ctx->d_doc_ptr, ctx->d_doc_span);
         CK(cudaGetLastError());
     }
-    const size_t smem = ((size_t)2 * ctx->K + (size_t)kMHWarps * (size_t)(ctx->K / 2)) * sizeof(float);
-    int grid = 1;
-    rc = persistent_grid(ctx, mh_kernel, kMHStepThreads, smem, &grid);
+    const size_t smem = ((size_t)ctx->K + (size_t)kMHWarps * (size_t)(ctx->K / 2)) * sizeof(float);  // inv, ph or cnt
+    int grid = 1, l2 = 0;
+    cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->device);
+    const size_t tables = ctx->has_proposal ? (sizeof(float) + sizeof(uint16_t)) * (size_t)ctx->D * ctx->K : 0;
+    const bool large = tables > (size_t)kMHTableL2 * (size_t)l2;
+    auto kernel = large && steps > 2 ? mh_kernel<true> : mh_kernel<false>;
+    rc = persistent_grid(ctx, kernel, kMHStepThreads, smem, &grid);
     if (rc) return rc;
-    mh_kernel<<<grid, kMHStepThreads, smem, s>>>(mh_params(ctx, cur, iteration, steps));
+    if (large) grid = std::min(grid, num_sms(ctx->device) * kMHTableBlocks);
+    kernel<<<grid, kMHStepThreads, smem, s>>>(mh_params(ctx, cur, iteration, steps));
     CK(cudaGetLastError());
     return CULDA_OK;
 }
