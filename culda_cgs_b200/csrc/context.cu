@@ -573,12 +573,15 @@ __global__ void item_segments_kernel(culda_item *items, int num_items, const int
 }
 
 // A process-wide pool of pinned slots of kStatsRing DevStats: a cudaMallocHost
-// costs milliseconds, so contexts take slots from shared pinned pages and give
-// them back on destroy (the pages live as long as the process).
+// costs milliseconds, so contexts (and encoders, which need a word) take slots from
+// shared pinned pages and give them back on destroy (the pages live as long as
+// the process).
 std::mutex g_pinned_mu;
 std::vector<DevStats *> g_pinned_free;
 
-DevStats *pinned_stats_get() {
+}  // namespace
+
+void *culda::pinned_slot_get() {
     std::lock_guard<std::mutex> lock(g_pinned_mu);
     if (g_pinned_free.empty()) {
         constexpr int kSlots = 64;
@@ -591,10 +594,12 @@ DevStats *pinned_stats_get() {
     return p;
 }
 
-void pinned_stats_put(DevStats *p) {
+void culda::pinned_slot_put(void *p) {
     std::lock_guard<std::mutex> lock(g_pinned_mu);
-    g_pinned_free.push_back(p);
+    g_pinned_free.push_back(static_cast<DevStats *>(p));
 }
+
+namespace {
 
 // A process-wide stream-ordered memory pool per device for the contexts'
 // blocks.  Its release threshold is "never", so a destroyed context's block
@@ -1115,7 +1120,7 @@ extern "C" int culda_create(const culda_corpus *c, const culda_params *p, culda_
     // theta's storage held set-up temporaries until now
     CKB(cudaMemsetAsync(ctx->d_theta, 0, sizeof(ThetaEntry) * (size_t)std::max<int64_t>(ctx->theta_cap, 1), s));
 
-    ctx->h_stats = pinned_stats_get();
+    ctx->h_stats = static_cast<DevStats *>(pinned_slot_get());
     if (!ctx->h_stats) {
         fail(ctx, CULDA_ERR_OOM, "culda_create: pinned host memory for the iteration statistics");
         return bail(CULDA_ERR_OOM);
@@ -1441,7 +1446,7 @@ extern "C" void culda_destroy(culda_ctx *ctx) {
             cudaFree(ctx->d_block);
         }
     }
-    if (ctx->h_stats) pinned_stats_put(ctx->h_stats);
+    if (ctx->h_stats) pinned_slot_put(ctx->h_stats);
     for (cudaEvent_t ev : {ctx->ev0, ctx->ev1})
         if (ev) cudaEventDestroy(ev);
     for (cudaEvent_t ev : ctx->ev_iter)

@@ -15,6 +15,7 @@
 //             dW2 = dP2^T H1,  dP1 = (dP2 W2) * GELU'(P1), db1
 //             dW1 = dP1^T X0,  dX0 = dP1 W1          FP32
 //             dE[w] = sum of dX0[b] / L_b over the tokens of w in the batch
+//                   (tokens grouped by word, one write per embedding row)
 // The weight gradients split their K range (the batch) over several CTAs
 // per tile.  Every GEMM is C = A B^T with both operands K-major, so each weight is kept
 // in BF16 twice (W and W^T) and each activation that feeds a weight gradient
@@ -22,7 +23,11 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <cub/device/device_radix_sort.cuh>
+#include <cub/device/device_scan.cuh>
+
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -167,79 +172,111 @@ __global__ void __launch_bounds__(256) embbag_fwd_kernel(int batch, int rows, co
     }
 }
 
-// The embedding gradient: dX0[b] / L_b goes to the row of each of row b's
-// words with one vector reduction per 4 columns; a run of one word (documents
-// list their words in order) takes one for the whole run.  gE holds zeros
-// before.  A CTA per batch row; documents of more than kBagLong tokens, which
-// would hold one SM's reductions long after the others' are done, are shared
-// by kBagHelpers more CTAs.  (Laying out (word, row) pairs, sorting them by word
-// and walking the sorted list was 9 launches and a read-back of the batch's
-// token count: 79 us and a 20 us wait for 102k tokens, 230 us for 836k; the
-// reductions take 24 and 159 us.)
-constexpr int kBagLong = 4096, kBagHelpers = 148;
+// The embedding gradient: the batch's (word, row) pairs are laid out in row
+// order (a scan of the row lengths), sorted by word (a radix sort, stable, so
+// a word's tokens stay in row order), and the sorted list is cut into chunks
+// of 32 tokens.  A warp walks its chunk in order, summing dX0[b] / L_b per
+// word in registers.  A word whose tokens all lie in the chunk is written with
+// plain stores; a word whose run crosses the chunk's first or last token (the
+// frequent ones) adds each chunk's partial sum with one vector atomic per
+// lane.  gE holds zeros before the pass; words outside [0, V) sort last under
+// the key V and are skipped.  So a word's terms are added in one order, but for
+// the words in several chunks, and a training run repeats but for those.
+// (Vector reductions straight to the words' rows need no sort, 24 us instead of
+// 79 for 102k tokens, but add every word's terms in the order of arrival: after
+// eight steps the weights of two runs were up to 3e-5 apart instead of 5e-6.)
 
-// Tokens [q0, q1) of a row: warps 2q and 2q + 1 take the two halves of the
-// columns for a quarter of them; g is the warp's part of dX0[b] / L_b.
-__device__ __forceinline__ void bag_scatter(int64_t q0, int64_t q1, const int32_t *__restrict__ words, int V, float4 g,
-                                            float *dst, int lane) {
-    for (int64_t tb = q0; tb < q1; tb += 32) {
-        const int w = tb + lane < q1 ? words[tb + lane] : -1;
-        const int prev = __shfl_up_sync(0xffffffffu, w, 1);
-        const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || w != prev);
-        for (unsigned m = __ballot_sync(0xffffffffu, (unsigned)w < (unsigned)V) & heads; m; m &= m - 1u) {
-            const int j = __ffs(m) - 1;
-            const unsigned after = heads & ~((2u << j) - 1u);  // the next run's start, if any
-            const float c = (float)((after ? __ffs(after) - 1 : 32) - j);
-            const int wj = __shfl_sync(0xffffffffu, w, j);
-            atomicAdd(reinterpret_cast<float4 *>(dst + (size_t)wj * kE),
-                      make_float4(c * g.x, c * g.y, c * g.z, c * g.w));
+// len[b] = L_b (for the scan of row offsets) and inv_len[b] = 1 / L_b.
+__global__ void bag_rows_kernel(int batch, const int32_t *__restrict__ docs, const int64_t *__restrict__ doc_ptr,
+                                int64_t *len, float *inv_len) {
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < batch; b += gridDim.x * blockDim.x) {
+        const int d = docs ? docs[b] : b;
+        const int64_t L = max((int64_t)0, (int64_t)(doc_ptr[d + 1] - doc_ptr[d]));
+        len[b] = L;
+        inv_len[b] = L > 0 ? 1.0f / (float)L : 0.f;
+    }
+}
+
+// key[off[b] + j] = word of the j-th token of row b (V when out of range), val = b.
+__global__ void __launch_bounds__(256) bag_pairs_kernel(int batch, const int32_t *__restrict__ docs,
+                                                        const int64_t *__restrict__ doc_ptr,
+                                                        const int32_t *__restrict__ words, int V,
+                                                        const int64_t *__restrict__ off, int32_t *key, int32_t *val) {
+    for (int b = blockIdx.x; b < batch; b += gridDim.x) {
+        const int d = docs ? docs[b] : b;
+        const int64_t t0 = doc_ptr[d], t1 = doc_ptr[d + 1];
+        const int64_t o = off[b];
+        for (int64_t t = t0 + threadIdx.x; t < t1; t += blockDim.x) {
+            const int w = words[t];
+            key[o + (t - t0)] = (unsigned)w < (unsigned)V ? w : V;
+            val[o + (t - t0)] = b;
         }
     }
 }
 
-__global__ void __launch_bounds__(256) embbag_bwd_kernel(int batch, const int32_t *__restrict__ docs,
-                                                         const int64_t *__restrict__ doc_ptr,
-                                                         const int32_t *__restrict__ words, int V,
-                                                         const float *__restrict__ dX0, float *gE) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int col = (warp & 1) * 128 + 4 * lane;
-    // part s of `parts` of row b's tokens [t0, t1)
-    auto scatter = [&](int b, int64_t t0, int64_t t1, int s, int parts) {
-        const float inv = 1.0f / (float)(t1 - t0);
-        float4 g = *reinterpret_cast<const float4 *>(dX0 + (size_t)b * kE + col);
-        g = make_float4(g.x * inv, g.y * inv, g.z * inv, g.w * inv);
-        const int64_t per = (t1 - t0 + 4 * parts - 1) / (4 * parts);
-        const int64_t q0 = min(t1, t0 + per * (4 * s + (warp >> 1))), q1 = min(t1, q0 + per);
-        bag_scatter(q0, q1, words, V, g, gE + col, lane);
-    };
-    if ((int)blockIdx.x < batch) {
-        const int b = blockIdx.x, d = docs ? docs[b] : b;
-        const int64_t t0 = doc_ptr[d], t1 = doc_ptr[d + 1];
-        if (t1 > t0 && t1 - t0 <= kBagLong) scatter(b, t0, t1, 0, 1);
-        return;
-    }
-    // the long documents, 8 rows per thread at a time
-    constexpr int kAhead = 8;
-    __shared__ int found[256 * kAhead], num_found;
-    for (int b0 = 0; b0 < batch; b0 += 256 * kAhead) {
-        if (threadIdx.x == 0) num_found = 0;
-        __syncthreads();
-        int64_t len[kAhead];
+// Warp per chunk of 32 sorted tokens; each lane holds 8 of the 256 columns.
+__global__ void embbag_bwd_grouped_kernel(int64_t n, int V, const int32_t *__restrict__ wid,
+                                          const int32_t *__restrict__ rows, const float *__restrict__ inv_len,
+                                          const float *__restrict__ dX0, float *gE) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t c0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; c0 < n; c0 += nw * 32) {
+        const int cn = (int)min((int64_t)32, n - c0);
+        const int my_w = lane < cn ? wid[c0 + lane] : V;
+        const int my_b = lane < cn ? rows[c0 + lane] : 0;
+        const float my_s = lane < cn ? inv_len[my_b] : 0.f;
+        // does the chunk's first (last) run continue from the chunk before (after) it?
+        const int w_before = c0 > 0 ? wid[c0 - 1] : -1;
+        const int w_after = c0 + cn < n ? wid[c0 + cn] : -1;
+        const int first_w = __shfl_sync(0xffffffffu, my_w, 0), last_w = __shfl_sync(0xffffffffu, my_w, cn - 1);
+        // the chunk's dX0 rows, 2 x 16 bytes per lane each, loaded 8 at a time ahead of their use
+        float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
+        float4 r0[8], r1[8];
+        for (int j = 0; j < cn; ++j) {
+            if ((j & 7) == 0) {
 #pragma unroll
-        for (int u = 0; u < kAhead; ++u) {
-            const int b = b0 + 256 * u + threadIdx.x;
-            const int d = b < batch ? (docs ? docs[b] : b) : -1;
-            len[u] = d >= 0 ? doc_ptr[d + 1] - doc_ptr[d] : 0;
-        }
+                for (int u = 0; u < 8; ++u) {
+                    const int bj = __shfl_sync(0xffffffffu, my_b, (j + u) & 31);
+                    const float4 *q = reinterpret_cast<const float4 *>(dX0 + (size_t)bj * kE) + 2 * lane;
+                    const bool in = j + u < cn;
+                    r0[u] = in ? q[0] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    r1[u] = in ? q[1] : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+            }
+            const int w = __shfl_sync(0xffffffffu, my_w, j);
+            const float sc = __shfl_sync(0xffffffffu, my_s, j);
+            float4 g0 = r0[0], g1 = r1[0];
 #pragma unroll
-        for (int u = 0; u < kAhead; ++u)
-            if (len[u] > kBagLong) found[atomicAdd(&num_found, 1)] = b0 + 256 * u + threadIdx.x;
-        __syncthreads();
-        for (int i = 0; i < num_found; ++i) {
-            const int b = found[i], d = docs ? docs[b] : b;
-            scatter(b, doc_ptr[d], doc_ptr[d + 1], blockIdx.x - batch, kBagHelpers);
+            for (int u = 1; u < 8; ++u)
+                if ((j & 7) == u) {
+                    g0 = r0[u];
+                    g1 = r1[u];
+                }
+            a0.x += g0.x * sc;
+            a0.y += g0.y * sc;
+            a0.z += g0.z * sc;
+            a0.w += g0.w * sc;
+            a1.x += g1.x * sc;
+            a1.y += g1.y * sc;
+            a1.z += g1.z * sc;
+            a1.w += g1.w * sc;
+            const int wn = __shfl_sync(0xffffffffu, my_w, (j + 1) & 31);
+            if (j + 1 == cn || wn != w) {  // the end of this word's run in the chunk
+                if (w < V) {
+                    float4 *dst = reinterpret_cast<float4 *>(gE + (size_t)w * kE) + 2 * lane;
+                    const bool shared = (w == first_w && w == w_before) || (w == last_w && w == w_after);
+                    if (!shared) {  // the whole word: no other chunk adds to it
+                        dst[0] = a0;
+                        dst[1] = a1;
+                    } else {
+                        atomicAdd(dst, a0);
+                        atomicAdd(dst + 1, a1);
+                    }
+                }
+                a0 = make_float4(0.f, 0.f, 0.f, 0.f);
+                a1 = a0;
+            }
         }
-        __syncthreads();  // the list is rewritten
     }
 }
 
@@ -442,6 +479,17 @@ struct culda_encoder {
     float *P1 = nullptr, *P2 = nullptr, *Z = nullptr, *dX0 = nullptr;
     double *d_loss = nullptr;
     int32_t *d_error = nullptr;
+    // the batch's (word, row) pairs sorted by word, for the embedding gradient
+    int64_t *bag_len = nullptr, *bag_off = nullptr;  // [Bmax + 1] row lengths and their exclusive scan
+    float *bag_inv_len = nullptr;                    // [Bmax] 1 / L of every batch row
+    int32_t *bag_key = nullptr, *bag_val = nullptr;  // [bag_cap] pairs in row order
+    int32_t *bag_wid = nullptr, *bag_rows = nullptr; // [bag_cap] the pairs sorted by word
+    int64_t bag_cap = 0;
+    void *scan_tmp = nullptr, *sort_tmp = nullptr;
+    size_t scan_tmp_bytes = 0, sort_tmp_bytes = 0;
+    int key_bits = 1;                                // bits of the keys 0..V
+    int64_t *h_tokens = nullptr;                     // pinned: a batch's token count, where the caller gave none
+    cudaEvent_t counted = nullptr;                   // it has arrived
     std::vector<void *> allocs;
 
     float *tensor(int t) { return params + off[t]; }
@@ -462,6 +510,13 @@ cudaError_t ealloc(culda_encoder *e, T **p, size_t n) {
 int fail_enc(int code, const char *fmt, const char *what) {
     set_global_error(fmt, what);
     return code;
+}
+
+void free_encoder(culda_encoder *e) {
+    for (void *q : e->allocs) cudaFree(q);
+    if (e->counted) cudaEventDestroy(e->counted);
+    if (e->h_tokens) pinned_slot_put(e->h_tokens);
+    delete e;
 }
 
 #define ECK(x)                                                                   \
@@ -543,7 +598,7 @@ int encoder_max_batch(const culda_encoder *e) { return e->Bmax; }
 int32_t *encoder_error_word(culda_encoder *e) { return e->d_error; }
 
 int encoder_pass(culda_encoder *e, int batch, const int32_t *docs, const int64_t *doc_ptr, const int32_t *words,
-                 const EncoderTarget *target, bool update, float *probs, cudaStream_t s) {
+                 const EncoderTarget *target, bool update, float *probs, cudaStream_t s, int64_t batch_tokens) {
     if (batch <= 0 || batch > e->Bmax || !doc_ptr || !words)
         return fail_enc(CULDA_ERR_INVALID_ARG, "encoder: %s", "batch outside 1..max_batch or null CSR");
     if (target && !target->dense && !target->acc)
@@ -551,6 +606,16 @@ int encoder_pass(culda_encoder *e, int batch, const int32_t *docs, const int64_t
     ECK(cudaSetDevice(e->device));
     const int Bp = (batch + 127) & ~127, K = e->K;
     int32_t *err = e->d_error;
+    if (target) {
+        // where each row's (word, row) pairs go; their number is on its way to the host during the passes
+        bag_rows_kernel<<<(batch + 255) / 256, 256, 0, s>>>(batch, docs, doc_ptr, e->bag_len, e->bag_inv_len);
+        ECK(cudaGetLastError());
+        ECK(cub::DeviceScan::ExclusiveSum(e->scan_tmp, e->scan_tmp_bytes, e->bag_len, e->bag_off, batch + 1, s));
+        if (batch_tokens < 0) {
+            ECK(cudaMemcpyAsync(e->h_tokens, e->bag_off + batch, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+            ECK(cudaEventRecord(e->counted, s));
+        }
+    }
     // forward
     // set also while s is being captured (a forward pass may be)
     ECK(allow_smem(reinterpret_cast<const void *>(&embbag_fwd_kernel), kBagSmem, nullptr));
@@ -609,9 +674,48 @@ int encoder_pass(culda_encoder *e, int batch, const int32_t *docs, const int64_t
     ECK(gemm_wgrad(kH, kE, Bp, e->dP1t, e->X0t, g1, err, s));  // dW1 = dP1^T X0
     g1.out_f32 = e->dX0;
     ECK(gemm(Bp, kE, kH, e->dP1, e->W1t, kEpiF32, g1, err, s));  // dX0 = dP1 W1
-    embbag_bwd_kernel<<<batch + kBagHelpers, 256, 0, s>>>(batch, docs, doc_ptr, words, e->V, e->dX0,
-                                                          e->grad(CULDA_ENC_E));
-    ECK(cudaGetLastError());
+    // the batch's (word, row) pairs sorted by word, then one pass over them
+    if (batch_tokens < 0) {
+        ECK(cudaEventSynchronize(e->counted));
+        batch_tokens = *e->h_tokens;
+    }
+    if (batch_tokens > INT_MAX)
+        return fail_enc(CULDA_ERR_UNSUPPORTED, "encoder: %s", "a training batch of more than 2^31 - 1 tokens");
+    if (batch_tokens > e->bag_cap) {
+        ECK(cudaStreamSynchronize(s));
+        for (void **q : {(void **)&e->bag_key, (void **)&e->bag_val, (void **)&e->bag_wid, (void **)&e->bag_rows,
+                         &e->sort_tmp}) {
+            if (*q) {
+                cudaFree(*q);
+                e->allocs.erase(std::find(e->allocs.begin(), e->allocs.end(), *q));
+                *q = nullptr;
+            }
+        }
+        const int64_t cap = std::min<int64_t>(std::max<int64_t>(batch_tokens, 2 * e->bag_cap), INT_MAX);
+        e->bag_cap = 0;
+        ECK(ealloc(e, &e->bag_key, (size_t)cap));
+        ECK(ealloc(e, &e->bag_val, (size_t)cap));
+        ECK(ealloc(e, &e->bag_wid, (size_t)cap));
+        ECK(ealloc(e, &e->bag_rows, (size_t)cap));
+        e->sort_tmp_bytes = 0;
+        ECK(cub::DeviceRadixSort::SortPairs(nullptr, e->sort_tmp_bytes, e->bag_key, e->bag_wid, e->bag_val,
+                                            e->bag_rows, (int)cap, 0, e->key_bits));
+        uint8_t *tmp = nullptr;
+        ECK(ealloc(e, &tmp, e->sort_tmp_bytes));
+        e->sort_tmp = tmp;
+        e->bag_cap = cap;
+    }
+    if (batch_tokens > 0) {
+        bag_pairs_kernel<<<std::min(batch, 148 * 16), 256, 0, s>>>(batch, docs, doc_ptr, words, e->V, e->bag_off,
+                                                                   e->bag_key, e->bag_val);
+        ECK(cudaGetLastError());
+        ECK(cub::DeviceRadixSort::SortPairs(e->sort_tmp, e->sort_tmp_bytes, e->bag_key, e->bag_wid, e->bag_val,
+                                            e->bag_rows, (int)batch_tokens, 0, e->key_bits, s));
+        embbag_bwd_grouped_kernel<<<grid_for(batch_tokens), 256, 0, s>>>(batch_tokens, e->V, e->bag_wid, e->bag_rows,
+                                                                         e->bag_inv_len, e->dX0,
+                                                                         e->grad(CULDA_ENC_E));
+        ECK(cudaGetLastError());
+    }
     if (update) {
         e->steps += 1;
         const float c1 = 1.0f / (1.0f - powf(e->b1, (float)e->steps));
@@ -723,8 +827,7 @@ extern "C" int culda_encoder_create(const culda_encoder_params *p, culda_encoder
     const size_t np = (size_t)e->off[kNumTensors];
     const size_t B = (size_t)e->Bmax, K = (size_t)e->K;
     auto bail = [&](cudaError_t r) {
-        for (void *q : e->allocs) cudaFree(q);
-        delete e;
+        free_encoder(e);
         return fail_enc(r == cudaErrorMemoryAllocation ? CULDA_ERR_OOM : CULDA_ERR_CUDA, "culda_encoder_create: %s",
                         cudaGetErrorString(r));
     };
@@ -762,6 +865,20 @@ extern "C" int culda_encoder_create(const culda_encoder_params *p, culda_encoder
     EALLOC(e->dX0, B * kE);
     EALLOC(e->d_loss, 2);  // the error word follows the loss, so one copy reads both
     e->d_error = reinterpret_cast<int32_t *>(e->d_loss + 1);
+    EALLOC(e->bag_len, (size_t)B + 1);
+    EALLOC(e->bag_off, (size_t)B + 1);
+    EALLOC(e->bag_inv_len, B);
+    while ((1u << e->key_bits) <= (unsigned)e->V) ++e->key_bits;  // keys 0..V
+    r = cub::DeviceScan::ExclusiveSum(nullptr, e->scan_tmp_bytes, e->bag_len, e->bag_off, B + 1);
+    if (r != cudaSuccess) return bail(r);
+    {
+        uint8_t *tmp = nullptr;
+        EALLOC(tmp, e->scan_tmp_bytes);
+        e->scan_tmp = tmp;
+    }
+    if (!(e->h_tokens = static_cast<int64_t *>(pinned_slot_get()))) return bail(cudaErrorMemoryAllocation);
+    r = cudaEventCreateWithFlags(&e->counted, cudaEventDisableTiming);
+    if (r != cudaSuccess) return bail(r);
 #undef EALLOC
     cudaStream_t s = nullptr;
     r = cudaMemsetAsync(e->grads, 0, sizeof(float) * np, s);
@@ -795,8 +912,7 @@ extern "C" int culda_encoder_destroy(culda_encoder *e) {
     if (!e) return CULDA_OK;
     cudaSetDevice(e->device);
     cudaDeviceSynchronize();
-    for (void *q : e->allocs) cudaFree(q);
-    delete e;
+    free_encoder(e);
     return CULDA_OK;
 }
 
@@ -843,7 +959,10 @@ static int backward_call(culda_encoder *e, int32_t batch, const int32_t *d_docs,
     EncoderTarget t;
     t.dense = d_target;
     int rc = encoder_pass(e, batch, d_docs, d_doc_ptr, d_words, &t, update, nullptr, s);
-    if (rc) return rc;
+    if (rc) {
+        encoder_take_loss(e, 0, nullptr, s);  // what the part of the pass that ran has added
+        return rc;
+    }
     return encoder_take_loss(e, batch, loss, s);
 }
 

@@ -25,6 +25,11 @@ int validate_corpus(const culda_corpus *c);
 // allocation is tried once more (returns the CUDA status).
 int device_malloc(void **p, size_t bytes);
 
+// A slot of pinned host memory (some hundred bytes) from the process-wide pool
+// that contexts take their statistics from; null when there is none.
+void *pinned_slot_get();
+void pinned_slot_put(void *p);
+
 // Device error word bits.
 enum : int32_t {
     kErrTopicRange = 1,   // a topic >= K was found in the topic array

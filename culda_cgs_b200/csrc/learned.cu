@@ -718,9 +718,14 @@ extern "C" int culda_train_encoder(culda_ctx *ctx, culda_encoder *enc, int32_t e
         const int steps = (ctx->D + B - 1) / B;
         for (int st = 0; st < steps && rc == CULDA_OK; ++st) {
             const int b0 = st * B, nb = std::min(B, ctx->D - b0);
-            rc = encoder_pass(enc, nb, d_order + b0, ctx->d_doc_ptr, ctx->d_doc_words, &tg, true, nullptr, s);
+            int64_t tokens = 0;  // the batch's tokens, known here from the host doc index
+            for (int i = b0; i < b0 + nb; ++i)
+                tokens += ctx->h_doc_ptr[(size_t)order[(size_t)i] + 1] - ctx->h_doc_ptr[(size_t)order[(size_t)i]];
+            rc = encoder_pass(enc, nb, d_order + b0, ctx->d_doc_ptr, ctx->d_doc_words, &tg, true, nullptr, s,
+                              tokens);
         }
-        if (rc == CULDA_OK) rc = encoder_take_loss(enc, ctx->D, &last, s);
+        const int taken = encoder_take_loss(enc, ctx->D, &last, s);  // also what a failed epoch has added
+        if (rc == CULDA_OK) rc = taken;
         if (rc) fail(ctx, rc, "culda_train_encoder: %s", global_error());
         // the host order buffer is rewritten by the next epoch
         if (cudaStreamSynchronize(s) != cudaSuccess && rc == CULDA_OK)

@@ -495,7 +495,8 @@ int culda_gemm_bf16(const culda_gemm_args *a, void *stream);
  * -sum_k target_k log q_k, averaged over the batch.
  * Batches are CSR slices: doc b of a batch is docs[b] (or b when docs is
  * NULL) of the CSR (doc_ptr int64[], words int32[] word ids), all device
- * pointers. */
+ * pointers.  A training batch holds fewer than 2^31 tokens
+ * (CULDA_ERR_UNSUPPORTED otherwise). */
 #define CULDA_ENC_EMBED 256
 #define CULDA_ENC_HIDDEN 512
 
