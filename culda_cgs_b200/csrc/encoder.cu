@@ -754,13 +754,13 @@ int encoder_take_loss(culda_encoder *e, int batch_rows, double *loss, cudaStream
         double loss;
         int32_t err;
     } got = {0.0, 0};
+    // cleared behind the copy and before the wait: the next pass may run on another stream
     ECK(cudaMemcpyAsync(&got, e->d_loss, sizeof got, cudaMemcpyDeviceToHost, s));
+    ECK(cudaMemsetAsync(e->d_loss, 0, sizeof got, s));
     ECK(cudaStreamSynchronize(s));
-    ECK(cudaMemsetAsync(e->d_loss, 0, sizeof(double), s));
     const double h = got.loss;
     const int32_t err = got.err;
     if (err) {
-        cudaMemsetAsync(e->d_error, 0, sizeof(int32_t), s);
         char msg[96];
         snprintf(msg, sizeof msg, "encoder: device error 0x%x", err);
         return fail_enc(CULDA_ERR_DEVICE_STATE, "%s", msg);
