@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "smem_limit.h"
+
 namespace culda {
 
 // Neumaier-compensated accumulation: s + c carries the running sum.  Both
@@ -84,14 +86,18 @@ __device__ __forceinline__ float group_excl(float v, int gl, unsigned m) {
     }
 }
 
-// Opt a kernel into more than the default dynamic shared memory (the
-// threshold leaves room for static shared memory).  Skipped while the stream
-// is being captured into a graph: the context sets every attribute first.
-inline cudaError_t allow_smem(const void *fn, size_t smem, cudaStream_t s) {
+// Opts a kernel into at least `smem` bytes of dynamic shared memory on the
+// current device (up to the threshold the default, less room for static shared
+// memory, will do).  May be called while a stream is captured.
+inline cudaError_t allow_smem(const void *fn, size_t smem) {
     if (smem <= 40 * 1024) return cudaSuccess;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (s && cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) return cudaSuccess;
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static SmemLimits limits;  // one per process
+    int device = 0;
+    const cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    return (cudaError_t)limits.raise(fn, device, smem, (int)cudaErrorMemoryAllocation, [fn](size_t bytes) {
+        return (int)cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    });
 }
 
 inline int grid_for(int64_t n) {

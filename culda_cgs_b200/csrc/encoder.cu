@@ -553,7 +553,7 @@ cudaError_t softmax_xent_n(int batch, int rows, int K, const float *Z, const Enc
                            const int64_t *doc_ptr, float *probs, bf16 *dZ, bf16 *dZt, float *db3, double *loss,
                            cudaStream_t s) {
     const size_t smem = dZ ? (size_t)kXentRows * K * sizeof(float) : 0;
-    const cudaError_t e = allow_smem(reinterpret_cast<const void *>(&softmax_xent_kernel<N>), smem, nullptr);
+    const cudaError_t e = allow_smem(reinterpret_cast<const void *>(&softmax_xent_kernel<N>), smem);
     if (e != cudaSuccess) return e;
     softmax_xent_kernel<N><<<(rows + kXentRows - 1) / kXentRows, 256, smem, s>>>(batch, rows, K, Z, tg, docs, doc_ptr,
                                                                                  probs, dZ, dZt, db3, loss);
@@ -617,8 +617,7 @@ int encoder_pass(culda_encoder *e, int batch, const int32_t *docs, const int64_t
         }
     }
     // forward
-    // set also while s is being captured (a forward pass may be)
-    ECK(allow_smem(reinterpret_cast<const void *>(&embbag_fwd_kernel), kBagSmem, nullptr));
+    ECK(allow_smem(reinterpret_cast<const void *>(&embbag_fwd_kernel), kBagSmem));
     embbag_fwd_kernel<<<Bp, 256, kBagSmem, s>>>(batch, Bp, docs, doc_ptr, words, e->V, e->emb_bf,
                                                                  e->X0, target ? e->X0t : nullptr, err);
     ECK(cudaGetLastError());

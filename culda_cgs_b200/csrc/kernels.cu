@@ -300,7 +300,7 @@ size_t theta_smem_bytes(int k) {
 
 int theta_blocks_per_sm(int k) {
     const size_t smem = theta_smem_bytes(k);
-    if (allow_smem(reinterpret_cast<const void *>(&theta_rebuild_kernel), smem, nullptr) != cudaSuccess) return 0;
+    if (allow_smem(reinterpret_cast<const void *>(&theta_rebuild_kernel), smem) != cudaSuccess) return 0;
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, theta_rebuild_kernel, kThetaWarps * 32, smem) !=
         cudaSuccess)
@@ -314,7 +314,7 @@ cudaError_t launch_theta_rebuild(int k, int num_docs, const int64_t *doc_ptr, co
                                  int num_long, int32_t *long_queue, const IterationEnd &end) {
     if (num_long > 0 && (!doc_order || !long_queue || num_long > num_docs)) return cudaErrorInvalidValue;
     const size_t smem = theta_smem_bytes(k);
-    cudaError_t e = allow_smem(reinterpret_cast<const void *>(&theta_rebuild_kernel), smem, s);
+    cudaError_t e = allow_smem(reinterpret_cast<const void *>(&theta_rebuild_kernel), smem);
     if (e != cudaSuccess) return e;
     if (num_long > 0 && !end.stats) {
         e = cudaMemsetAsync(long_queue, 0, sizeof(int32_t), s);
@@ -704,8 +704,7 @@ __global__ void __launch_bounds__(kPhiThreads) update_phi_kernel(int K, int V, c
 cudaError_t launch_update_phi(int k, int num_words, const int64_t *word_ptr, const uint16_t *topics, int32_t *phi,
                               int32_t *nk, int32_t *error, cudaStream_t s) {
     const size_t smem = (2 * (size_t)k + (size_t)kPhiWarps * (size_t)(k / 2)) * sizeof(int);
-    // set also while s is being captured: the entry point may be captured at any K
-    cudaError_t e = allow_smem(reinterpret_cast<const void *>(&update_phi_kernel), smem, nullptr);
+    cudaError_t e = allow_smem(reinterpret_cast<const void *>(&update_phi_kernel), smem);
     if (e != cudaSuccess) return e;
     int dev = 0, bps = 0;
     cudaGetDevice(&dev);
@@ -1007,7 +1006,7 @@ __global__ void __launch_bounds__(kPhiThreads) loglik_joint_kernel(const JointPa
 
 cudaError_t launch_loglik_joint(const JointParams &p, int max_partials, cudaStream_t s) {
     const size_t smem = ((size_t)p.k + (size_t)kPhiWarps * (size_t)(p.k / 2)) * sizeof(int);
-    cudaError_t e = allow_smem(reinterpret_cast<const void *>(&loglik_joint_kernel), smem, s);
+    cudaError_t e = allow_smem(reinterpret_cast<const void *>(&loglik_joint_kernel), smem);
     if (e != cudaSuccess) return e;
     int dev = 0, bps = 0;
     cudaGetDevice(&dev);

@@ -601,7 +601,7 @@ int hot_rows_if_needed(culda_ctx *ctx, int cur) {
 
 template <class Kernel>
 int persistent_grid(culda_ctx *ctx, Kernel kernel, int threads, size_t smem, int *grid) {
-    CK(allow_smem(reinterpret_cast<const void *>(kernel), smem, ctx->stream));
+    CK(allow_smem(reinterpret_cast<const void *>(kernel), smem));
     int bps = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kernel, threads, smem));
     *grid = std::max(1, std::min(ctx->num_items, num_sms(ctx->device) * std::max(bps, 1)));
@@ -752,7 +752,7 @@ extern "C" int culda_encoder_init_from_phi(culda_ctx *ctx, culda_encoder *enc, u
         rc = fail(ctx, CULDA_ERR_OOM, "culda_encoder_init_from_phi: out of device memory");
     } else {
         const size_t smem = (size_t)K * sizeof(int);
-        cudaError_t e = allow_smem(reinterpret_cast<const void *>(&phi_profile_kernel), smem, s);
+        cudaError_t e = allow_smem(reinterpret_cast<const void *>(&phi_profile_kernel), smem);
         if (e == cudaSuccess) {
             phi_profile_kernel<<<std::min(Vp, num_sms(ctx->device) * 8), 256, smem, s>>>(
                 V, Vp, K, ctx->params.beta, ctx->d_word_ptr, ctx->d_z[ctx->cur], prof);

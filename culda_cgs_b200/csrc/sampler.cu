@@ -1536,12 +1536,7 @@ int sample_blocks_per_sm(int k, int group_lanes, int blocks_per_sm) {
     const void *fn = sample_kernel_for(group_lanes, blocks_per_sm);
     if (!fn) return 0;
     const size_t smem = sample_smem_bytes(k, group_lanes);
-    if (allow_smem(fn, smem, nullptr) != cudaSuccess) return 0;
-    // launch_sample may choose the wide form, also while a stream is captured
-    if (group_lanes == kFlatLanes &&
-        allow_smem(reinterpret_cast<const void *>(&sample_flat_kernel<kWideBlocks, kWideThreads>),
-                   flat_smem_bytes(k, kWideThreads / 32), nullptr) != cudaSuccess)
-        return 0;
+    if (allow_smem(fn, smem) != cudaSuccess) return 0;
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kSampleThreads, smem) != cudaSuccess) return 0;
     return n;
@@ -1572,7 +1567,7 @@ cudaError_t launch_sample(const SampleParams &p, int group_lanes, int blocks_per
         smem = flat_smem_bytes(p.k, kWideThreads / 32);
         grid = first;
     }
-    cudaError_t e = allow_smem(fn, smem, s);
+    cudaError_t e = allow_smem(fn, smem);
     if (e != cudaSuccess) return e;
     if (first > 0) {
         void *args[] = {&head};
@@ -1584,7 +1579,7 @@ cudaError_t launch_sample(const SampleParams &p, int group_lanes, int blocks_per
     // writes)
     const size_t wsmem = sample_warp_smem_bytes(p.k);
     const void *wfn = reinterpret_cast<const void *>(&sample_warp_kernel);
-    e = allow_smem(wfn, wsmem, s);
+    e = allow_smem(wfn, wsmem);
     if (e != cudaSuccess) return e;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, wfn, 32, wsmem);
     if (e != cudaSuccess) return e;
@@ -1628,7 +1623,7 @@ cudaError_t launch_hot_rows(int k, const culda_item *hot_items, int num_hot_item
                             int32_t *hot_phi, int32_t *error, cudaStream_t s) {
     if (num_hot_items <= 0) return cudaSuccess;
     const size_t smem = (size_t)k * sizeof(int);
-    cudaError_t e = allow_smem(reinterpret_cast<const void *>(&hot_rows_kernel), smem, s);
+    cudaError_t e = allow_smem(reinterpret_cast<const void *>(&hot_rows_kernel), smem);
     if (e != cudaSuccess) return e;
     hot_rows_kernel<<<num_hot_items, 256, smem, s>>>(k, hot_items, topics, hot_phi, error);
     return cudaGetLastError();

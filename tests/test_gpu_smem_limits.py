@@ -1,0 +1,78 @@
+"""A kernel's dynamic shared-memory limit belongs to the process, the sizes to the
+topic count: contexts and calls of different K, one after the other and from two
+threads, must not take each other's room away.  Results are compared with those
+of the same calls alone, bit for bit."""
+from __future__ import annotations
+
+import ctypes as C
+import threading
+
+import numpy as np
+import pytest
+
+import culda_cgs_b200 as cb
+from culda_cgs_b200.configs import TINY
+
+pytestmark = pytest.mark.gpu
+
+
+def _chain(k, between=lambda: None):
+    """Topics and joint log-likelihood of a short chain against frozen counts, whose graphs are captured after `between`."""
+    corpus = cb.Corpus.generate(TINY.gen)
+    with cb.LDA(corpus, k, 50.0 / k, 0.01, seed=3, device=0) as m:
+        m.iterate(1)
+        phi, nk = m.phi()
+        between()
+        m.set_frozen_phi(phi, nk)  # captures the iteration again
+        ll = [s["loglik"] for s in m.iterate(2)]
+        return m.topics(), ll, m.loglik_joint()
+
+
+def _same(a, b):
+    return np.array_equal(a[0], b[0]) and a[1:] == b[1:]
+
+
+@pytest.mark.parametrize("k,smaller", [(1024, 64), (4096, 2048), (4096, 32)])
+def test_a_smaller_context_leaves_the_limit(k, smaller):
+    want = _chain(k)
+    assert _same(_chain(k, lambda: _chain(smaller)), want)
+
+
+def _update_phi(k, stream):
+    import torch
+
+    n, v = 20_000, 50
+    ptr = torch.arange(0, n + 1, n // v, dtype=torch.int64, device="cuda")
+    z = (torch.arange(n, device="cuda") * 7 % k).to(torch.int16)
+    phi = torch.zeros(v, k, dtype=torch.int32, device="cuda")
+    nk = torch.zeros(k, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    assert cb.lib().culda_update_phi(k, v, *[C.c_void_p(t.data_ptr()) for t in (ptr, z, phi, nk)],
+                                     C.c_void_p(stream.cuda_stream)) == 0
+    stream.synchronize()
+    return phi.cpu().numpy(), nk.cpu().numpy()
+
+
+def test_threads_of_different_k():
+    import torch
+
+    sizes = (64, 2048, 4096)
+    want = {k: (_chain(k), _update_phi(k, torch.cuda.Stream())) for k in sizes}
+    wrong = []
+
+    def work(k):
+        try:
+            stream = torch.cuda.Stream()
+            for _ in range(12):
+                assert _same(_chain(k), want[k][0])
+                for _ in range(20):
+                    assert all(np.array_equal(a, b) for a, b in zip(_update_phi(k, stream), want[k][1]))
+        except BaseException as e:  # noqa: BLE001
+            wrong.append((k, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in sizes]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, wrong
