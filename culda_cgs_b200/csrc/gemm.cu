@@ -23,8 +23,10 @@
 
 #include <mutex>
 
+#include "device_util.cuh"
 #include "gemm.cuh"
 #include "internal.h"
+#include "kernels.cuh"
 #include "umma.cuh"
 
 namespace culda {
@@ -283,12 +285,7 @@ cudaError_t make_map(CUtensorMap *map, const void *ptr, int rows, int cols, int 
 template <int EPI, int BN>
 cudaError_t launch(const CUtensorMap &a, const CUtensorMap &b, int M, int N, int K, const GemmEpilogue &ep,
                    int32_t *error, cudaStream_t s) {
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-        attr = cudaFuncSetAttribute(gemm_bf16_kernel<EPI, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)Tile<BN>::kSmem);
-    });
+    const cudaError_t attr = allow_smem(reinterpret_cast<const void *>(&gemm_bf16_kernel<EPI, BN>), Tile<BN>::kSmem);
     if (attr != cudaSuccess) return attr;
     gemm_bf16_kernel<EPI, BN>
         <<<dim3(N / BN, M / kBM, ep.k_splits), kGemmThreads, Tile<BN>::kSmem, s>>>(a, b, K, ep, error);
@@ -311,13 +308,9 @@ cudaError_t launch_tile(int bn, const CUtensorMap &a, const CUtensorMap &b, int 
 // 14.3 us; 4096 x 1024 13.9, 15.3 and 18.9 us.  Every width adds an output's
 // products in the same order.
 int tile_columns(int M, int N, int splits) {
-    static const int sms = [] {
-        int dev = 0, n = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-            n = 148;
-        return n;
-    }();
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const int sms = num_sms(dev);
     const int64_t wide = (int64_t)(M / kBM) * (N / 128) * splits;
     return wide * 4 <= 2 * sms ? 32 : wide * 2 <= 2 * sms ? 64 : 128;
 }
