@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -464,6 +465,13 @@ __global__ void __launch_bounds__(256) adam_kernel(const AdamParams a, const Ada
 
 using namespace culda;
 
+// What an encoder's calls read back, in pinned memory.
+struct EncoderReadback {
+    int64_t tokens;  // of a training batch, where the caller gave none
+    double loss;     // with the error word, as they lie on the device
+    int32_t error;
+};
+
 // ------------------------------------------------------------------ object
 struct culda_encoder {
     int device = 0;
@@ -488,8 +496,8 @@ struct culda_encoder {
     void *scan_tmp = nullptr, *sort_tmp = nullptr;
     size_t scan_tmp_bytes = 0, sort_tmp_bytes = 0;
     int key_bits = 1;                                // bits of the keys 0..V
-    int64_t *h_tokens = nullptr;                     // pinned: a batch's token count, where the caller gave none
-    cudaEvent_t counted = nullptr;                   // it has arrived
+    EncoderReadback *h_back = nullptr;               // pinned
+    cudaEvent_t counted = nullptr;                   // h_back->tokens has arrived
     std::vector<void *> allocs;
 
     float *tensor(int t) { return params + off[t]; }
@@ -515,7 +523,7 @@ int fail_enc(int code, const char *fmt, const char *what) {
 void free_encoder(culda_encoder *e) {
     for (void *q : e->allocs) cudaFree(q);
     if (e->counted) cudaEventDestroy(e->counted);
-    if (e->h_tokens) pinned_slot_put(e->h_tokens);
+    if (e->h_back) pinned_slot_put(e->h_back);
     delete e;
 }
 
@@ -612,7 +620,7 @@ int encoder_pass(culda_encoder *e, int batch, const int32_t *docs, const int64_t
         ECK(cudaGetLastError());
         ECK(cub::DeviceScan::ExclusiveSum(e->scan_tmp, e->scan_tmp_bytes, e->bag_len, e->bag_off, batch + 1, s));
         if (batch_tokens < 0) {
-            ECK(cudaMemcpyAsync(e->h_tokens, e->bag_off + batch, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+            ECK(cudaMemcpyAsync(&e->h_back->tokens, e->bag_off + batch, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
             ECK(cudaEventRecord(e->counted, s));
         }
     }
@@ -676,7 +684,7 @@ int encoder_pass(culda_encoder *e, int batch, const int32_t *docs, const int64_t
     // the batch's (word, row) pairs sorted by word, then one pass over them
     if (batch_tokens < 0) {
         ECK(cudaEventSynchronize(e->counted));
-        batch_tokens = *e->h_tokens;
+        batch_tokens = e->h_back->tokens;
     }
     if (batch_tokens > INT_MAX)
         return fail_enc(CULDA_ERR_UNSUPPORTED, "encoder: %s", "a training batch of more than 2^31 - 1 tokens");
@@ -749,16 +757,15 @@ int encoder_pass(culda_encoder *e, int batch, const int32_t *docs, const int64_t
 }
 
 int encoder_take_loss(culda_encoder *e, int batch_rows, double *loss, cudaStream_t s) {
-    struct {
-        double loss;
-        int32_t err;
-    } got = {0.0, 0};
+    constexpr size_t kBytes = sizeof(double) + sizeof(int32_t);
+    static_assert(offsetof(EncoderReadback, error) == offsetof(EncoderReadback, loss) + sizeof(double),
+                  "the two are copied together");
     // cleared behind the copy and before the wait: the next pass may run on another stream
-    ECK(cudaMemcpyAsync(&got, e->d_loss, sizeof got, cudaMemcpyDeviceToHost, s));
-    ECK(cudaMemsetAsync(e->d_loss, 0, sizeof got, s));
+    ECK(cudaMemcpyAsync(&e->h_back->loss, e->d_loss, kBytes, cudaMemcpyDeviceToHost, s));
+    ECK(cudaMemsetAsync(e->d_loss, 0, kBytes, s));
     ECK(cudaStreamSynchronize(s));
-    const double h = got.loss;
-    const int32_t err = got.err;
+    const double h = e->h_back->loss;
+    const int32_t err = e->h_back->error;
     if (err) {
         char msg[96];
         snprintf(msg, sizeof msg, "encoder: device error 0x%x", err);
@@ -875,7 +882,7 @@ extern "C" int culda_encoder_create(const culda_encoder_params *p, culda_encoder
         EALLOC(tmp, e->scan_tmp_bytes);
         e->scan_tmp = tmp;
     }
-    if (!(e->h_tokens = static_cast<int64_t *>(pinned_slot_get()))) return bail(cudaErrorMemoryAllocation);
+    if (!(e->h_back = static_cast<EncoderReadback *>(pinned_slot_get()))) return bail(cudaErrorMemoryAllocation);
     r = cudaEventCreateWithFlags(&e->counted, cudaEventDisableTiming);
     if (r != cudaSuccess) return bail(r);
 #undef EALLOC
