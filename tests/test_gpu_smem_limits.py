@@ -38,35 +38,47 @@ def test_a_smaller_context_leaves_the_limit(k, smaller):
     assert _same(_chain(k, lambda: _chain(smaller)), want)
 
 
-def _update_phi(k, stream):
-    import torch
+class _UpdatePhi:
+    """culda_update_phi at one K on a stream of its own.  Nothing here waits for the whole
+    device, which is not allowed while another thread captures."""
 
-    n, v = 20_000, 50
-    ptr = torch.arange(0, n + 1, n // v, dtype=torch.int64, device="cuda")
-    z = (torch.arange(n, device="cuda") * 7 % k).to(torch.int16)
-    phi = torch.zeros(v, k, dtype=torch.int32, device="cuda")
-    nk = torch.zeros(k, dtype=torch.int32, device="cuda")
-    torch.cuda.synchronize()
-    assert cb.lib().culda_update_phi(k, v, *[C.c_void_p(t.data_ptr()) for t in (ptr, z, phi, nk)],
-                                     C.c_void_p(stream.cuda_stream)) == 0
-    stream.synchronize()
-    return phi.cpu().numpy(), nk.cpu().numpy()
+    def __init__(self, k):
+        import torch
+
+        n, v = 20_000, 50
+        self.k, self.v, self.stream = k, v, torch.cuda.Stream()
+        with torch.cuda.stream(self.stream):
+            self.ptr = torch.arange(0, n + 1, n // v, dtype=torch.int64, device="cuda")
+            self.z = (torch.arange(n, device="cuda") * 7 % k).to(torch.int16)
+            self.out = [torch.zeros(v, k, dtype=torch.int32, device="cuda"),
+                        torch.zeros(k, dtype=torch.int32, device="cuda")]
+            self.host = [torch.empty_like(t, device="cpu").pin_memory() for t in self.out]
+        self.stream.synchronize()
+
+    def __call__(self):
+        import torch
+
+        tables = [C.c_void_p(t.data_ptr()) for t in (self.ptr, self.z, *self.out)]
+        assert cb.lib().culda_update_phi(self.k, self.v, *tables, C.c_void_p(self.stream.cuda_stream)) == 0
+        with torch.cuda.stream(self.stream):
+            for h, d in zip(self.host, self.out):
+                h.copy_(d, non_blocking=True)
+        self.stream.synchronize()
+        return [h.numpy().copy() for h in self.host]
 
 
 def test_threads_of_different_k():
-    import torch
-
     sizes = (64, 2048, 4096)
-    want = {k: (_chain(k), _update_phi(k, torch.cuda.Stream())) for k in sizes}
+    tables = {k: _UpdatePhi(k) for k in sizes}
+    want = {k: (_chain(k), tables[k]()) for k in sizes}
     wrong = []
 
     def work(k):
         try:
-            stream = torch.cuda.Stream()
             for _ in range(12):
                 assert _same(_chain(k), want[k][0])
                 for _ in range(20):
-                    assert all(np.array_equal(a, b) for a, b in zip(_update_phi(k, stream), want[k][1]))
+                    assert all(np.array_equal(a, b) for a, b in zip(tables[k](), want[k][1]))
         except BaseException as e:  # noqa: BLE001
             wrong.append((k, repr(e)))
 
