@@ -1164,12 +1164,12 @@ extern "C" int culda_create(const culda_corpus *c, const culda_params *p, culda_
 }
 
 // -------------------------------------------------------------- iterate
-// Iterations are queued up to kQueueDepth ahead of the host, so the GPU does
-// not wait for the host to read one iteration's statistics before it starts
-// the next (30 us of a 300 us iteration at 1M tokens).  Slot i of the event
-// ring lies between iterations i-1 and i of the call.
+// One iteration is queued behind the running one, so the GPU does not wait for
+// the host to read an iteration's statistics before it starts the next (30 us
+// of a 300 us iteration at 1M tokens; three behind it are no faster).  Slot i
+// of the event ring lies between iterations i-1 and i of the call.
 int run_iterations(culda_ctx *ctx, int n, culda_iter_stats *stats, bool mh, const std::function<int()> &launch) {
-    constexpr int kQueueDepth = kStatsRing / 2;
+    constexpr int kQueueDepth = 2;  // give_up can go back one iteration
     cudaStream_t s = ctx->stream;
     const uint32_t first = ctx->next_iteration;
     int launched = 0, done = 0;
@@ -1200,10 +1200,19 @@ int run_iterations(culda_ctx *ctx, int n, culda_iter_stats *stats, bool mh, cons
             return fail(ctx, CULDA_ERR_DEVICE_STATE, "iteration %u: device error word 0x%x", h.iteration, h.error);
         return CULDA_OK;
     };
-    // after a failure: whatever is queued has run, and the next iteration follows it
+    // After a failure: whatever is queued has run, and the next iteration follows
+    // it; but behind an iteration that reported an error the one queued is undone.
+    // It has read that iteration's topics and written the other buffers.
     auto give_up = [&](int rc) {
         cudaStreamSynchronize(s);
         ctx->next_iteration = first + (uint32_t)launched;
+        if (rc == CULDA_ERR_DEVICE_STATE && launched > done) {
+            const std::string why = ctx->err;
+            ctx->cur = 1 - ctx->cur;
+            culda_set_iteration(ctx, first + (uint32_t)done);
+            rebuild_counts(ctx);  // reports the error word again
+            fail(ctx, rc, "%s", why.c_str());
+        }
         return rc;
     };
     for (; launched < n; ++launched) {
@@ -1219,11 +1228,12 @@ int run_iterations(culda_ctx *ctx, int n, culda_iter_stats *stats, bool mh, cons
             if (rc) return rc;
             fresh = true;
         }
-        if (fresh) CK(cudaEventRecord(ctx->ev_iter[launched % kStatsRing], s));
+        cudaError_t e = fresh ? cudaEventRecord(ctx->ev_iter[launched % kStatsRing], s) : cudaSuccess;
+        if (e != cudaSuccess) return give_up(fail(ctx, CULDA_ERR_CUDA, "iteration: %s", cudaGetErrorString(e)));
         fresh = false;
         if (const int rc = launch()) return give_up(rc);
         ctx->cur = 1 - ctx->cur;
-        const cudaError_t e = cudaEventRecord(ctx->ev_iter[(launched + 1) % kStatsRing], s);
+        e = cudaEventRecord(ctx->ev_iter[(launched + 1) % kStatsRing], s);
         if (e != cudaSuccess) {
             ++launched;
             return give_up(fail(ctx, CULDA_ERR_CUDA, "iteration: %s", cudaGetErrorString(e)));

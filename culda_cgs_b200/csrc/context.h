@@ -132,7 +132,7 @@ cudaError_t iteration_prologue(culda_ctx *ctx, int cur, bool uniforms, uint32_t 
 // iteration's statistics into the pinned ring.
 cudaError_t iteration_rebuild(culda_ctx *ctx, int cur, int num_items);
 // Runs n iterations that `launch` queues on the context's stream (each from
-// d_z[cur] to d_z[1-cur], with the two calls above), a few of them ahead of
+// d_z[cur] to d_z[1-cur], with the two calls above), one of them ahead of
 // the host, and fills stats.
 int run_iterations(culda_ctx *ctx, int n, culda_iter_stats *stats, bool mh, const std::function<int()> &launch);
 

@@ -97,7 +97,7 @@ cudaError_t launch_prologue(const PrologueParams &p, cudaStream_t s);
 // per-item log terms (each CTA has summed its share into partials) and
 // writes the iteration's statistics to slot *iteration_dev % kStatsRing of
 // the pinned ring.  stats null: nothing.
-constexpr int kStatsRing = 8;
+constexpr int kStatsRing = 4;
 struct IterationEnd {
     DevStats *stats = nullptr;
     const double *item_ll = nullptr;

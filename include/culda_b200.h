@@ -238,9 +238,8 @@ int culda_create(const culda_corpus *c, const culda_params *p, culda_ctx **out);
 
 /* Run n iterations (sample, log-likelihood, rebuild counts), one CUDA graph
  * launch each, writing one culda_iter_stats per iteration into stats (may be
- * NULL).  A few iterations are queued ahead of the host; when one reports a
- * device error, those behind it have run too.  Replaces the loop body
- * SingleChunkSingleGPU.h:70-127. */
+ * NULL).  The call ends with the first iteration that reports a device error.
+ * Replaces the loop body SingleChunkSingleGPU.h:70-127. */
 int culda_iterate(culda_ctx *ctx, int n, culda_iter_stats *stats);
 
 /* Replace all topics from a host array and rebuild the counts. */
