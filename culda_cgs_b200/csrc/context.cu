@@ -560,7 +560,7 @@ __global__ void seg_scatter_kernel(int64_t n, const int32_t *__restrict__ flag, 
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
         if (flag[t]) {
             seg_start[index[t]] = (int32_t)t;
-            seg_doc[index[t]] = doc_ids[t];
+            if (seg_doc) seg_doc[index[t]] = doc_ids[t];
         }
 }
 
@@ -695,6 +695,15 @@ int build_segments_device(culda_ctx *ctx, SetupArena &arena) {
         CKS(cudaMemcpyAsync(&total, B + N, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
         CKS(cudaStreamSynchronize(s));
         ctx->num_segs = total;  // d_seg_start holds one entry per token, the most there can be
+        // The segments' docs spare the flat walk a dependent load; where they do
+        // not fit, it looks a segment's first token up instead.
+        const size_t doc_bytes = sizeof(int32_t) * (size_t)total;
+        if ((ctx->block_pooled
+                 ? cudaMallocFromPoolAsync((void **)&ctx->d_seg_doc, doc_bytes, block_pool(ctx->device), s)
+                 : cudaMalloc((void **)&ctx->d_seg_doc, doc_bytes)) != cudaSuccess) {
+            cudaGetLastError();
+            ctx->d_seg_doc = nullptr;
+        }
         seg_scatter_kernel<<<grid(N), 256, 0, s>>>(N, A, B, ctx->d_doc_ids, ctx->d_seg_start, ctx->d_seg_doc);
         item_segments_kernel<<<grid(ctx->num_items), 256, 0, s>>>(ctx->d_items, ctx->num_items, B);
         CKS(cudaGetLastError());
@@ -930,7 +939,6 @@ extern "C" int culda_create(const culda_corpus *c, const culda_params *p, culda_
         // the region set-up borrows, in the order it gives the buffers back
         const size_t o_doc_tok = add(sizeof(int32_t) * (size_t)N);
         const size_t o_seg_start = add(sizeof(int32_t) * (size_t)N);  // at most one segment per token
-        const size_t o_seg_doc = add(sizeof(int32_t) * (size_t)N);
         const size_t o_z0 = add(sizeof(uint16_t) * (size_t)N);
         const size_t o_z1 = add(sizeof(uint16_t) * (size_t)N);
         const size_t o_zx = add(sizeof(uint16_t) * (size_t)N);
@@ -960,7 +968,6 @@ extern "C" int culda_create(const culda_corpus *c, const culda_params *p, culda_
         ctx->d_hot_phi = reinterpret_cast<int32_t *>(b + o_hot_phi);
         ctx->d_item_ll = reinterpret_cast<double *>(b + o_item_ll);
         ctx->d_seg_start = reinterpret_cast<int32_t *>(b + o_seg_start);
-        ctx->d_seg_doc = reinterpret_cast<int32_t *>(b + o_seg_doc);
         ctx->d_counter = reinterpret_cast<int32_t *>(b + o_counter);
         ctx->d_iter = reinterpret_cast<uint32_t *>(b + o_iter);
         ctx->d_stats = reinterpret_cast<DevStats *>(b + o_stats);
@@ -1423,7 +1430,7 @@ extern "C" int culda_get_info(const culda_ctx *ctx, culda_info *info) {
     (void)D;
     (void)V;
     (void)K;
-    info->device_bytes = (int64_t)ctx->block_bytes;
+    info->device_bytes = (int64_t)ctx->block_bytes + (ctx->d_seg_doc ? (int64_t)sizeof(int32_t) * ctx->num_segs : 0);
     info->doc_term = ctx->doc_term;
     return CULDA_OK;
 }
@@ -1448,12 +1455,13 @@ extern "C" void culda_destroy(culda_ctx *ctx) {
     free_learned_state(ctx);
     for (int c = 0; c < 2; ++c)
         if (ctx->graph[c]) cudaGraphExecDestroy(ctx->graph[c]);
-    if (ctx->d_block) {
+    for (void *p : {(void *)ctx->d_seg_doc, (void *)ctx->d_block}) {
+        if (!p) continue;
         if (ctx->block_pooled) {  // back to the pool, ordered after the stream's work
-            cudaFreeAsync(ctx->d_block, ctx->stream);
+            cudaFreeAsync(p, ctx->stream);
             cudaStreamSynchronize(ctx->stream);
         } else {
-            cudaFree(ctx->d_block);
+            cudaFree(p);
         }
     }
     if (ctx->h_stats) pinned_slot_put(ctx->h_stats);

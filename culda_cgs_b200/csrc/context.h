@@ -47,7 +47,7 @@ struct culda_ctx {
     int32_t num_long_items = 0;          // items counted by a whole CTA (long_items)
     double *d_partials = nullptr;        // [kMaxPartials] per-CTA sums of the reductions
     int32_t *d_seg_start = nullptr;  // first stored token of every segment
-    int32_t *d_seg_doc = nullptr;    // its doc
+    int32_t *d_seg_doc = nullptr;    // its doc: an allocation of its own, or null when there was no room
     float *d_inv = nullptr;          // [K] 1 / (n_k + V beta) of the iteration (prologue)
     int32_t first_warp = 0;          // items from here on are sampled a warp each
     int32_t num_segs = 0;
