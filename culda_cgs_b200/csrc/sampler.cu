@@ -867,6 +867,7 @@ __global__ void __launch_bounds__(THREADS, MINB) sample_flat_kernel(const Sample
             if (tid == 0) s_tiny = 0;  // read by every thread before the barrier above
         }
 
+        // the walk, the scan and the draw: a second time behind this kernel, for warps that work alone
         double ll = 0.0;
         const int sg_end = item.seg_begin + item.seg_count;
         // chunks of a quarter of the item's segments (at most 32), so the four
@@ -1044,6 +1045,13 @@ __global__ void __launch_bounds__(THREADS, MINB) sample_flat_kernel(const Sample
     if (tid == 0) clock_end(p.clock);
 }
 
+// From here to sample_warp_kernel: the walk, the scan of its sums and the draw
+// once more, for a warp that works alone.  They and sample_flat_kernel's own
+// must keep the same sums in the same order and change together (the tests
+// compare their draws): as functions that both kernels share, the same registers
+// but another schedule, sample_flat_kernel takes 5.83 ms instead of 5.70 at 61M
+// tokens.
+
 // The shared-memory arrays of one warp of the flat walk.
 struct FlatWarp {
     const float *ph;  // [K] phihat of the word
@@ -1100,11 +1108,6 @@ __device__ __forceinline__ SegMeta load_row(const SampleParams &p, bool valid, S
     else
         atomicOr(p.error, kErrRowRange);
     return m;
-}
-
-__device__ __forceinline__ SegMeta load_segment(const SampleParams &p, bool valid, int sg, int sg_end, int64_t ibeg,
-                                                int64_t iend, int B) {
-    return load_row(p, valid, load_tokens(p, valid, sg, sg_end, iend), ibeg, iend, B);
 }
 
 // One walk group's range [gb, ge) of units, of a batch of n segments: every
@@ -1180,15 +1183,6 @@ __device__ __forceinline__ void draw_one(const SampleParams &p, const FlatWarp &
     ll += (double)w.m_lg[i];
 }
 
-// Draws the total_t tokens of a walked batch of n segments, one per lane: lane
-// f takes tokens f, f + 32, ...  Adds their log terms to ll.
-__device__ __forceinline__ void draw_batch(const SampleParams &p, const FlatWarp &w, int n, int total_t, float Q,
-                                           bool tiny, const int *tk, const float *tdc, int tm, uint32_t iter,
-                                           double &ll) {
-    for (int f = threadIdx.x & 31; f < total_t; f += 32)
-        draw_one(p, w, draw_token(p, w, n, f, iter), Q, tiny, tk, tdc, tm, ll);
-}
-
 // The batch's segments [0, n) (lane `first` + i holds segment i, incl and tincl
 // the inclusive sums of units and tokens from lane `first`) into the warp's
 // arrays; ends with a warp barrier.
@@ -1226,8 +1220,8 @@ __device__ __forceinline__ int range_steps(int total_u) { return ((total_u + 31)
 
 // A warp's own items: walks and draws n segments, held from lane `first` on,
 // as one batch that joins up to kJoinedParts parts of `part` segments.  A part
-// is what flat_batches walks at a time (a chunk, or as much of it as fits the
-// budget), and its units are cut into the same ranges, so every prefix has the
+// is what sample_flat_kernel walks at a time (a chunk, or as much of it as fits
+// the budget), and its units are cut into the same ranges, so every prefix has the
 // same bits; but the ranges of all parts share the 8 walk groups, and their
 // tokens one round of draws.  A small item's chunks are a few segments each:
 // one after the other they leave most lanes idle.
@@ -1278,7 +1272,7 @@ __device__ __forceinline__ void joined_parts(const SampleParams &p, const FlatWa
     __syncwarp();
     const float my_v = gb < ge ? js.gv[lane] : 0.f;
     const int my_flag = gb < ge ? js.lead[lane] & 1 : 0;
-    // the segmented scan over a part's ranges, as flat_batches makes it
+    // the segmented scan over a part's ranges, as sample_flat_kernel makes it
     double vd = (double)my_v;
     int fl = my_flag;
 #pragma unroll
