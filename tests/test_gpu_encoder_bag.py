@@ -46,6 +46,42 @@ def test_forward_at_the_bag_limits(batch):
         assert forward() == _ffi.CULDA_ERR_DEVICE_STATE
 
 
+BAG_LENGTHS = [1, 7, 8, 9, 31, 32, 33, 95, 96, 97, 8 * 12 + 1, 8 * 32 - 1, 8 * 32, 8 * 32 + 1, 8 * 96, 8 * 97, 5000]
+
+
+@pytest.mark.parametrize("seed", [0, 1])
+def test_the_bag_alone(seed):
+    """The mean itself, bit for bit.  Word c's embedding is 1 in column c and in column
+    255, so a column's sum is a whole number (a token left out or taken twice changes
+    it) and column 255 of the mean is 1.  With one document in the batch
+    dW1[h, c] = dP1[h] * mean[c], a product of two BF16 numbers, which FP32 holds
+    exactly: the mean is dW1[h, c] / dW1[h, 255]."""
+    import torch
+
+    rng = np.random.default_rng(seed)
+    V, K = 255, 128
+    lens = np.array(BAG_LENGTHS)
+    doc_ptr = np.concatenate([[0], np.cumsum(lens)])
+    words = rng.integers(0, V, doc_ptr[-1])
+    emb = np.zeros((V, 256))
+    emb[np.arange(V), np.arange(V)] = emb[:, 255] = 1.0
+    with cb.Encoder(V, K, max_batch=1, seed=3 + seed) as enc:
+        enc.set("E", emb)
+        d = [torch.from_numpy(x).cuda() for x in (doc_ptr.astype(np.int64), words.astype(np.int32))]
+        target = torch.from_numpy(EO.random_target(rng, 1, K).astype(np.float32)).cuda()
+        for i, n in enumerate(lens):
+            which = torch.tensor([i], dtype=torch.int32, device="cuda")
+            loss = C.c_double()
+            assert cb.lib().culda_encoder_backward(enc.handle, 1, *[C.c_void_p(x.data_ptr()) for x in
+                                                   (which, *d, target)], C.byref(loss), None) == 0
+            g = enc.get("W1", grad=True)
+            h = np.abs(g[:, 255]).argmax()
+            count = np.bincount(words[doc_ptr[i]:doc_ptr[i + 1]], minlength=256)
+            count[255] = n
+            mean = torch.from_numpy(count.astype(np.float32) * (np.float32(1.0) / np.float32(n)))
+            assert np.array_equal(g[h] / g[h, 255], mean.to(torch.bfloat16).float().numpy()), n
+
+
 def _batch(rng, V, lens):
     """Documents of the given lengths, each with its words in order, so runs of one word occur."""
     doc_ptr = np.concatenate([[0], np.cumsum(lens)])
