@@ -15,10 +15,11 @@
 #include <atomic>
 #include <cstdint>
 #include <cstring>
+#include <exception>
 #include <mutex>
-#include <system_error>
+#include <new>
 #include <thread>
-#include <vector>
+#include <utility>
 
 #include "internal.h"
 
@@ -43,7 +44,7 @@ struct Ring {
 constexpr int kDevices = 64;
 constexpr size_t kKept = 2;
 std::mutex g_mu;
-std::vector<Ring *> g_idle[kDevices];
+Ring *g_idle[kDevices][kKept] = {};
 
 void free_ring(Ring *r) {
     for (cudaEvent_t e : r->free_at)
@@ -58,13 +59,11 @@ void free_ring(Ring *r) {
 Ring *take_ring(int device) {
     {
         std::lock_guard<std::mutex> lock(g_mu);
-        if (!g_idle[device].empty()) {
-            Ring *r = g_idle[device].back();
-            g_idle[device].pop_back();
-            return r;
-        }
+        for (Ring *&kept : g_idle[device])
+            if (kept) return std::exchange(kept, nullptr);
     }
-    Ring *r = new Ring;
+    Ring *r = new (std::nothrow) Ring;
+    if (!r) return nullptr;
     bool ok = cudaMallocHost((void **)&r->base, kSlotBytes * kSlots) == cudaSuccess;
     if (!ok) r->base = nullptr;
     for (cudaEvent_t &e : r->free_at)
@@ -83,10 +82,11 @@ Ring *take_ring(int device) {
 void put_ring(int device, Ring *r) {
     {
         std::lock_guard<std::mutex> lock(g_mu);
-        if (g_idle[device].size() < kKept) {
-            g_idle[device].push_back(r);
-            return;
-        }
+        for (Ring *&kept : g_idle[device])
+            if (!kept) {
+                kept = r;
+                return;
+            }
     }
     free_ring(r);
 }
@@ -149,7 +149,7 @@ cudaError_t staged_copy(char *host, char *dev, size_t bytes, bool to_host, Ring 
     const int threads = (int)std::min<int64_t>(kSlots, blocks);
     try {
         for (int t = 1; t < threads; ++t) team[t] = std::thread(work, t);
-    } catch (const std::system_error &) {  // no more threads: those that run share the blocks
+    } catch (const std::exception &) {  // no more threads (or no memory for one): those that run share the blocks
     }
     work(0);
     for (std::thread &t : team)
@@ -185,12 +185,13 @@ cudaError_t copy_to_device(void *dst, const void *src, size_t bytes, cudaStream_
 
 void release_staging(int device) {
     if (device < 0 || device >= kDevices) return;
-    std::vector<Ring *> idle;
+    Ring *idle[kKept];
     {
         std::lock_guard<std::mutex> lock(g_mu);
-        idle.swap(g_idle[device]);
+        for (size_t i = 0; i < kKept; ++i) idle[i] = std::exchange(g_idle[device][i], nullptr);
     }
-    for (Ring *r : idle) free_ring(r);
+    for (Ring *r : idle)
+        if (r) free_ring(r);
 }
 
 }  // namespace culda
