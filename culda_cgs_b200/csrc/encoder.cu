@@ -757,12 +757,18 @@ int encoder_take_loss(culda_encoder *e, int batch_rows, double *loss, cudaStream
     constexpr size_t kBytes = sizeof(double) + sizeof(int32_t);
     static_assert(offsetof(EncoderReadback, error) == offsetof(EncoderReadback, loss) + sizeof(double),
                   "the two are copied together");
-    // cleared behind the copy and before the wait: the next pass may run on another stream
+    // Cleared before the call returns: the next pass may run on another stream.  Behind
+    // a forward pass there is nothing to clear but its error word, if it set one (a
+    // clearing behind every pass: 3 us of the 60 for one document).
     ECK(cudaMemcpyAsync(&e->h_back->loss, e->d_loss, kBytes, cudaMemcpyDeviceToHost, s));
-    ECK(cudaMemsetAsync(e->d_loss, 0, kBytes, s));
+    if (batch_rows > 0) ECK(cudaMemsetAsync(e->d_loss, 0, kBytes, s));
     ECK(cudaStreamSynchronize(s));
     const double h = e->h_back->loss;
     const int32_t err = e->h_back->error;
+    if (batch_rows == 0 && (err || h != 0.0)) {
+        ECK(cudaMemsetAsync(e->d_loss, 0, kBytes, s));
+        ECK(cudaStreamSynchronize(s));
+    }
     if (err) {
         char msg[96];
         snprintf(msg, sizeof msg, "encoder: device error 0x%x", err);

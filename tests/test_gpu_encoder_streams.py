@@ -47,3 +47,24 @@ def test_losses_of_passes_on_alternating_streams(batch):
             if i % 4 == 3:
                 assert backward(s, C.c_void_p(bad.data_ptr())) == _ffi.CULDA_ERR_DEVICE_STATE
                 assert s.query()
+
+
+def test_a_forward_pass_that_fails_leaves_no_error_behind():
+    import torch
+
+    rng = np.random.default_rng(4)
+    V, K, batch = 200, 128, 5
+    doc_ptr, words = EO.random_batch(rng, V, batch, 30)
+    ptr, good = (torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in
+                 (doc_ptr.astype(np.int64), words.astype(np.int32)))
+    bad = torch.full_like(good, V)
+    probs = torch.zeros(batch, K, device="cuda")
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    with cb.Encoder(V, K, max_batch=batch) as enc:
+        for i in range(20):
+            s = streams[i % 2]
+            for w, rc in ((bad, _ffi.CULDA_ERR_DEVICE_STATE), (good, 0)):
+                assert cb.lib().culda_encoder_forward(enc.handle, batch, None, *[C.c_void_p(x.data_ptr()) for x in
+                                                      (ptr, w, probs)], C.c_void_p(s.cuda_stream)) == rc
+                assert s.query()
