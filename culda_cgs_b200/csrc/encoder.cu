@@ -183,11 +183,12 @@ __global__ void __launch_bounds__(256) embbag_fwd_kernel(int batch, int rows, co
 // plain stores; a word whose run crosses the chunk's first or last token (the
 // frequent ones) adds each chunk's partial sum with one vector atomic per
 // lane.  gE holds zeros before the pass; words outside [0, V) sort last under
-// the key V and are skipped.  So a word's terms are added in one order, but for
-// the words in several chunks, and a training run repeats but for those.
-// (Vector reductions straight to the words' rows need no sort, 24 us instead of
-// 79 for 102k tokens, but add every word's terms in the order of arrival: after
-// eight steps the weights of two runs were up to 3e-5 apart instead of 5e-6.)
+// the key V and are skipped.  So a word's terms are added in one order, and its
+// row repeats bit for bit, unless it spans three chunks or more.  (Vector
+// reductions straight to the words' rows need no sort, 24 us instead of 79 for
+// 102k tokens, but add every word's terms in the order of arrival, rounded once
+// more: at 1024 documents two runs then differ in 16% of the gradient's values
+// instead of 0.3%, and by 4.5e-7 instead of 2.4e-7 in norm.)
 
 // len[b] = L_b (for the scan of row offsets) and inv_len[b] = 1 / L_b.
 __global__ void bag_rows_kernel(int batch, const int32_t *__restrict__ docs, const int64_t *__restrict__ doc_ptr,
