@@ -58,7 +58,7 @@ struct culda_ctx {
     culda::DevStats *d_stats = nullptr;
     int32_t *d_error = nullptr;
     culda::DevStats *h_stats = nullptr;  // pinned ring of kStatsRing (a slot of the process-wide pool)
-    char *d_block = nullptr;             // every buffer above that culda_create allocates, in one allocation
+    char *d_block = nullptr;             // the other buffers above that culda_create allocates, in one allocation
     size_t block_bytes = 0;
     bool block_pooled = false;           // d_block came from the device's block pool (freed back to it)
 
